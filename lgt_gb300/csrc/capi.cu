@@ -1115,7 +1115,7 @@ void lgt_ham_destroy(lgt_ham* h) {
   // by cudaFree, which waits for the device
   cudaStream_t s = h->b ? h->b->B.stream : nullptr;
   if (h->b) cudaSetDevice(h->b->device);
-  krylov_cache_free(h->cache);
+  krylov_cache_free(h->cache, s);
   h->x.release(s);
   h->y.release(s);
   h->part.release(s);

@@ -30,6 +30,7 @@
 #include <vector>
 
 #include "lgt_bulk.cuh"
+#include "lgt_cheb.h"
 #include "lgt_dfloat.cuh"
 #include "lgt_krylov.h"
 #include "lgt_tridiag.cuh"
@@ -2404,6 +2405,7 @@ struct KrylovCache {
   Work<double> dots;  // reduction buffers of panel_dots only
   Work<double> tune_d;  // explicit autotuning (lgt_autotune), released after use
   Work<float> tune_f;
+  ChebWork cheb_d, cheb_f;  // exponentials by Chebyshev expansion (cheb.cu)
   ~KrylovCache() {
     gs_d.release();
     gs_f.release();
@@ -2446,7 +2448,12 @@ std::string ensure_row_order(OpDev* op, cudaStream_t s) {
 }
 
 KrylovCache* krylov_cache_new() { return new KrylovCache(); }
-void krylov_cache_free(KrylovCache* c) { delete c; }
+void krylov_cache_free(KrylovCache* c, cudaStream_t s) {
+  if (!c) return;
+  c->cheb_d.release(s);
+  c->cheb_f.release(s);
+  delete c;
+}
 
 cudaError_t apply_h_d(const OpDev& op, const double* x, double* y, int ncomp, cudaStream_t s) {
   return apply_h<double>(op, x, nullptr, 0, y, ncomp, s);
@@ -2492,6 +2499,20 @@ std::string krylov_expm(const OpDev& op, const KrylovParams& p, KrylovCache* cac
                         int n_steps, double* X, double* norm_drift, StepObserver* obs,
                         cudaStream_t s, KrylovReport* rep) {
   if (op.K * 2 > kT) return "at most 128 complex points per panel";
+  // A step whose Chebyshev expansion takes at most krylovdim products runs as
+  // one (4x4 K = 8 mixed: see cheb.cu); longer steps, a forced H*psi kernel
+  // or LGT_EXPM=krylov (cross-checks) take the Krylov space, which halves
+  // the step until its space is large enough.
+  const char* ex = getenv("LGT_EXPM");
+  if (!(ex && ex[0] == 'k') && !hpsi_forced()) {
+    OpDev o = op;
+    bool done = false;
+    if (dt > 0.0 && n_steps > 0 && ensure_table(&o, s)) {
+      const std::string err = cheb_expm(o, p, p.mixed ? &cache->cheb_f : &cache->cheb_d, dt,
+                                        n_steps, X, norm_drift, obs, s, rep, &done);
+      if (done || !err.empty()) return err;
+    }
+  }
   if (p.mixed)
     return expm_impl<float>(op, p, cache->ex_f, dt, n_steps, X, norm_drift, obs, s, rep);
   return expm_impl<double>(op, p, cache->ex_d, dt, n_steps, X, norm_drift, obs, s, rep);

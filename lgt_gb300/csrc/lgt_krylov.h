@@ -93,7 +93,7 @@ struct KrylovReport {
 // Workspaces and captured graphs of the drivers, kept per Hamiltonian.
 struct KrylovCache;
 KrylovCache* krylov_cache_new();
-void krylov_cache_free(KrylovCache* c);
+void krylov_cache_free(KrylovCache* c, cudaStream_t s);
 
 // Lowest eigenpair of each of the K operators.  X (device, double, [N][K])
 // receives the normalised eigenvectors; when start_given, X holds the start

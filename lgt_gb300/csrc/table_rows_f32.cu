@@ -1,0 +1,29 @@
+// table_rows_f32.cu -- FP32 instances of the table products of
+// lgt_table_rows.cuh.
+#include "lgt_cheb.h"
+#include "lgt_table_rows.cuh"
+
+namespace lgt {
+
+// Slices of 32, 16 or 8 bytes: the widest that divides the panel row.
+cudaError_t launch_cheb_product(const NbrTable& T, uint32_t model, int64_t N, int K, const float* x,
+                                float* y, const float* prev, const float* coef, cudaStream_t s) {
+  rows::Args<float> a = {};
+  a.meta = T.meta;
+  a.off = T.tile_off;
+  a.nbr = T.nbr;
+  a.mm = T.mm;
+  a.N = N;
+  a.C = 2 * K;
+  a.ncomp = 2;
+  a.K = K;
+  a.x = x;
+  a.y = y;
+  a.prev = prev;
+  a.coef = coef;
+  if (a.C % 8 == 0) return rows::launch_model<float, 8, 4, true>(a, model, s);
+  if (a.C % 4 == 0) return rows::launch_model<float, 4, 8, true>(a, model, s);
+  return rows::launch_model<float, 2, 8, true>(a, model, s);
+}
+
+}  // namespace lgt
