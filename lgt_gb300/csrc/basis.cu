@@ -386,6 +386,110 @@ __global__ void k_tab_check(RankView R, int* bad) {
   if (i < R.dim && !tab_ranks_own_index(R, i)) atomicOr(bad, 1);
 }
 
+// ---- the basis from its rank tables -----------------------------------------
+//
+// The tables above need only the Gauss law, not the keys, so where they fit
+// they also enumerate: entry [F] of T_0 is the size of each mask's segment,
+// and state i of the sector is found by descending the tables row by row
+// (the inverse of its rank).  One thread per state writes its key; nothing
+// is scanned for candidates.  Against two passes of the ordered compaction
+// over all (mask, free digits) candidates (253 M of them at 4x4, 3.3 + 3.7
+// ms of integer work) the tables take 0.08 ms and the descent, bound by its
+// dependent table loads (L2), well below that.
+
+// segc = exclusive scan of the segment sizes T_0[mask][F] (before segc is
+// folded into T_0); total[0] = the sector dimension.  One block: a scan of
+// one value per mask.
+__global__ void __launch_bounds__(1024) k_seg_scan(const uint32_t* masks, int nmasks, int F,
+                                                   const uint32_t* T0, uint32_t* segc,
+                                                   uint64_t* total) {
+  __shared__ uint64_t warp_sum[32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  // thread t owns the contiguous masks t * per .. t * per + per - 1
+  const int per = (nmasks + 1023) / 1024;
+  const int m0 = int(threadIdx.x) * per, m1 = (m0 + per < nmasks) ? m0 + per : nmasks;
+  uint64_t v = 0;
+  for (int m = m0; m < m1; ++m) v += T0[uint64_t(masks[m]) * (F + 1) + F];
+  uint64_t x = v;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint64_t y = __shfl_up_sync(0xffffffffu, x, d);
+    if (lane >= d) x += y;
+  }
+  if (lane == 31) warp_sum[wid] = x;
+  __syncthreads();
+  if (wid == 0) {
+    uint64_t s = warp_sum[lane];
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint64_t y = __shfl_up_sync(0xffffffffu, s, d);
+      if (lane >= d) s += y;
+    }
+    warp_sum[lane] = s;
+  }
+  __syncthreads();
+  uint64_t run = x - v + (wid > 0 ? warp_sum[wid - 1] : 0);
+  for (int m = m0; m < m1; ++m) {
+    segc[m] = uint32_t(run);
+    run += T0[uint64_t(masks[m]) * (F + 1) + F];
+  }
+  if (threadIdx.x == 0) {
+    segc[nmasks] = uint32_t(warp_sum[31]);
+    total[0] = warp_sum[31];
+  }
+}
+
+// One block per mask, one thread per state of its segment.  A state that
+// the Gauss law refuses (never for consistent tables) raises `bad`.
+__global__ void __launch_bounds__(128) k_tab_emit(Geom G, RankView R, const uint32_t* masks,
+                                                  const uint32_t* segc, uint64_t* keys,
+                                                  uint32_t* low, int* bad) {
+  const uint32_t mask = masks[blockIdx.x];
+  const uint32_t first = segc[blockIdx.x], last = segc[blockIdx.x + 1];
+  const uint32_t F1 = uint32_t(R.F) + 1u;
+  const int nx = G.nx, nrows = R.nrows;
+  for (uint32_t i = first + threadIdx.x; i < last; i += blockDim.x) {
+    uint32_t left = i;  // T_0 carries the segment start
+    uint32_t fp = 0;
+    uint64_t digits = 0;
+    int S = 0;  // row sum S_r = -sum over the site rows above r
+    for (int j = 1; j < G.ny; ++j)
+      S -= __popc((mask >> (j * nx)) & ((1u << nx) - 1u)) + G.grow[j];
+    bool ok = true;
+    for (int r = 0; r < nrows; ++r) {
+      const uint32_t* T =
+          (r == 0) ? R.tab + uint64_t(mask) * F1
+                   : R.tab + R.tab_off[r] + (uint64_t(mask >> (r * nx)) * uint64_t(R.F) + fp) * F1;
+      // the last v whose count of earlier states is <= left
+      uint32_t lo = 0, hi = uint32_t(R.F);
+      while (hi - lo > 1) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (__ldg(T + mid) <= left) lo = mid;
+        else hi = mid;
+      }
+      left -= __ldg(T + lo);
+      fp = lo;
+      int sum = 0;
+      for (int ix = 0; ix < nx; ++ix) {
+        int d;
+        if (ix < nx - 1) {
+          d = int((lo / uint32_t(R.pw[ix])) % uint32_t(R.B)) - G.dg;
+          sum += d;
+        } else {
+          d = S - sum;
+          ok = ok && d >= -G.dg && d <= G.dg;
+        }
+        digits = (digits << G.w) | uint64_t(uint32_t(d + G.dg) & ((1u << G.w) - 1u));
+      }
+      if (r + 1 < G.ny) S += __popc((mask >> ((r + 1) * nx)) & ((1u << nx) - 1u)) + G.grow[r + 1];
+    }
+    uint64_t rp;
+    if (!ok || left != 0 || !derive_eR(G, mask, digits, &rp)) atomicOr(bad, 1);
+    keys[i] = make_key(G, mask, digits);
+    if (low) low[i] = uint32_t(digits);
+  }
+}
+
 // ---- small sectors in one launch -------------------------------------------
 //
 // For a candidate space of at most kFusedMaxCandidates and tables of at most
@@ -636,12 +740,27 @@ bool tab_plan(const Geom& G, int* Fo, int64_t* off, int64_t* toto, int64_t* nlas
   return true;
 }
 
+// The tables T_r (segment starts not yet folded in), bottom up.
+std::string launch_tables(const Geom& G, int F, const int64_t* off, int64_t nlast, uint32_t* tab,
+                          uint32_t* L, cudaStream_t s) {
+  const int nrows = G.ny - 1;
+  k_tab_last<<<unsigned((nlast * F + 255) / 256), 256, 0, s>>>(G, F, L), lgt::note_launch();
+  for (int r = nrows - 1; r >= 0; --r) {
+    const int64_t nm = int64_t(1) << (G.nx * (G.ny - r));
+    const int Fp = (r == 0) ? 1 : F;
+    const uint32_t* next = (r == nrows - 1) ? L : tab + off[r + 1];
+    k_tab_row<<<unsigned((nm * Fp + 255) / 256), 256, 0, s>>>(G, F, r, next, r == nrows - 1,
+                                                              tab + off[r], Fp, nm), lgt::note_launch();
+  }
+  CK(cudaGetLastError());
+  return std::string();
+}
+
 // Builds the row-count rank tables when they fit (at most 2^25 entries) and
 // keeps them only if every basis key ranks to its own index through them.
 std::string build_rank_tables(BasisDev* B) {
   const Geom& G = B->G;
   cudaStream_t s = B->stream;
-  const int nrows = G.ny - 1;
   int F = 0;
   int64_t off[kMaxTabRows], tot = 0, nlast = 0;
   if (B->dim == 0 || !tab_plan(G, &F, off, &tot, &nlast)) return std::string();
@@ -652,14 +771,8 @@ std::string build_rank_tables(BasisDev* B) {
   CK(dev_alloc_n(&L, size_t(nlast * F), s));
   CK(dev_alloc_n(&bad, 1, s));
   CK(cudaMemsetAsync(bad, 0, sizeof(int), s));
-  k_tab_last<<<unsigned((nlast * F + 255) / 256), 256, 0, s>>>(G, F, L), lgt::note_launch();
-  for (int r = nrows - 1; r >= 0; --r) {
-    const int64_t nm = int64_t(1) << (G.nx * (G.ny - r));
-    const int Fp = (r == 0) ? 1 : F;
-    const uint32_t* next = (r == nrows - 1) ? L : tab + off[r + 1];
-    k_tab_row<<<unsigned((nm * Fp + 255) / 256), 256, 0, s>>>(G, F, r, next, r == nrows - 1,
-                                                              tab + off[r], Fp, nm), lgt::note_launch();
-  }
+  const std::string e = launch_tables(G, F, off, nlast, tab, L, s);
+  if (!e.empty()) return e;
   k_tab_seg<<<unsigned((int64_t(B->nmasks) * (F + 1) + 255) / 256), 256, 0, s>>>(
       G, B->masks, B->segc, B->nmasks, F, tab), lgt::note_launch();
   CK(cudaGetLastError());
@@ -678,6 +791,57 @@ std::string build_rank_tables(BasisDev* B) {
     B->tab_F = 0;
     return "rank tables failed their self-check";
   }
+  return std::string();
+}
+
+// Segments, keys, low parts and rank tables of a sector whose tables fit
+// (k_seg_scan, k_tab_emit); B->masks holds its masks.  *done stays false,
+// with nothing kept, where the tables do not apply.
+std::string build_basis_tables(BasisDev* B, bool* done) {
+  const Geom& G = B->G;
+  cudaStream_t s = B->stream;
+  int F = 0;
+  int64_t off[kMaxTabRows], tot = 0, nlast = 0;
+  if (B->nmasks < 1 || !tab_plan(G, &F, off, &tot, &nlast)) return std::string();
+  uint32_t* L = nullptr;
+  uint64_t* hdr = nullptr;  // dimension, then the check's flag
+  CK(dev_alloc_n(&B->tab, size_t(tot), s));
+  CK(dev_alloc_n(&L, size_t(nlast * F), s));
+  CK(dev_alloc_n(&hdr, 2, s));
+  CK(dev_alloc_n(&B->segc, size_t(B->nmasks) + 1, s));
+  CK(cudaMemsetAsync(hdr, 0, 2 * sizeof(uint64_t), s));
+  std::string e = launch_tables(G, F, off, nlast, B->tab, L, s);
+  if (!e.empty()) return e;
+  k_seg_scan<<<1, 1024, 0, s>>>(B->masks, B->nmasks, F, B->tab, B->segc, hdr), lgt::note_launch();
+  k_tab_seg<<<unsigned((int64_t(B->nmasks) * (F + 1) + 255) / 256), 256, 0, s>>>(
+      G, B->masks, B->segc, B->nmasks, F, B->tab), lgt::note_launch();
+  CK(cudaGetLastError());
+  uint64_t dim = 0;
+  CK(cudaMemcpyAsync(&dim, hdr, sizeof(dim), cudaMemcpyDeviceToHost, s));
+  CK(dev_free(L, s));
+  CK(cudaStreamSynchronize(s));
+  if (dim >= (uint64_t(1) << 32) - 1) return "sector dimension exceeds 2^32";
+  B->dim = int64_t(dim);
+  B->tab_F = F;
+  for (int r = 0; r < kMaxTabRows; ++r) B->tab_off[r] = off[r];
+  *done = true;
+  if (dim == 0) {  // an empty sector keeps no tables
+    CK(dev_free(B->tab, s));
+    CK(dev_free(hdr, s));
+    B->tab = nullptr;
+    B->tab_F = 0;
+    return std::string();
+  }
+  CK(dev_alloc_n(&B->keys, size_t(dim), s));
+  if (G.ushift <= 32) CK(dev_alloc_n(&B->low, size_t(dim), s));
+  k_tab_emit<<<unsigned(B->nmasks), 128, 0, s>>>(G, B->view(), B->masks, B->segc, B->keys, B->low,
+                                                 reinterpret_cast<int*>(hdr + 1)), lgt::note_launch();
+  CK(cudaGetLastError());
+  int bad = 0;
+  CK(cudaMemcpyAsync(&bad, hdr + 1, sizeof(int), cudaMemcpyDeviceToHost, s));
+  CK(dev_free(hdr, s));
+  CK(cudaStreamSynchronize(s));
+  if (bad) return "rank tables failed their self-check";
   return std::string();
 }
 
@@ -801,7 +965,16 @@ std::string build_basis_device(BasisDev* B) {
   if (!err.empty()) return err;
   B->nmasks = int(nmasks);
 
-  // 2. candidates (mask, free e_U digits) -> sorted order keys
+  // 2. keys, segments and tables from the row counts where those fit
+  //    (LGT_BASIS_TABLES=0: the compaction below, for cross-checks)
+  const char* tz = std::getenv("LGT_BASIS_TABLES");
+  if (!(tz && tz[0] == '0')) {
+    bool done = false;
+    err = build_basis_tables(B, &done);
+    if (done || !err.empty()) return err;
+  }
+
+  // 3. candidates (mask, free e_U digits) -> sorted order keys
   int64_t dim = 0;
   if (nmasks > 0) {
     switch (G.dg) {
@@ -827,7 +1000,7 @@ std::string build_basis_device(BasisDev* B) {
   if (dim >= (int64_t(1) << 32) - 1) return "sector dimension exceeds 2^32";
   B->dim = dim;
 
-  // 3. ranking tables
+  // 4. ranking tables
   CK(dev_alloc_n(&B->segc, size_t(nmasks) + 1, s));
   k_segments<<<int((nmasks + 1 + 255) / 256), 256, 0, s>>>(B->keys, dim, B->masks, int(nmasks),
                                                           G.ushift, B->segc), lgt::note_launch();
