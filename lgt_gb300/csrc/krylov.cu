@@ -33,6 +33,7 @@
 #include "lgt_cheb.h"
 #include "lgt_dfloat.cuh"
 #include "lgt_krylov.h"
+#include "lgt_lanczos_grid.h"
 #include "lgt_tridiag.cuh"
 
 namespace lgt {
@@ -1371,6 +1372,8 @@ struct Work {
   int* len = nullptr;
   int* jstate = nullptr;
   int* fail = nullptr;
+  double* gbuf = nullptr;  // partials of the one-launch cycles (lanczos_grid.cu)
+  size_t gbuf_n = 0;
   Reducer red;
   cudaGraphExec_t graph = nullptr;
   int graph_steps = 0, graph_reorth = 0;
@@ -1453,6 +1456,9 @@ struct Work {
     cudaFree(len);
     cudaFree(jstate);
     cudaFree(fail);
+    cudaFree(gbuf);
+    gbuf = nullptr;
+    gbuf_n = 0;
     V = W = nullptr;
     R = part = npart = h = alpha = beta = coef = theta = resid = bnorm = rho = zeros = nb = nullptr;
     status = len = jstate = fail = need = nullptr;
@@ -2093,6 +2099,84 @@ std::string reset_cycle(Work<S>& w, cudaStream_t s) {
   return std::string();
 }
 
+// The one-launch Lanczos cycle of lanczos_grid.cu where it serves: the table
+// is built and a block's rows fit its shared memory.  Measured on the GB300
+// against the multi-launch steps: see there.  LGT_PANEL_GRID=0, a forced
+// H*psi kernel and FP64 reductions of FP32 panels (LGT_DF_REDUCTIONS=0) keep
+// the multi-launch steps.
+struct GridPlan {
+  bool on = false;
+  const NbrTable* T = nullptr;
+  int rpb = 0, nblk = 0, list_smem = 0, bytes = 0;
+};
+template <typename S>
+GridPlan plan_grid(OpDev* op, int64_t N, int C, int m, cudaStream_t s) {
+  GridPlan g;
+  const char* e = getenv("LGT_PANEL_GRID");
+  if ((e && e[0] == '0') || hpsi_forced() || (sizeof(S) == 4 && !df_reductions_enabled()))
+    return g;
+  if (!ensure_table(op, s)) return g;
+  g.T = op->table_ord && op->table_ord->state == 1 && op->table_ord->perm ? op->table_ord
+                                                                          : op->table;
+  g.on = lanczos_grid_plan<S>(N, C, m, g.T->mm, &g.rpb, &g.nblk, &g.list_smem, &g.bytes);
+  return g;
+}
+
+template <typename S>
+std::string run_grid_cycle(const OpDev& op, Work<S>& w, const KrylovParams& p, const GridPlan& g,
+                           double tol, double tiny_rel, cudaStream_t s, int* steps) {
+  const size_t per = size_t(w.C) * g.nblk;
+  const size_t need = (size_t(w.m) + 2) * per + (size_t(w.m) + 1) * w.C + 2;
+  if (w.gbuf_n < need) {
+    cudaFree(w.gbuf);
+    w.gbuf = nullptr;
+    w.gbuf_n = 0;
+    KCK(cudaMalloc(&w.gbuf, sizeof(double) * need));
+    w.gbuf_n = need;
+  }
+  GridArgs<S> a = {};
+  a.meta = g.T->meta;
+  a.off = g.T->tile_off;
+  a.nbr = g.T->nbr;
+  a.mm = g.T->mm;
+  a.N = w.N;
+  a.C = w.C;
+  a.rpb = g.rpb;
+  a.nblk = g.nblk;
+  a.m = w.m;
+  a.reorth = p.reorth;
+  a.check_every = p.check_every;
+  a.tol = tol;
+  a.tiny_rel = tiny_rel;
+  if constexpr (sizeof(S) == 4) {
+    a.cE = op.cE_f, a.cm = op.cm_f, a.ch = op.ch_f, a.cp = op.cp_f;
+  } else {
+    a.cE = op.cE_d, a.cm = op.cm_d, a.ch = op.ch_d, a.cp = op.cp_d;
+  }
+  a.V = w.V;
+  a.vstride = w.vstride;
+  a.alpha = w.alpha;
+  a.beta = w.beta;
+  a.ldT = w.ldT;
+  a.status = w.status;
+  a.len = w.len;
+  a.theta = w.theta;
+  a.resid = w.resid;
+  a.coef = w.coef;
+  a.bar = reinterpret_cast<unsigned*>(w.gbuf);  // counter and step count, then the sums
+  a.steps = reinterpret_cast<int*>(w.gbuf + 1);
+  a.h = w.gbuf + 2;
+  a.npart = a.h + (size_t(w.m) + 1) * w.C;
+  a.part = a.npart + per;
+  a.err = op.err;
+  a.list_smem = g.list_smem;
+  KCK(cudaMemsetAsync(w.gbuf, 0, sizeof(double), s));
+  KCK(cudaMemsetAsync(w.gbuf + 1, 0xff, sizeof(double), s));  // -1: a cycle that was cut short
+  KCK(launch_lanczos_grid<S>(a, g.bytes, s));
+  KCK(cudaMemcpyAsync(steps, a.steps, sizeof(int), cudaMemcpyDeviceToHost, s));
+  return std::string();
+}
+
 template <typename S>
 std::string ground_state_impl(const OpDev& op_in, const KrylovParams& p, Work<S>& w, double* X,
                               double* E0, double* resid_out, cudaStream_t s, KrylovReport* rep) {
@@ -2109,13 +2193,18 @@ std::string ground_state_impl(const OpDev& op_in, const KrylovParams& p, Work<S>
     w.release();
     return err;
   }
-  err = autotune<S>(&op, w, s, nullptr);
-  if (!err.empty()) return err;
+  const GridPlan grid = plan_grid<S>(&op, N, C, m, s);
+  if (grid.on) {
+    op.use_table = 1;  // the FP64 finish
+  } else {
+    err = autotune<S>(&op, w, s, nullptr);
+    if (!err.empty()) return err;
+  }
   // the Krylov vectors in the table's row order when its kernel was chosen
   // and serves these panels: X is gathered into V_0 and the combinations
   // scattered back
-  op.krylov_order = (use_krylov_order(op) && table_serves(op, w)) ? 1 : 0;
-  const int* perm = op.krylov_order ? op.table_ord->perm : nullptr;
+  op.krylov_order = (!grid.on && use_krylov_order(op) && table_serves(op, w)) ? 1 : 0;
+  const int* perm = grid.on ? grid.T->perm : op.krylov_order ? op.table_ord->perm : nullptr;
   const bool fp32 = sizeof(S) == 4;
   const double tiny_rel = fp32 ? 1e-6 : 1e-12;
   // FP32 panels cannot resolve residuals much below 1e-6 |H|: the inner
@@ -2143,15 +2232,24 @@ std::string ground_state_impl(const OpDev& op_in, const KrylovParams& p, Work<S>
   int64_t matvecs = 0;
   bool noconv = false;
   while (true) {
-    const int steps = (m - j < p.check_every) ? (m - j) : p.check_every;
-    err = run_steps<S>(op, w, p, steps, tiny_rel, s, &matvecs);
-    if (!err.empty()) return err;
-    j += steps;
-    k_check_lowest<<<K, 32, 0, s>>>(w.alpha, w.beta, w.ldT, w.status, w.len, w.theta, w.resid,
-                                    w.coef, tol_inner, fp32 ? 1 : 0), lgt::note_launch();
+    int cycle = 0;
+    if (grid.on) {
+      err = run_grid_cycle<S>(op, w, p, grid, tol_inner, tiny_rel, s, &cycle);
+      if (!err.empty()) return err;
+      j = m;
+    } else {
+      const int steps = (m - j < p.check_every) ? (m - j) : p.check_every;
+      err = run_steps<S>(op, w, p, steps, tiny_rel, s, &matvecs);
+      if (!err.empty()) return err;
+      j += steps;
+      k_check_lowest<<<K, 32, 0, s>>>(w.alpha, w.beta, w.ldT, w.status, w.len, w.theta, w.resid,
+                                      w.coef, tol_inner, fp32 ? 1 : 0), lgt::note_launch();
+    }
     KCK(cudaGetLastError());
     KCK(cudaMemcpyAsync(st.data(), w.status, sizeof(int) * K, cudaMemcpyDeviceToHost, s));
     KCK(cudaStreamSynchronize(s));
+    if (cycle < 0) return "a bounded wait of the Lanczos cycle expired";
+    matvecs += cycle;
     bool all = true;
     for (int k = 0; k < K; ++k) all = all && (st[k] >= kConverged);
     if (all) break;
