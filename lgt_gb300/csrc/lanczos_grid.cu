@@ -39,8 +39,12 @@ namespace {
 // and 16 warps with 16 to 32 loads each already cover the L2 latency (1024
 // threads with 4-vector chunks: dots 122k cycles a step at 4x3 K = 16 and
 // 66k at K = 1, most of it those sums).
-constexpr int kNT = 512;
-constexpr int kNW = kNT / 32;
+template <typename S>
+struct Threads {
+  // FP64: 168 registers a thread, so that the loads ahead do not spill (L1 has
+  // what shared memory leaves)
+  static constexpr int n = sizeof(S) == 4 ? 512 : 384;
+};
 constexpr int kQ = 8;               // basis vectors per dot chunk
 constexpr int kSmemMax = 214 * 1024;  // beside the static arrays
 constexpr long long kGridSpinCycles = 8000000000LL;  // ~4 s: another kernel may hold SMs
@@ -66,11 +70,12 @@ struct Layout {
 };
 template <typename S>
 __host__ __device__ inline Layout layout(int rpb, int C, int m, int mm, int list_smem) {
+  constexpr int kNT = Threads<S>::n;
   auto up = [](int b) { return (b + 15) / 16 * 16; };
   Layout L;
   int o = 0;
   L.W = o;
-  o += up(rpb * C * int(sizeof(S)));
+  o += up(rpb * C * 8);  // FP32: the leading parts, then the trailing ones
   L.list = o;
   o += list_smem ? up(rpb * mm * 4) : 0;
   L.meta = o;
@@ -90,21 +95,24 @@ __host__ __device__ inline Layout layout(int rpb, int C, int m, int mm, int list
 }
 
 template <typename S>
-__global__ void __launch_bounds__(kNT, 1) k_lanczos_grid(GridArgs<S> a) {
+__global__ void __launch_bounds__(Threads<S>::n, 1) k_lanczos_grid(GridArgs<S> a) {
+  constexpr int kNT = Threads<S>::n, kNW = kNT / 32;
   constexpr bool kDF = sizeof(S) == 4;
-  constexpr int kU = kDF ? 4 : 2;  // rows per trip
+  constexpr int kU = kDF ? 2 : 1;  // rows per trip
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ int s_n, s_bad;
   __shared__ S s_int[256], s_stag[256];  // small integers: conversions to FP64 are slow
   __shared__ double s_ta[kTriMax], s_tb[kTriMax], s_tz[kTriMax], s_work[3 * kTriMax];
   const Layout L = layout<S>(a.rpb, a.C, a.m, a.mm, a.list_smem);
   S* s_W = reinterpret_cast<S*>(smem + L.W);
+  S* s_lo = s_W + a.rpb * a.C;  // (FP32 only)
   uint32_t* s_list = reinterpret_cast<uint32_t*>(smem + L.list);
   uint32_t* s_meta = reinterpret_cast<uint32_t*>(smem + L.meta);
   uint32_t* s_loff = reinterpret_cast<uint32_t*>(smem + L.loff);
   double* s_h = reinterpret_cast<double*>(smem + L.h);
   float* s_hh = reinterpret_cast<float*>(smem + L.h);
   const int C = a.C, m = a.m;
+  const uint32_t vs = uint32_t(a.vstride);  // (m + 1) N C < 2^32: the plan checks it
   float* s_hl = s_hh + m * C;
   using Acc = typename std::conditional<kDF, df, double>::type;  // running sums
   Acc* s_red = reinterpret_cast<Acc*>(smem + L.red);
@@ -173,7 +181,7 @@ __global__ void __launch_bounds__(kNT, 1) k_lanczos_grid(GridArgs<S> a) {
     __syncthreads();
     const int nout = nq * nl;
     int LN = 32;
-    while (LN > 1 && nout * LN > kNT) LN >>= 1;
+    while (LN > 1 && nout * LN > kNT) LN >>= 1;  // (LN divides a warp)
     for (int o0 = 0; o0 < nout; o0 += kNT / LN) {
       const int o = o0 + tid / LN;
       const int q = o / nl, ci = o - q * nl;
@@ -281,73 +289,60 @@ __global__ void __launch_bounds__(kNT, 1) k_lanczos_grid(GridArgs<S> a) {
       // ---- dots against V_0 .. V_j (and W itself in the first pass)
       for (int i0 = 0; i0 < J; i0 += kQ) {
         const bool self = pass == 0 && i0 == 0;
-        if constexpr (kDF) {
-          df acc[kQ], ss{0.f, 0.f};
+        if (on) {
+          Acc acc[kQ], ss = zero();
 #pragma unroll
-          for (int q = 0; q < kQ; ++q) acc[q] = df{0.f, 0.f};
-          if (on) {
-            const float* vq[kQ];
-#pragma unroll
-            for (int q = 0; q < kQ; ++q)
-              vq[q] = reinterpret_cast<const float*>(Vc) +
-                      size_t(i0 + q < J ? i0 + q : J - 1) * a.vstride;
-            for (int r = rg; r < nr; r += kU * RG) {
-              float w[kU], v[kQ][kU];  // rows past the block's count as zeros
-#pragma unroll
-              for (int u = 0; u < kU; ++u) w[u] = r + u * RG < nr ? s_W[(r + u * RG) * C + c] : 0.f;
-#pragma unroll
-              for (int q = 0; q < kQ; ++q)
-#pragma unroll
-                for (int u = 0; u < kU; ++u)
-                  v[q][u] = (i0 + q < J && r + u * RG < nr) ? vq[q][(r + u * RG) * C] : 0.f;
-#pragma unroll
-              for (int q = 0; q < kQ; ++q)
-                if (i0 + q < J) {
-#pragma unroll
-                  for (int u = 0; u < kU; ++u) df_fma(acc[q], v[q][u], w[u]);
-                }
-              if (self) {
-#pragma unroll
-                for (int u = 0; u < kU; ++u) df_fma(ss, w[u], w[u]);
-              }
-            }
-#pragma unroll
-            for (int q = 0; q < kQ; ++q) s_red[q * kNT + tid] = acc[q];
-            if (self) s_red[kQ * kNT + tid] = ss;
-          }
-        } else {
-          double acc[kQ], ss = 0.0;
-#pragma unroll
-          for (int q = 0; q < kQ; ++q) acc[q] = 0.0;
-          if (on) {
-            const S* vq[kQ];
+          for (int q = 0; q < kQ; ++q) acc[q] = zero();
+          // rows r, r + RG, ... (kU at once); those past the block's count as
+          // zeros
+          auto load = [&](int r, S(&v)[kQ][kU]) {
 #pragma unroll
             for (int q = 0; q < kQ; ++q)
-              vq[q] = Vc + size_t(i0 + q < J ? i0 + q : J - 1) * a.vstride;
-            for (int r = rg; r < nr; r += kU * RG) {
-              double w[kU], v[kQ][kU];
 #pragma unroll
-              for (int u = 0; u < kU; ++u) w[u] = r + u * RG < nr ? s_W[(r + u * RG) * C + c] : S(0);
+              for (int u = 0; u < kU; ++u)
+                v[q][u] = (i0 + q < J && r + u * RG < nr)
+                              ? Vc[uint32_t(i0 + q) * vs + uint32_t((r + u * RG) * C)]
+                              : S(0);
+          };
+          auto use = [&](int r, const S(&v)[kQ][kU]) {
+            S w[kU];
 #pragma unroll
-              for (int q = 0; q < kQ; ++q)
+            for (int u = 0; u < kU; ++u) w[u] = r + u * RG < nr ? s_W[(r + u * RG) * C + c] : S(0);
 #pragma unroll
-                for (int u = 0; u < kU; ++u)
-                  v[q][u] = (i0 + q < J && r + u * RG < nr) ? vq[q][(r + u * RG) * C] : S(0);
+            for (int q = 0; q < kQ; ++q)
+              if (i0 + q < J) {
 #pragma unroll
-              for (int q = 0; q < kQ; ++q)
-                if (i0 + q < J) {
-#pragma unroll
-                  for (int u = 0; u < kU; ++u) acc[q] = fma(v[q][u], w[u], acc[q]);
+                for (int u = 0; u < kU; ++u) {
+                  if constexpr (kDF) df_fma(acc[q], v[q][u], w[u]);
+                  else acc[q] = fma(v[q][u], w[u], acc[q]);
                 }
-              if (self) {
+              }
+            if (self) {
 #pragma unroll
-                for (int u = 0; u < kU; ++u) ss = fma(w[u], w[u], ss);
+              for (int u = 0; u < kU; ++u) {
+                if constexpr (kDF) df_fma(ss, w[u], w[u]);
+                else ss = fma(w[u], w[u], ss);
               }
             }
-#pragma unroll
-            for (int q = 0; q < kQ; ++q) s_red[q * kNT + tid] = acc[q];
-            if (self) s_red[kQ * kNT + tid] = ss;
+          };
+          // the next rows' loads are issued before the current rows'
+          // arithmetic: the warps of a block run in step, so nothing else
+          // covers their latency
+          S va[kQ][kU], vb[kQ][kU];
+          int r = rg;
+          if (r < nr) load(r, va);
+          while (r < nr) {
+            const int r2 = r + kU * RG, r3 = r2 + kU * RG;
+            if (r2 < nr) load(r2, vb);
+            use(r, va);
+            if (r2 >= nr) break;
+            if (r3 < nr) load(r3, va);
+            use(r2, vb);
+            r = r3;
           }
+#pragma unroll
+          for (int q = 0; q < kQ; ++q) s_red[q * kNT + tid] = acc[q];
+          if (self) s_red[kQ * kNT + tid] = ss;
         }
         // slot kQ (the self-dot) goes to row J of the partials
         const int nv = J - i0 < kQ ? J - i0 : kQ;
@@ -387,76 +382,80 @@ __global__ void __launch_bounds__(kNT, 1) k_lanczos_grid(GridArgs<S> a) {
       }
       __syncthreads();
       // ---- W -= sum_i h_i V_i, and |W|^2
-      Acc n2 = zero();
       if (on) {
-        if constexpr (kDF) {
-          df& nrm = n2;
-          const float* Vf = reinterpret_cast<const float*>(Vc);
-          auto one = [&](float& hi, float& lo, float hh, float hl, float x) {
-            float p, e, t;
-            two_prod(hh, x, p, e);
-            e = df_fma_rn(hl, x, e);
-            two_sum(hi, -p, hi, t);
-            lo = df_add_rn(lo, df_sub_rn(t, e));
+        Acc n2 = zero();
+        // eight vectors at a time, the latest first (the dots read them last,
+        // so they are what L2 still holds), W in shared memory between the
+        // groups -- with its trailing part in FP32
+        for (int i = (J - 1) / 8 * 8; i >= 0; i -= 8) {
+          const bool first = i + 8 >= J, last = i == 0;
+          auto load = [&](int r, S(&x)[8][kU]) {
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+#pragma unroll
+              for (int u = 0; u < kU; ++u)
+                x[q][u] = (i + q < J && r + u * RG < nr)
+                              ? Vc[uint32_t(i + q) * vs + uint32_t((r + u * RG) * C)]
+                              : S(0);
           };
-          for (int r = rg; r < nr; r += kU * RG) {
-            float hi[kU], lo[kU];
+          auto use = [&](int r, const S(&x)[8][kU]) {
+            S hi[kU], lo[kU];
 #pragma unroll
             for (int u = 0; u < kU; ++u) {
-              hi[u] = r + u * RG < nr ? s_W[(r + u * RG) * C + c] : 0.f;
-              lo[u] = 0.f;
+              const int at = (r + u * RG) * C + c;
+              const bool in = r + u * RG < nr;
+              hi[u] = in ? s_W[at] : S(0);
+              lo[u] = S(0);
+              if (kDF && in && !first) lo[u] = s_lo[at];
             }
-            for (int i = 0; i < J; i += 8) {
-              float x[8][kU];
 #pragma unroll
-              for (int q = 0; q < 8; ++q)
-#pragma unroll
-                for (int u = 0; u < kU; ++u)
-                  x[q][u] = (i + q < J && r + u * RG < nr)
-                                ? Vf[size_t(i + q) * a.vstride + (r + u * RG) * C]
-                                : 0.f;
-#pragma unroll
-              for (int q = 0; q < 8; ++q)
-                if (i + q < J) {
+            for (int q = 0; q < 8; ++q)
+              if (i + q < J) {
+                if constexpr (kDF) {
                   const float hh = s_hh[(i + q) * C + c], hl = s_hl[(i + q) * C + c];
 #pragma unroll
-                  for (int u = 0; u < kU; ++u) one(hi[u], lo[u], hh, hl, x[q][u]);
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < kU; ++u) {
-              const float w = df_add_rn(hi[u], lo[u]);
-              if (r + u * RG < nr) s_W[(r + u * RG) * C + c] = w;
-              df_fma(nrm, w, w);
-            }
-          }
-        } else {
-          for (int r = rg; r < nr; r += kU * RG) {
-            double w[kU];
-#pragma unroll
-            for (int u = 0; u < kU; ++u) w[u] = r + u * RG < nr ? s_W[(r + u * RG) * C + c] : S(0);
-            for (int i = 0; i < J; i += 8) {
-              double x[8][kU];
-#pragma unroll
-              for (int q = 0; q < 8; ++q)
-#pragma unroll
-                for (int u = 0; u < kU; ++u)
-                  x[q][u] = (i + q < J && r + u * RG < nr)
-                                ? Vc[size_t(i + q) * a.vstride + (r + u * RG) * C]
-                                : S(0);
-#pragma unroll
-              for (int q = 0; q < 8; ++q)
-                if (i + q < J) {
+                  for (int u = 0; u < kU; ++u) {
+                    float p, e, t;
+                    two_prod(hh, x[q][u], p, e);
+                    e = df_fma_rn(hl, x[q][u], e);
+                    two_sum(hi[u], -p, hi[u], t);
+                    lo[u] = df_add_rn(lo[u], df_sub_rn(t, e));
+                  }
+                } else {  // two chains: even and odd vectors
                   const double h = s_h[(i + q) * C + c];
 #pragma unroll
-                  for (int u = 0; u < kU; ++u) w[u] = fma(-h, x[q][u], w[u]);
+                  for (int u = 0; u < kU; ++u) {
+                    if (q & 1) lo[u] = fma(-h, x[q][u], lo[u]);
+                    else hi[u] = fma(-h, x[q][u], hi[u]);
+                  }
                 }
-            }
+              }
 #pragma unroll
             for (int u = 0; u < kU; ++u) {
-              if (r + u * RG < nr) s_W[(r + u * RG) * C + c] = S(w[u]);
-              n2 = fma(w[u], w[u], n2);
+              const int at = (r + u * RG) * C + c;
+              S w = hi[u];
+              if (!kDF || last) w = hi[u] + lo[u];
+              if (r + u * RG < nr) {
+                s_W[at] = w;
+                if (kDF && !last) s_lo[at] = lo[u];
+              }
+              if (last) {
+                if constexpr (kDF) df_fma(n2, w, w);
+                else n2 = fma(w, w, n2);
+              }
             }
+          };
+          S xa[8][kU], xb[8][kU];
+          int r = rg;
+          if (r < nr) load(r, xa);
+          while (r < nr) {
+            const int r2 = r + kU * RG, r3 = r2 + kU * RG;
+            if (r2 < nr) load(r2, xb);
+            use(r, xa);
+            if (r2 >= nr) break;
+            if (r3 < nr) load(r3, xa);
+            use(r2, xb);
+            r = r3;
           }
         }
         s_red[tid] = n2;
@@ -581,7 +580,8 @@ bool lanczos_grid_plan(int64_t N, int C, int m, int mm, int* rpb, int* nblk, int
     return false;
   if (N < 1 || C < 1 || C > 256 || m < 1 || m >= kTriMax) return false;
   const int64_t rows = ((N + sms - 1) / sms + 31) / 32 * 32;
-  if (rows * C > kSmemMax / int(sizeof(S)) || rows > kSmemMax / 8) return false;
+  if ((m + 1) * N * C >= (int64_t(1) << 32)) return false;
+  if (rows * C > kSmemMax / 8 || rows > kSmemMax / 8) return false;
   for (int ls = 1; ls >= 0; --ls) {
     if (ls && rows * mm > kSmemMax / 4) continue;
     const Layout L = layout<S>(int(rows), C, m, mm, ls);
@@ -604,7 +604,7 @@ cudaError_t launch_lanczos_grid(const GridArgs<S>& a, int bytes, cudaStream_t s)
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(unsigned(a.nblk));
-  cfg.blockDim = dim3(kNT);
+  cfg.blockDim = dim3(Threads<S>::n);
   cfg.dynamicSmemBytes = size_t(bytes);
   cfg.stream = s;
   cudaLaunchAttribute at[1];
