@@ -261,8 +261,8 @@ bool hpsi_fixed_applies(const HpsiArgs<T>& a, int* max_vpl) {
   const Geom& G = a.G;
   const bool shape = (G.nx == 4 && G.ny == 4) || (G.nx == 4 && G.ny == 3) ||
                      (G.nx == 3 && G.ny == 4);
-  const bool ok = shape && G.dg == 1 && a.R.tab && a.N < (int64_t(1) << 31) && vec_ok(a);
-  const bool two = a.C % (2 * (16 / int(sizeof(T)))) == 0;
+  const bool ok = shape && G.dg == 1 && a.R.tab && a.N < (int64_t(1) << 31);
+  const bool two = vec_ok(a) && a.C % (2 * (16 / int(sizeof(T)))) == 0;
   const bool wide = two && (reinterpret_cast<uintptr_t>(a.x) & 31) == 0 &&
                     (reinterpret_cast<uintptr_t>(a.y) & 31) == 0 &&
                     (a.xsel == nullptr || (a.xstride * sizeof(T)) % 32 == 0);

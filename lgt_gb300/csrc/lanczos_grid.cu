@@ -28,6 +28,7 @@
 
 #include "lgt_dfloat.cuh"
 #include "lgt_internal.h"
+#include "lgt_intsum.cuh"
 #include "lgt_lanczos_grid.h"
 #include "lgt_tridiag.cuh"
 
@@ -59,9 +60,6 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
 
 __device__ __forceinline__ float flip(float v, uint32_t ent) {
   return __uint_as_float(__float_as_uint(v) ^ (ent & 0x80000000u));
-}
-__device__ __forceinline__ double flip(double v, uint32_t ent) {
-  return __hiloint2double(__double2hiint(v) ^ int(ent & 0x80000000u), __double2loint(v));
 }
 
 // Shared-memory layout of a block.
@@ -254,21 +252,32 @@ __global__ void __launch_bounds__(Threads<S>::n, 1) k_lanczos_grid(GridArgs<S> a
           const uint32_t* l = list + s_loff[r];
           const S xd = Vj[size_t(r0 + r) * C + c];
           S sh = S(0), sp = S(0);
-          for (int n = 0; n < n1; n += 8) {
-            S v[8];
-            uint32_t ent[8];
+          if constexpr (!kDF) {
+            double t[1];
+            auto load = [&](uint32_t i, double(&v)[1]) { v[0] = Vj[size_t(i) * C + c]; };
+            int_sum<1, 8, true>(l, 0, nh, t, load);
+            sh = t[0];
+            if (n1 > nh) {
+              int_sum<1, 8, false>(l, nh, n1, t, load);
+              sp = t[0];
+            }
+          } else {
+            for (int n = 0; n < n1; n += 8) {
+              S v[8];
+              uint32_t ent[8];
 #pragma unroll
-            for (int u = 0; u < 8; ++u)
-              if (n + u < n1) {
-                ent[u] = l[n + u];
-                v[u] = Vj[size_t(ent[u] & 0x7fffffffu) * C + c];
-              }
+              for (int u = 0; u < 8; ++u)
+                if (n + u < n1) {
+                  ent[u] = l[n + u];
+                  v[u] = Vj[size_t(ent[u] & 0x7fffffffu) * C + c];
+                }
 #pragma unroll
-            for (int u = 0; u < 8; ++u)
-              if (n + u < n1) {
-                if (n + u < nh) sh += flip(v[u], ent[u]);
-                else sp += v[u];
-              }
+              for (int u = 0; u < 8; ++u)
+                if (n + u < n1) {
+                  if (n + u < nh) sh += flip(v[u], ent[u]);
+                  else sp += v[u];
+                }
+            }
           }
           const S cd = fma(cE, s_int[(mw >> 16) & 255u], cm * s_stag[mw >> 24]);
           S y = fma(ch, sh, cd * xd);

@@ -93,7 +93,8 @@ template <typename T>
 cudaError_t launch_hpsi_table(const HpsiArgs<T>& a, uint32_t model, cudaStream_t s);
 
 // Whether a fixed-shape kernel serves these arguments, and the widest load
-// mode it may use (1, 2 when C is a multiple of two vectors, 3 when the
+// mode it may use (1: one vector, or single elements where width or
+// alignment take none; 2 when C is a multiple of two vectors, 3 when the
 // panels are also 32-byte aligned).
 template <typename T>
 bool hpsi_fixed_applies(const HpsiArgs<T>& a, int* max_vpl);
@@ -103,7 +104,7 @@ int hpsi_seg_smem_default(int nmasks);
 
 // y = H x.  With use_table and a table present, the stored-table kernel;
 // else lattices with a compile-time kernel (4x4, 4x3, 3x4 at dg = 1, rank
-// tables present, vector-aligned panels) use it; all others the
+// tables present) use it; all others the
 // run-time-geometry kernel.  All give the same product.
 template <typename T>
 cudaError_t launch_hpsi(HpsiArgs<T> a, uint32_t model, cudaStream_t s);

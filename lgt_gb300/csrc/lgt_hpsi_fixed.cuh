@@ -105,7 +105,7 @@ __device__ __forceinline__ uint32_t rank_fixed(const uint32_t* __restrict__ tab,
 }
 
 template <int NX, int NY, typename T, int LD, bool PLAQ, bool JW>
-__global__ void __launch_bounds__(kThreads, PLAQ ? LGT_FIXED_MINB_PLAQ : LGT_FIXED_MINB)
+__global__ void __launch_bounds__(kThreads, PLAQ || sizeof(T) == 8 ? LGT_FIXED_MINB_PLAQ : LGT_FIXED_MINB)
     k_hpsi_fixed(HpsiArgs<T> a) {
   using S = Shape<NX, NY>;
   constexpr int MM = list_stride<NX, NY, PLAQ>();
@@ -251,8 +251,7 @@ __global__ void __launch_bounds__(kThreads, PLAQ ? LGT_FIXED_MINB_PLAQ : LGT_FIX
 }
 
 // Launches the fixed-shape kernel for (NX, NY); the caller has checked
-// dg == 1, rank tables present, N < 2^31, C % (16 / sizeof(T)) == 0 and
-// 16-byte aligned panels.
+// dg == 1, rank tables present and N < 2^31.
 template <int NX, int NY, typename T, int LD, bool PLAQ, bool JW>
 cudaError_t launch_shape_v(const HpsiArgs<T>& a, cudaStream_t s) {
   auto kern = k_hpsi_fixed<NX, NY, T, LD, PLAQ, JW>;
@@ -269,10 +268,17 @@ cudaError_t launch_shape_v(const HpsiArgs<T>& a, cudaStream_t s) {
 
 // Load mode: a.vpl = 1 one vector per lane, 2 two vectors, 3 two vectors as
 // one 32-byte access; 0 the built-in rule (two vectors when C allows).  A mode
-// the panel cannot take falls back to the next narrower one.
+// the panel cannot take falls back to the next narrower one, down to single
+// elements for odd widths and unaligned panels (4x3 K = 5 FP64 with
+// plaquettes: the run-time-geometry kernel, their only one before, took 44
+// us).
 template <int NX, int NY, typename T, bool PLAQ, bool JW>
 cudaError_t launch_shape_m(const HpsiArgs<T>& a, cudaStream_t s) {
   constexpr int V = 16 / int(sizeof(T));
+  const bool vec = a.C % V == 0 && (reinterpret_cast<uintptr_t>(a.x) & 15) == 0 &&
+                   (reinterpret_cast<uintptr_t>(a.y) & 15) == 0 &&
+                   (a.xsel == nullptr || (a.xstride * sizeof(T)) % 16 == 0);
+  if (!vec) return launch_shape_v<NX, NY, T, 0, PLAQ, JW>(a, s);
   const bool two = a.C % (2 * V) == 0;
   // 32-byte accesses: panels and the Krylov panel stride keep every row
   // slice 32-byte aligned

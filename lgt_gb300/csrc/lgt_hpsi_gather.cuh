@@ -5,7 +5,8 @@
 //
 // Lanes run over (row, W-column slice) of the warp's 32 rows: each of a
 // row's lanes loads one or two vectors of V elements per neighbour (LD = 1,
-// 2), or two vectors as one 32-byte access (LD = 4), sums the hop
+// 2), two vectors as one 32-byte access (LD = 4), or one element where the
+// width or alignment takes no vectors (LD = 0), sums the hop
 // neighbours (times the Jordan-Wigner sign) and the plaquette neighbours in
 // two accumulators, and applies the couplings once per row:
 //   y = (cE e2 + cm stag) x_row + ch * sum_hops (+-) x_j + cp * sum_plaq x_j
@@ -13,16 +14,17 @@
 #pragma once
 
 #include "lgt_hpsi.h"
+#include "lgt_intsum.cuh"
 
 namespace lgt {
 namespace gather {
 
 // Neighbour rows gathered per loop trip: measured on the 4x4 lattice, K = 8
 // complex, 8 rows in flight for FP32 (the table kernel: 0.757 -> 0.714 ms
-// against 4; the fixed-shape kernel is indifferent), 2 for FP64 (bound by
-// the FP64 pipe, not by latency; 8 costs 15%).
+// against 4; the fixed-shape kernel is indifferent).  FP64 sums run in
+// integers (lgt_intsum.cuh), 8 columns in flight.
 #ifndef LGT_GATHER_UNROLL
-#define LGT_GATHER_UNROLL (sizeof(T) == 4 ? 8 : 2)
+#define LGT_GATHER_UNROLL 8
 #endif
 
 // Per-row meta word of a neighbour list: entry count, hop count (hops come
@@ -99,8 +101,10 @@ __device__ __forceinline__ void st32(double* p, const double* r) {
 // vectors as one 32-byte access.
 template <typename T, int V, int LD>
 __device__ __forceinline__ void ld_slice(const T* p, T* r) {
-  if (LD == 4) {
+  if constexpr (LD == 4) {
     ld32(p, r);
+  } else if constexpr (LD == 0) {
+    r[0] = __ldg(p);
   } else {
 #pragma unroll
     for (int q = 0; q < LD; ++q) ld<T, V>(p + q * V, r + q * V);
@@ -108,8 +112,10 @@ __device__ __forceinline__ void ld_slice(const T* p, T* r) {
 }
 template <typename T, int V, int LD>
 __device__ __forceinline__ void st_slice(T* p, const T* r) {
-  if (LD == 4) {
+  if constexpr (LD == 4) {
     st32(p, r);
+  } else if constexpr (LD == 0) {
+    __stcs(p, r[0]);
   } else {
 #pragma unroll
     for (int q = 0; q < LD; ++q) st<T, V>(p + q * V, r + q * V);
@@ -124,7 +130,7 @@ template <typename T, int LD, bool PLAQ, bool JW, class List>
 __device__ __forceinline__ void gather_rows(const HpsiArgs<T>& a, int64_t warp_row0, int lane,
                                             const uint32_t* s_meta, const T* s_coef, List list) {
   constexpr int V = 16 / int(sizeof(T));
-  constexpr int W = V * (LD == 1 ? 1 : 2);  // columns per lane
+  constexpr int W = LD == 0 ? 1 : V * (LD == 1 ? 1 : 2);  // columns per lane
   const int K = a.K;
   const int C = a.C;
   const int lpr = C / W;  // lanes per row (C % W == 0 on the host)
@@ -143,7 +149,7 @@ __device__ __forceinline__ void gather_rows(const HpsiArgs<T>& a, int64_t warp_r
     const int cnt = int(m & 255u), nh = int((m >> 8) & 255u);
     const T e2 = T(int((m >> 16) & 255u)), stag = T(int(m >> 24) - 128);
     const uint32_t* lst = list(rl);
-    T ah[W], ap[W], xd[W], xs[LGT_GATHER_UNROLL][W];
+    T ah[W], ap[W], xd[W];
     const T* px = x + size_t(row) * C + col0;
     ld_slice<T, V, LD>(px, xd);
 #pragma unroll
@@ -151,47 +157,57 @@ __device__ __forceinline__ void gather_rows(const HpsiArgs<T>& a, int64_t warp_r
       ah[e] = T(0);
       ap[e] = T(0);
     }
-    // LGT_GATHER_UNROLL neighbour rows in flight per trip; the tail trip
-    // gathers only the rows that exist and adds zeros for the rest
-    for (int n = 0; n < nh; n += LGT_GATHER_UNROLL) {
-      uint32_t ent[LGT_GATHER_UNROLL];
-#pragma unroll
-      for (int u = 0; u < LGT_GATHER_UNROLL; ++u) {
-        ent[u] = (n + u < nh) ? lst[n + u] : 0u;
-        if (n + u < nh) {
-          ld_slice<T, V, LD>(x + size_t(ent[u] & 0x7fffffffu) * C + col0, xs[u]);
-        } else {
-#pragma unroll
-          for (int e = 0; e < W; ++e) xs[u][e] = T(0);
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < LGT_GATHER_UNROLL; ++u) {
-        if (JW) {
-          const T sg = (ent[u] >> 31) ? T(-1) : T(1);
-#pragma unroll
-          for (int e = 0; e < W; ++e) ah[e] = fma(sg, xs[u][e], ah[e]);
-        } else {
-#pragma unroll
-          for (int e = 0; e < W; ++e) ah[e] += xs[u][e];
-        }
-      }
-    }
-    if (PLAQ) {
-      for (int n = nh; n < cnt; n += LGT_GATHER_UNROLL) {
+    if constexpr (sizeof(T) == 8) {
+      constexpr int U = 8 / W;
+      auto load = [&](uint32_t j, double(&v)[W]) {
+        ld_slice<T, V, LD>(x + size_t(j) * C + col0, v);
+      };
+      int_sum<W, U, JW>(lst, 0, nh, ah, load);
+      if (PLAQ) int_sum<W, U, false>(lst, nh, cnt, ap, load);
+    } else {
+      T xs[LGT_GATHER_UNROLL][W];
+      // LGT_GATHER_UNROLL neighbour rows in flight per trip; the tail trip
+      // gathers only the rows that exist and adds zeros for the rest
+      for (int n = 0; n < nh; n += LGT_GATHER_UNROLL) {
+        uint32_t ent[LGT_GATHER_UNROLL];
 #pragma unroll
         for (int u = 0; u < LGT_GATHER_UNROLL; ++u) {
-          if (n + u < cnt) {
-            ld_slice<T, V, LD>(x + size_t(lst[n + u]) * C + col0, xs[u]);
+          ent[u] = (n + u < nh) ? lst[n + u] : 0u;
+          if (n + u < nh) {
+            ld_slice<T, V, LD>(x + size_t(ent[u] & 0x7fffffffu) * C + col0, xs[u]);
           } else {
 #pragma unroll
             for (int e = 0; e < W; ++e) xs[u][e] = T(0);
           }
         }
 #pragma unroll
-        for (int u = 0; u < LGT_GATHER_UNROLL; ++u)
+        for (int u = 0; u < LGT_GATHER_UNROLL; ++u) {
+          if (JW) {
+            const T sg = (ent[u] >> 31) ? T(-1) : T(1);
 #pragma unroll
-          for (int e = 0; e < W; ++e) ap[e] += xs[u][e];
+            for (int e = 0; e < W; ++e) ah[e] = fma(sg, xs[u][e], ah[e]);
+          } else {
+#pragma unroll
+            for (int e = 0; e < W; ++e) ah[e] += xs[u][e];
+          }
+        }
+      }
+      if (PLAQ) {
+        for (int n = nh; n < cnt; n += LGT_GATHER_UNROLL) {
+#pragma unroll
+          for (int u = 0; u < LGT_GATHER_UNROLL; ++u) {
+            if (n + u < cnt) {
+              ld_slice<T, V, LD>(x + size_t(lst[n + u]) * C + col0, xs[u]);
+            } else {
+#pragma unroll
+              for (int e = 0; e < W; ++e) xs[u][e] = T(0);
+            }
+          }
+#pragma unroll
+          for (int u = 0; u < LGT_GATHER_UNROLL; ++u)
+#pragma unroll
+            for (int e = 0; e < W; ++e) ap[e] += xs[u][e];
+        }
       }
     }
     // y = (cE e2 + cm stag) x + ch * hops (+ cp * plaquettes); the diagonal

@@ -16,6 +16,7 @@
 
 #include "lgt_hpsi.h"
 #include "lgt_hpsi_gather.cuh"
+#include "lgt_intsum.cuh"
 
 namespace lgt {
 namespace rows {
@@ -78,22 +79,20 @@ __device__ __forceinline__ void st_cols(T* p, const T (&r)[W]) {
   }
 }
 
-// s = the sum of the slices of entries lst[n0 .. n1), U of them in flight;
-// SGN: bit 31 of an entry flips the sign.  The last trip of an FP32 sum adds
-// zeros for the entries it lacks; FP64 sums, bound by the FP64 pipe, finish
-// entry by entry instead.
+// s = the sum of the slices of entries lst[n0 .. n1), U of them in flight (the
+// last trip adds zeros for the entries it lacks); SGN: bit 31 of an entry
+// flips the sign.
 template <typename T, int W, int U, bool SGN>
 __device__ __forceinline__ void sum_slices(const T* x, int C, int col0, const uint32_t* lst,
                                            int n0, int n1, T (&s)[W]) {
 #pragma unroll
   for (int e = 0; e < W; ++e) s[e] = T(0);
-  int n = n0;
-  for (; sizeof(T) == 4 ? n < n1 : n + U <= n1; n += U) {
+  for (int n = n0; n < n1; n += U) {
     T v[U][W];
     uint32_t ent[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      if (sizeof(T) == 8 || n + u < n1) {
+      if (n + u < n1) {
         ent[u] = lst[n + u];
         ld_cols<T, W>(x + size_t(ent[u] & 0x7fffffffu) * C + col0, v[u]);
       } else {
@@ -108,15 +107,18 @@ __device__ __forceinline__ void sum_slices(const T* x, int C, int col0, const ui
       for (int e = 0; e < W; ++e)
         s[e] = SGN ? fma((ent[u] >> 31) ? T(-1) : T(1), v[u][e], s[e]) : s[e] + v[u][e];
   }
-  if (sizeof(T) == 8)
-    for (; n < n1; ++n) {
-      T v[W];
-      const uint32_t ent = lst[n];
-      ld_cols<T, W>(x + size_t(ent & 0x7fffffffu) * C + col0, v);
-#pragma unroll
-      for (int e = 0; e < W; ++e)
-        s[e] = SGN ? fma((ent >> 31) ? T(-1) : T(1), v[e], s[e]) : s[e] + v[e];
-    }
+}
+
+// A row's sum over entries lst[n0 .. n1) in T: FP64 by integers.
+template <typename T, int W, int U, bool SGN>
+__device__ __forceinline__ void sum_entries(const T* x, int C, int col0, const uint32_t* lst,
+                                            int n0, int n1, T (&s)[W]) {
+  if constexpr (sizeof(T) == 8)
+    int_sum<W, U, SGN>(lst, n0, n1, s, [&](uint32_t j, double(&v)[W]) {
+      ld_cols<double, W>(x + size_t(j) * C + col0, v);
+    });
+  else
+    sum_slices<T, W, U, SGN>(x, C, col0, lst, n0, n1, s);
 }
 
 __host__ __device__ inline int coef_words(bool cheb, int K) { return (cheb ? 5 : 4) * K; }
@@ -137,7 +139,7 @@ __device__ __forceinline__ int incl_scan(int v, int lane) {
 }
 
 template <typename T, int W, int U, bool PLAQ, bool JW, bool CHEB>
-__global__ void __launch_bounds__(kThreads, PLAQ ? 4 : 5) k_table_rows(Args<T> a) {
+__global__ void __launch_bounds__(kThreads, PLAQ || sizeof(T) == 8 ? 4 : 5) k_table_rows(Args<T> a) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int K = a.K, C = a.C;
   T* s_coef = reinterpret_cast<T*>(smem);
@@ -185,7 +187,7 @@ __global__ void __launch_bounds__(kThreads, PLAQ ? 4 : 5) k_table_rows(Args<T> a
     const size_t at = size_t(row) * C + col0;
     T xd[W], ah[W], out[W];
     ld_cols<T, W>(x + at, xd);
-    sum_slices<T, W, U, JW>(x, C, col0, l, 0, nh, ah);
+    sum_entries<T, W, U, JW>(x, C, col0, l, 0, nh, ah);
 #pragma unroll
     for (int e = 0; e < W; ++e) {
       const int k = a.ncomp == 2 ? (col0 + e) >> 1 : col0 + e;
@@ -194,7 +196,7 @@ __global__ void __launch_bounds__(kThreads, PLAQ ? 4 : 5) k_table_rows(Args<T> a
       out[e] = fma(s_coef[2 * K + k], ah[e], cd * xd[e]);
     }
     if (PLAQ) {
-      sum_slices<T, W, U, false>(x, C, col0, l, nh, n1, ah);
+      sum_entries<T, W, U, false>(x, C, col0, l, nh, n1, ah);
 #pragma unroll
       for (int e = 0; e < W; ++e) {
         const int k = a.ncomp == 2 ? (col0 + e) >> 1 : col0 + e;

@@ -165,7 +165,7 @@ __host__ __device__ inline int table_smem(int K, int mm) {
 // warp scan of their counts gives each row's list offset) and the tile's
 // entries are copied into shared memory, then the gather phase runs.
 template <typename T, int LD, bool PLAQ, bool JW>
-__global__ void __launch_bounds__(kTabThreads, PLAQ ? LGT_TABLE_MINB_PLAQ : LGT_TABLE_MINB)
+__global__ void __launch_bounds__(kTabThreads, PLAQ || sizeof(T) == 8 ? LGT_TABLE_MINB_PLAQ : LGT_TABLE_MINB)
     k_hpsi_table(HpsiArgs<T> a) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int K = a.K;
