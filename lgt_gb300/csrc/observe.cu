@@ -24,6 +24,7 @@
 #include <type_traits>
 
 #include "lgt_dfloat.cuh"
+#include "lgt_hpsi_fixed.cuh"
 #include "lgt_observe.h"
 #include "lgt_rank.cuh"
 
@@ -44,17 +45,16 @@ __device__ __forceinline__ df split_df(double d) {
   const uint32_t sign = uh & 0x80000000u;
   const int e = int((uh >> 20) & 0x7ffu);
   const int e32 = e - 896;  // FP32 biased exponent of the leading bit
-  if (e32 <= 0 || e32 >= 255) return df{0.f, 0.f};
+  const bool in = e32 > 0 && e32 < 255;
   const uint32_t hm = ((uh & 0xfffffu) << 3) | (ul >> 29);
-  const float hi = __uint_as_float(sign | (uint32_t(e32) << 23) | hm);
-  const uint32_t rem = ul & 0x1fffffffu;  // value rem * 2^(e - 1075)
-  float lo = 0.f;
-  if (rem != 0u) {
-    const int lz = __clz(int(rem));  // >= 3
-    const int el = (31 - lz) + e - 948;  // biased exponent of rem's leading bit
-    if (el > 0) lo = __uint_as_float(sign | (uint32_t(el) << 23) | ((rem << (lz + 1)) >> 9));
-  }
-  return df{hi, lo};
+  const uint32_t hb = sign | (uint32_t(e32) << 23) | hm;
+  // the other 29 bits (truncated to 24 by the conversion) times 2^(e - 1075)
+  const uint32_t rem = ul & 0x1fffffffu;
+  const uint32_t fb = __float_as_uint(__uint2float_rz(rem));
+  const int el = int(fb >> 23) + e - 1075;  // biased exponent of rem's leading bit
+  const uint32_t lb = sign | (fb + (uint32_t(e - 1075) << 23));
+  return df{__uint_as_float(in ? hb : 0u),
+            __uint_as_float(in && rem != 0u && el > 0 ? lb : 0u)};
 }
 
 // acc += (xh + xl): TwoSum of the leading parts, trailing parts summed
@@ -317,6 +317,353 @@ __global__ void __launch_bounds__(kT) k_observe(Geom G, RankView R, const T* __r
     }
     __syncthreads();
   }
+}
+
+// The sums at dg = 1 with rank tables, in two block roles: occupations, E^2
+// and the norm (double-float, FP32 pipe); and the plaquettes (FP64).  One
+// thread that did both waited on up to nine dependent neighbour gathers a
+// row, nearly all of them taken by some lane of its warp (4x4 K = 8: 4.6 ms,
+// against 1.1 GB of state).  Apart, the first role streams the state; the
+// second ranks a tile's neighbours once, lists the (row, neighbour) pairs
+// that exist plaquette by plaquette and runs its threads over that list,
+// kOP pairs' loads in flight.  Its two FMAs a pair use the FP64 pipe, which
+// the other role leaves idle (in double-float they were 100 instructions a
+// pair, and the unrolled code missed the instruction cache: 6.0 ms).  4x4
+// K = 8: 4.6 -> 3.05 ms, the shape fixed at compile time (run-time geometry
+// 3.56 ms); issue 42 %, FP64 pipe 41 %, 16 warps an SM waiting on shared and
+// global loads.
+template <typename T, int NC>
+__device__ __forceinline__ void obs_amp(const T* p, bool vec, T& a0, T& a1) {
+  if constexpr (NC == 1) {
+    a0 = __ldg(p);
+    a1 = T(0);
+  } else if (vec) {
+    if constexpr (sizeof(T) == 8) {
+      const double2 v = __ldg(reinterpret_cast<const double2*>(p));
+      a0 = v.x;
+      a1 = v.y;
+    } else {
+      const float2 v = __ldg(reinterpret_cast<const float2*>(p));
+      a0 = v.x;
+      a1 = v.y;
+    }
+  } else {
+    a0 = __ldg(p);
+    a1 = __ldg(p + 1);
+  }
+}
+__device__ __forceinline__ df obs_split(double d) { return split_df(d); }
+__device__ __forceinline__ df obs_split(float f) { return df{f, 0.f}; }
+
+// Adds the block's values red[q * kT + tid] of nq slots (point tid % K, row
+// group tid / K) and hands each sum to put(q, k, sum); called by the block.
+template <class Put>
+__device__ __forceinline__ void obs_block_sums(int nq, int K, const double* red, Put put) {
+  const int RS = kT / K, nout = nq * K;
+  int LN = 32;  // lanes per output
+  while (LN > 1 && nout * LN > kT) LN >>= 1;
+  for (int o0 = 0; o0 < nout; o0 += kT / LN) {
+    const int o = o0 + int(threadIdx.x) / LN, q = o / K, kk = o - q * K;
+    double sum = 0.0;
+    if (o < nout)
+      for (int g = int(threadIdx.x) % LN; g < RS; g += LN) sum += red[q * kT + g * K + kk];
+    for (int d = LN >> 1; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+    if (o < nout && int(threadIdx.x) % LN == 0) put(q, kk, sum);
+  }
+}
+
+constexpr int kOP = 8;  // plaquette pairs of a thread in flight
+
+// A row's link values with the lattice shape fixed at compile time (dg = 1).
+template <int NX, int NY>
+struct ObsRow {
+  using S = fixed::Shape<NX, NY>;
+  uint32_t mask;
+  int eu[S::NU], er[S::NR];
+  __device__ __forceinline__ ObsRow(const Geom& G, uint64_t key) {
+    mask = uint32_t(key >> S::USHIFT);
+    const uint32_t dig =
+        S::USHIFT == 32 ? uint32_t(key) : uint32_t(key) & ((1u << (S::USHIFT & 31)) - 1u);
+#pragma unroll
+    for (int j = 0; j < S::NU; ++j) eu[j] = int((dig >> (2 * (S::NU - 1 - j))) & 3u) - 1;
+#pragma unroll
+    for (int iy = 0; iy < NY; ++iy) {
+      int acc = 0;
+#pragma unroll
+      for (int ix = 0; ix < NX - 1; ++ix) {
+        const int st = iy * NX + ix;
+        acc += int((mask >> st) & 1u) + int(G.gq[st]);
+        if (iy < NY - 1) acc -= eu[st];
+        if (iy > 0) acc += eu[st - NX];
+        er[iy * (NX - 1) + ix] = acc;
+      }
+    }
+  }
+  // e^2 per site, two bits each
+  __device__ __forceinline__ uint32_t e2_word() const {
+    uint32_t w = 0u;
+#pragma unroll
+    for (int iy = 0; iy < NY; ++iy)
+#pragma unroll
+      for (int ix = 0; ix < NX; ++ix) {
+        int e2 = 0;
+        if (ix < NX - 1) e2 += er[iy * (NX - 1) + ix] & 1;
+        if (iy < NY - 1) e2 += eu[iy * NX + ix] & 1;
+        w |= uint32_t(e2) << (2 * (iy * NX + ix));
+      }
+    return w;
+  }
+};
+
+// NX = 0: any shape, from the run-time geometry.
+template <typename T, int NC, int MS, int MP, int NX, int NY>
+__global__ void __launch_bounds__(kT, 2) k_observe_roles(Geom G, RankView R,
+                                                         const T* __restrict__ x, int64_t N,
+                                                         int K, int nfeat, int64_t rpb,
+                                                         double* part, int* err, int vec) {
+  __shared__ uint32_t s_mask[kT], s_e2[kT];
+  __shared__ int32_t s_nbr[MP * kT];
+  __shared__ uint16_t s_row[MP * kT];
+  __shared__ int s_cnt[MP][kT / 32];
+  constexpr int kAcc = MP > kFCh ? MP : kFCh;
+  __shared__ double s_acc[kAcc * kT];
+  const int C = K * NC;
+  const int RS = kT / K;  // row subgroups
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int k = tid % K, rs = tid / K;
+  const bool worker = rs < RS;
+  const int ns = G.ns, nP = G.nP;
+  // the roles alternate over the blocks (runs of 152 blocks of one role, so
+  // that an SM's two blocks differ, measured the same)
+  const int roles = nP > 0 ? 2 : 1;
+  const int blk = int(blockIdx.x) / roles, role = int(blockIdx.x) % roles;
+  const int64_t r0 = int64_t(blk) * rpb;
+  const int64_t r1 = (r0 + rpb < N) ? r0 + rpb : N;
+
+  if (role == 0) {
+    // slots: [0, MS) occupations, [MS, 2 MS) E^2, 2 MS the norm
+    df acc[2 * MS + 1];
+#pragma unroll
+    for (int i = 0; i < 2 * MS + 1; ++i) acc[i] = df{0.f, 0.f};
+    df seg{0.f, 0.f};
+    uint32_t seg_mask = 0u;
+    auto flush = [&]() {
+#pragma unroll
+      for (int i = 0; i < MS; ++i)
+        if (i < ns && ((seg_mask >> i) & 1u)) df_add_lite(acc[i], seg.hi, seg.lo);
+      seg = df{0.f, 0.f};
+    };
+    for (int64_t t0 = r0; t0 < r1; t0 += kT) {
+      __syncthreads();
+      if (t0 + tid < r1) {
+        if constexpr (NX > 0) {
+          const ObsRow<NX, NY> o(G, __ldg(R.keys + t0 + tid));
+          s_mask[tid] = o.mask;
+          s_e2[tid] = o.e2_word();
+        } else {
+          const Config c = decode(G, __ldg(R.keys + t0 + tid));
+          uint32_t w = 0u;  // e^2 per site, two bits each (dg = 1: at most 2)
+          for (int iy = 0; iy < G.ny; ++iy)
+            for (int ix = 0; ix < G.nx; ++ix) {
+              int e2 = 0;
+              if (ix < G.nx - 1) e2 += get_eR(G, c.rpack, iy * (G.nx - 1) + ix) & 1;
+              if (iy < G.ny - 1) e2 += get_eU(G, c.digits, iy * G.nx + ix) & 1;
+              w |= uint32_t(e2) << (2 * (iy * G.nx + ix));
+            }
+          s_mask[tid] = c.mask;
+          s_e2[tid] = w;
+        }
+      }
+      __syncthreads();
+      if (!worker) continue;
+      const int rows = int((r1 - t0 < kT) ? (r1 - t0) : kT);
+      for (int rl = rs; rl < rows; rl += RS) {
+        T x0, x1;
+        obs_amp<T, NC>(x + size_t(t0 + rl) * C + k * NC, vec != 0, x0, x1);
+        const df a0 = obs_split(x0), a1 = obs_split(x1);
+        // p = |a|^2: the leading squares exactly, the cross terms rounded
+        float ph, pl;
+        two_prod(a0.hi, a0.hi, ph, pl);
+        pl = df_fma_rn(df_add_rn(a0.hi, a0.hi), a0.lo, pl);
+        if (NC == 2) {
+          float q, qe, t;
+          two_prod(a1.hi, a1.hi, q, qe);
+          qe = df_fma_rn(df_add_rn(a1.hi, a1.hi), a1.lo, qe);
+          two_sum(ph, q, ph, t);
+          pl = df_add_rn(pl, df_add_rn(qe, t));
+        }
+        fast_two_sum(ph, pl, ph, pl);
+        const uint32_t mask = s_mask[rl];
+        if (mask != seg_mask) {
+          flush();
+          seg_mask = mask;
+        }
+        df_add_lite(seg, ph, pl);
+        df_add_lite(acc[2 * MS], ph, pl);
+        const uint32_t w = s_e2[rl];
+#pragma unroll
+        for (int i = 0; i < MS; ++i) {
+          // times 0, 1 or 2: exact
+          const float f = small_int_f((w >> (2 * i)) & 3u);
+          df_add_lite(acc[MS + i], df_mul_rn(f, ph), df_mul_rn(f, pl));
+        }
+      }
+      // the trailing parts renormalised once per tile
+#pragma unroll
+      for (int i = 0; i < 2 * MS + 1; ++i) df_renorm(acc[i]);
+      df_renorm(seg);
+    }
+    if (worker) flush();
+#pragma unroll
+    for (int s0 = 0; s0 < 2 * MS + 1; s0 += kFCh) {
+      __syncthreads();
+#pragma unroll
+      for (int q = 0; q < kFCh; ++q)
+        if (s0 + q < 2 * MS + 1)
+          s_acc[q * kT + tid] = worker ? widen(acc[s0 + q].hi) + widen(acc[s0 + q].lo) : 0.0;
+      __syncthreads();
+      const int nq = 2 * MS + 1 - s0 < kFCh ? 2 * MS + 1 - s0 : kFCh;
+      obs_block_sums(nq, K, s_acc, [&](int q, int kk, double v) {
+        const int sl = s0 + q;
+        const int f = sl < MS ? (sl < ns ? sl : -1)
+                              : sl < 2 * MS ? (sl - MS < ns ? ns + sl - MS : -1) : 2 * ns + nP;
+        if (f >= 0) part[(size_t(blk) * K + kk) * nfeat + f] = v;
+      });
+    }
+    return;
+  }
+
+  for (int q = 0; q < MP; ++q) s_acc[q * kT + tid] = 0.0;
+  for (int64_t t0 = r0; t0 < r1; t0 += kT) {
+    __syncthreads();
+    int32_t nb[MP];
+    unsigned bal[MP];
+    const bool in = t0 + tid < r1;
+    const uint64_t key = __ldg(R.keys + (in ? t0 + tid : r0));
+    if constexpr (NX > 0) {
+      using S = fixed::Shape<NX, NY>;
+      const ObsRow<NX, NY> o(G, key);
+      uint32_t off[kMaxTabRows], f[kMaxTabRows], g[kMaxTabRows];
+#pragma unroll
+      for (int r = 0; r < kMaxTabRows; ++r) {
+        off[r] = uint32_t(R.tab_off[r]);
+        uint32_t v = 0u;
+        if (r < S::NROWS) {
+#pragma unroll
+          for (int ix = 0; ix < NX - 1; ++ix) v += uint32_t(o.eu[r * NX + ix] + 1) * S::pw(ix);
+        }
+        f[r] = v;
+        g[r] = (r >= 1 && r < S::NROWS) ? f[r > 0 ? r - 1 : 0] * uint32_t(S::F1) + v : 0u;
+      }
+#pragma unroll
+      for (int iy = 0; iy < NY - 1; ++iy)
+#pragma unroll
+        for (int ix = 0; ix < NX - 1; ++ix) {
+          const int q = iy * (NX - 1) + ix;
+          bool ok = in && o.er[q] > -1 && o.eu[iy * NX + ix] < 1 && o.eu[iy * NX + ix + 1] > -1 &&
+                    o.er[q + NX - 1] < 1;
+          // (a row without the move ranks itself: every load stays in range)
+          const uint32_t fn = ok ? f[iy] + S::pw(ix) - S::pw(ix + 1) : f[iy];
+          const uint32_t j = fixed::rank_fixed<NX, NY>(R.tab, off, o.mask, f, g, iy, fn);
+          if (ok && j >= uint32_t(N)) {
+            raise_err(err, kDevErrRank);
+            ok = false;
+          }
+          nb[q] = int32_t(j);
+          bal[q] = __ballot_sync(0xffffffffu, ok);
+          if (lane == 0) s_cnt[q][wid] = __popc(bal[q]);
+        }
+    } else {
+      const Config c = decode(G, key);
+      uint32_t f[kMaxTabRows];
+#pragma unroll
+      for (int r = 0; r < kMaxTabRows; ++r) f[r] = (r < R.nrows) ? row_index(R, c.digits, r) : 0u;
+      int iy = 0, ix = 0;
+#pragma unroll
+      for (int q = 0; q < MP; ++q) {
+        bool ok = false;
+        nb[q] = 0;
+        if (q < nP) {
+          const int rb = q, rt = q + (G.nx - 1), jl = iy * G.nx + ix;
+          ok = in && get_eR(G, c.rpack, rb) > -1 && get_eU(G, c.digits, jl) < 1 &&
+               get_eU(G, c.digits, jl + 1) > -1 && get_eR(G, c.rpack, rt) < 1;
+          uint32_t fy = 0u;
+#pragma unroll
+          for (int r = 0; r < kMaxTabRows; ++r)
+            if (r == iy) fy = f[r];
+          // (a row without the move ranks itself: every load stays in range)
+          const uint32_t fn = ok ? fy + uint32_t(R.pw[ix]) - uint32_t(R.pw[ix + 1]) : fy;
+          const int64_t j = rank_rows(R, c.mask, f, iy, fn);
+          if (ok && (j < 0 || j >= N)) {
+            raise_err(err, kDevErrRank);
+            ok = false;
+          }
+          nb[q] = int32_t(j);
+          if (++ix == G.nx - 1) {
+            ix = 0;
+            ++iy;
+          }
+        }
+        bal[q] = __ballot_sync(0xffffffffu, ok);
+        if (lane == 0) s_cnt[q][wid] = __popc(bal[q]);
+      }
+    }
+    __syncthreads();
+    int total = 0;  // the pairs of plaquette 0, then of plaquette 1, ...
+#pragma unroll
+    for (int q = 0; q < MP; ++q) {
+      int before = total;
+#pragma unroll
+      for (int w = 0; w < kT / 32; ++w) {
+        const int c = s_cnt[q][w];
+        before += w < wid ? c : 0;
+        total += c;
+      }
+      if ((bal[q] >> lane) & 1u) {
+        const int at = before + __popc(bal[q] & ((1u << lane) - 1u));
+        s_nbr[at] = nb[q];
+        s_row[at] = uint16_t(tid | (q << 8));
+      }
+    }
+    __syncthreads();
+    if (!worker) continue;
+    const T* xt = x + size_t(t0) * C + k * NC;
+    const T* xk = x + k * NC;
+    double acc = 0.0;
+    int cur = 0;
+    for (int p = rs; p < total; p += kOP * RS) {
+      T a0[kOP], a1[kOP], b0[kOP], b1[kOP];
+      int pq[kOP];
+#pragma unroll
+      for (int u = 0; u < kOP; ++u) {
+        const int at = p + u * RS;
+        pq[u] = -1;
+        if (at < total) {
+          const int rq = s_row[at];
+          pq[u] = rq >> 8;
+          obs_amp<T, NC>(xt + size_t(rq & 255) * C, vec != 0, a0[u], a1[u]);
+          obs_amp<T, NC>(xk + size_t(s_nbr[at]) * C, vec != 0, b0[u], b1[u]);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < kOP; ++u)
+        if (pq[u] >= 0) {
+          if (pq[u] != cur) {
+            s_acc[cur * kT + tid] += acc;
+            acc = 0.0;
+            cur = pq[u];
+          }
+          // Re conj(b) a (doubled at the end)
+          acc = fma(double(b0[u]), double(a0[u]), acc);
+          if (NC == 2) acc = fma(double(b1[u]), double(a1[u]), acc);
+        }
+    }
+    s_acc[cur * kT + tid] += acc;
+  }
+  __syncthreads();
+  obs_block_sums(MP, K, s_acc, [&](int q, int kk, double v) {
+    if (q < nP) part[(size_t(blk) * K + kk) * nfeat + 2 * ns + q] = 2.0 * v;
+  });
 }
 
 // Any lattice up to 96 features: the accumulators indexed at run time (FP64,
@@ -582,11 +929,35 @@ cudaError_t launch_obs_fixed(const Geom& G, const RankView& R, const T* x, int K
   return cudaGetLastError();
 }
 
+template <typename T, int NC, int MS, int MP, int NX = 0, int NY = 0>
+cudaError_t launch_obs_roles(const Geom& G, const RankView& R, const T* x, int K, int nfeat,
+                             int nblk, int64_t rpb, double* part, int* err, cudaStream_t s) {
+  const int vec = (reinterpret_cast<uintptr_t>(x) % (2 * sizeof(T))) == 0 ? 1 : 0;
+  k_observe_roles<T, NC, MS, MP, NX, NY><<<unsigned(nblk) * (G.nP > 0 ? 2u : 1u), kT, 0, s>>>(
+      G, R, x, R.dim, K, nfeat, rpb, part, err, vec), lgt::note_launch();
+  return cudaGetLastError();
+}
+
 template <typename T, int NC, bool DF>
 cudaError_t launch_obs_df(const Geom& G, const RankView& R, const T* x, int K, int nfeat,
                           int nblk, int64_t rpb, double* part, int* err, cudaStream_t s) {
-  // register-resident accumulators for lattices up to 16 sites and 9
-  // plaquettes (4x4), run-time indexed ones beyond
+  // two roles where e^2 per site fits two bits and neighbours rank by table;
+  // else one, with register-resident accumulators for lattices up to 16 sites
+  // and 9 plaquettes (4x4), run-time indexed ones beyond
+  if (DF && G.dg == 1 && R.tab && R.dim < (int64_t(1) << 31)) {
+    if (G.nx == 4 && G.ny == 4)
+      return launch_obs_roles<T, NC, 16, 9, 4, 4>(G, R, x, K, nfeat, nblk, rpb, part, err, s);
+    if (G.nx == 4 && G.ny == 3)
+      return launch_obs_roles<T, NC, 12, 6, 4, 3>(G, R, x, K, nfeat, nblk, rpb, part, err, s);
+    if (G.nx == 3 && G.ny == 4)
+      return launch_obs_roles<T, NC, 12, 6, 3, 4>(G, R, x, K, nfeat, nblk, rpb, part, err, s);
+    if (G.ns <= 8 && G.nP <= 4)
+      return launch_obs_roles<T, NC, 8, 4>(G, R, x, K, nfeat, nblk, rpb, part, err, s);
+    if (G.ns <= 12 && G.nP <= 6)
+      return launch_obs_roles<T, NC, 12, 6>(G, R, x, K, nfeat, nblk, rpb, part, err, s);
+    if (G.ns <= 16 && G.nP <= 9)
+      return launch_obs_roles<T, NC, 16, 9>(G, R, x, K, nfeat, nblk, rpb, part, err, s);
+  }
   if (G.ns <= 8 && G.nP <= 4)
     return launch_obs_fixed<T, NC, 8, 4, DF>(G, R, x, K, nfeat, nblk, rpb, part, err, s);
   if (G.ns <= 12 && G.nP <= 6)
