@@ -981,8 +981,8 @@ __global__ void k_set_int(int* p, int n, int v, const int* status, int only_stat
 __global__ void k_check_lowest(const double* alpha, const double* beta, int ldT, int* status,
                                const int* len, double* theta, double* resid, double* coef,
                                double tol, int fp32) {
-  // one warp per point: warp multisection of the Sturm count (FP32 for the
-  // mixed path, whose basis resolves no more), bracket warm-started from
+  // one warp per point: for the mixed path warp multisection of the Sturm
+  // count in FP32 (its basis resolves no more), bracket warm-started from
   // this point's previous theta and residual (verified by Sturm counts, so
   // stale values only cost the fallback to the Gershgorin interval)
   __shared__ double s_a[kMaxDim], s_b[kMaxDim], s_z[kMaxDim], s_work[3 * kMaxDim];
@@ -998,9 +998,16 @@ __global__ void k_check_lowest(const double* alpha, const double* beta, int ldT,
   __syncwarp();
   const double tp = theta[k], rp = resid[k];
   const bool warm = isfinite(tp) && isfinite(rp);
-  const double th = fp32 ? warp_lowest_eig_f32(s_a, s_b, n, s_z, s_work, warm, false, tp, rp)
-                         : warp_lowest_eig(s_a, s_b, n, s_z, s_work, warm, false, tp, rp);
-  const double r = fabs(beta[size_t(k) * ldT + n - 1] * s_z[n - 1]);
+  const double bn = beta[size_t(k) * ldT + n - 1];
+  double th, r;
+  bool conv;
+  if (fp32) {
+    th = warp_lowest_eig_f32(s_a, s_b, n, s_z, s_work, warm, false, tp, rp);
+    r = fabs(bn * s_z[n - 1]);
+    conv = r <= tol;
+  } else {
+    conv = warp_check_lowest(s_a, s_b, n, bn, tol, true, s_z, s_work, &th, &r);
+  }
   for (int i = lane; i < ldT; i += 32) {
     coef[(size_t(k) * ldT + i) * 2 + 0] = (i < n) ? s_z[i] : 0.0;
     coef[(size_t(k) * ldT + i) * 2 + 1] = 0.0;
@@ -1008,7 +1015,7 @@ __global__ void k_check_lowest(const double* alpha, const double* beta, int ldT,
   if (lane != 0) return;
   theta[k] = th;
   resid[k] = (st == kExhausted) ? 0.0 : r;
-  if (st == kExhausted || r <= tol) status[k] = kConverged;
+  if (st == kExhausted || conv) status[k] = kConverged;
 }
 
 // Implicit QL with eigenvectors (symmetric tridiagonal, Wilkinson-type

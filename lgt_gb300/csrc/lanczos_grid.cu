@@ -554,17 +554,25 @@ __global__ void __launch_bounds__(Threads<S>::n, 1) k_lanczos_grid(GridArgs<S> a
             __syncwarp();
             const double tp = __ldcg(a.theta + k), rp = __ldcg(a.resid + k);
             const bool warm = isfinite(tp) && isfinite(rp);
-            const double th = kDF ? warp_lowest_eig_f32(s_ta, s_tb, n, s_tz, s_work, warm, false, tp, rp)
-                                  : warp_lowest_eig(s_ta, s_tb, n, s_tz, s_work, warm, false, tp, rp);
-            const double r = fabs(bn * s_tz[n - 1]);
-            for (int i = lane; i < a.ldT; i += 32) {
+            double th, r;
+            bool conv, vec = true;  // vec: s_tz holds the vector
+            if constexpr (kDF) {
+              th = warp_lowest_eig_f32(s_ta, s_tb, n, s_tz, s_work, warm, false, tp, rp);
+              r = fabs(bn * s_tz[n - 1]);
+              conv = r <= a.tol;
+            } else {
+              const bool need = j == m || st == kExhausted;
+              conv = warp_check_lowest(s_ta, s_tb, n, bn, a.tol, need, s_tz, s_work, &th, &r);
+              vec = conv || need;
+            }
+            for (int i = lane; i < a.ldT && vec; i += 32) {
               a.coef[(size_t(k) * a.ldT + i) * 2 + 0] = (i < n) ? s_tz[i] : 0.0;
               a.coef[(size_t(k) * a.ldT + i) * 2 + 1] = 0.0;
             }
             if (lane == 0) {
               a.theta[k] = th;
               a.resid[k] = (st == kExhausted) ? 0.0 : r;
-              if (st == kExhausted || r <= a.tol) a.status[k] = kConverged;
+              if (st == kExhausted || conv) a.status[k] = kConverged;
             }
             __syncwarp();
           }

@@ -1,7 +1,9 @@
 // lgt_tridiag.cuh -- lowest eigenpair of the Lanczos tridiagonal T, on one
 // warp: Sturm-count multisection (division-free recurrence) and inverse
-// iteration, in FP64 or, for the FP32-mixed path, FP32.  Used by the
-// per-CTA solver (small.cu) and the panel solver's checks (krylov.cu).
+// iteration, in FP64 or, for the FP32-mixed path, FP32; and the FP64 path's
+// convergence check, which decides in FP32 and forms the FP64 pair by defect
+// correction.  Used by the per-CTA solver (small.cu) and the panel solver's
+// checks (krylov.cu, lanczos_grid.cu).
 // The work array holds at least 3 * kTriMax doubles, z at least kTriMax.
 #pragma once
 
@@ -384,6 +386,238 @@ __device__ inline double warp_lowest_eig_f32(const double* a64, const double* b6
   for (int i = lane; i < n; i += 32) z[i] = double(sg * zf[i]);
   __syncwarp();
   return double(theta);
+}
+
+// ---- FP64 convergence check ---------------------------------------------------
+//
+// A dependent FP64 operation takes 64 cycles on GB300 (2 lanes a clock and
+// SM), so the FP64 multisection of warp_lowest_eig costs about 150 000 cycles
+// at n = 40 -- 45 % of a 4x2 FP64 solve at a check every five steps.  The
+// check itself needs little precision:
+//   * T - a_0 in FP32, multisection there (4-cycle operations);
+//   * the bottom-up pivots u_i = d_i - s - b_i^2 / u_{i+1} at the lower end s
+//     of the bracket (all positive but the top one) give the eigenvector by
+//     its ratios z_i / z_{i-1} = -b_{i-1} / u_i: products, no differences, so
+//     even a tail component of 1e-13 has a few FP32 ulps per factor, and the
+//     residual |beta_n z_n| is known to about 1e-5 of itself.
+// Only a converged check, or one that must hand out the vector, goes on to
+// FP64: defect correction, the residual (T - theta) z in FP64 by all lanes,
+// the correction from the FP32 pivots (projected against z), about six digits
+// a round.  Clustered lowest eigenvalues (a second one within 4e-6 of the
+// spread), ranges FP32 cannot hold and corrections that stall take
+// warp_lowest_eig instead.
+__device__ __forceinline__ float warp_max_f(float v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+  return v;
+}
+__device__ __forceinline__ float warp_sum_f(float v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+__device__ __forceinline__ double warp_sum_d(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// FP32 part: true when the FP32 data describe T's lowest pair (see above);
+// theta relative to a[0] (*th), the vector's residual factor |z_{n-1}| / |z|
+// (*tail), and in work: d, b, pivots u, reciprocal pivots and the normalised
+// vector (five arrays of kTriMax floats).
+__device__ inline bool warp_lowest_f32_pivots(const double* a, const double* b, int n,
+                                              float* work, float* th, float* tail,
+                                              float* spread) {
+  const int lane = threadIdx.x & 31;
+  float* d = work;
+  float* bf = d + kTriMax;
+  float* bb = bf + kTriMax;  // then the reciprocal pivots
+  float* u = bb + kTriMax;
+  float* zf = u + kTriMax;
+  const double c0 = a[0];
+  float R = 0.0f;
+  for (int i = lane; i < n; i += 32) {
+    const float di = float(a[i] - c0);
+    const float bi = (i < n - 1) ? float(b[i]) : 0.0f;
+    d[i] = di;
+    bf[i] = bi;
+    bb[i] = bi * bi;
+    R = fmaxf(R, fabsf(di) + 2.0f * fabsf(bi));
+  }
+  __syncwarp();
+  R = warp_max_f(R);
+  if (!(R > 1e-15f && R < 1e15f)) return false;
+  // Gershgorin by rows
+  float lo = 3.0e38f, hi = -3.0e38f;
+  for (int i = lane; i < n; i += 32) {
+    const float r = ((i > 0) ? fabsf(bf[i - 1]) : 0.0f) + fabsf(bf[i]);
+    lo = fminf(lo, d[i] - r);
+    hi = fmaxf(hi, d[i] + r);
+  }
+  lo = -warp_max_f(-lo);
+  hi = warp_max_f(hi);
+  const float width = hi - lo;
+  lo -= 1e-6f * width;
+  hi += 1e-6f * width;
+  for (int it = 0; it < 12; ++it) {
+    if (hi - lo <= 4e-7f * width) break;
+    const float step = (hi - lo) * (1.0f / 33.0f);
+    const float x = lo + step * float(lane + 1);
+    const unsigned bal = __ballot_sync(0xffffffffu, sturm_below_f(d, bb, n, x) >= 1);
+    const int L = bal ? __ffs(bal) - 1 : 32;
+    const float nlo = lo + step * float(L), nhi = (L < 32) ? lo + step * float(L + 1) : hi;
+    if (!(nhi < hi) && !(nlo > lo)) break;
+    if (L > 0) lo = nlo;
+    hi = nhi;
+  }
+  // one eigenvalue only near the bracket
+  const int near = sturm_below_f(d, bb, n, hi + 4e-6f * width);
+  if (near > 1) return false;
+  const float s = lo - 4e-7f * width;
+  __syncwarp();
+  // pivots and ratios from the bottom, by lane 0
+  int ok = 1;
+  if (lane == 0) {
+    float un = d[n - 1] - s, rn = 1.0f / un;
+    u[n - 1] = un;
+    ok = un > 1e-6f * width || n == 1;
+    for (int i = n - 2; i >= 0; --i) {
+      const float b2 = bf[i] * bf[i];
+      un = (d[i] - s) - b2 * rn;
+      bb[i + 1] = rn;
+      if (i > 0 && !(un > 1e-6f * width)) ok = 0;
+      if (i == 0 && !(un > 1e-7f * width)) un = 1e-7f * width;
+      rn = 1.0f / un;
+      u[i] = un;
+    }
+    bb[0] = rn;
+    float z = 1.0f;
+    zf[0] = 1.0f;
+    for (int i = 1; i < n; ++i) {
+      z = -z * (bf[i - 1] * bb[i]);
+      zf[i] = z;
+    }
+  }
+  __syncwarp();
+  ok = __shfl_sync(0xffffffffu, ok, 0);
+  float m = 0.0f;
+  for (int i = lane; i < n; i += 32) m = fmaxf(m, fabsf(zf[i]));
+  m = warp_max_f(m);
+  if (!ok || !(m < 1e15f)) return false;
+  float q = 0.0f;
+  for (int i = lane; i < n; i += 32) q = fmaf(zf[i] / m, zf[i] / m, q);
+  const float inv = 1.0f / (m * sqrtf(warp_sum_f(q)));
+  *tail = fabsf(zf[n - 1]) * inv;
+  __syncwarp();
+  for (int i = lane; i < n; i += 32) zf[i] *= inv;
+  __syncwarp();
+  *th = 0.5f * (lo + hi);
+  *spread = width;
+  return true;
+}
+
+// The check of the n x n Lanczos tridiagonal (a, b) with beta_n = bn, by one
+// warp: *theta and the residual |bn z_{n-1}| in *resid, and whether it is at
+// most tol.  z (kTriMax doubles) holds the FP64 eigenvector when the check
+// converged or `need` is set (theta is FP64-accurate only then).  work: 3 *
+// kTriMax doubles.
+__device__ inline bool warp_check_lowest(const double* a, const double* b, int n, double bn,
+                                         double tol, bool need, double* z, double* work,
+                                         double* theta, double* resid) {
+  const int lane = threadIdx.x & 31;
+  float* w = reinterpret_cast<float*>(work);
+  float th = 0.0f, tail = 0.0f, width = 0.0f;
+  if (n > 1 && warp_lowest_f32_pivots(a, b, n, w, &th, &tail, &width)) {
+    const double r = fabs(bn) * double(tail);
+    *resid = r;
+    const bool conv = r <= tol;
+    const double s0 = a[0] + double(th);
+    if (!conv && !need) {
+      *theta = s0;
+      return false;
+    }
+    const float* bf = w + kTriMax;
+    const float* ru = w + 2 * kTriMax;
+    float* y = w + 3 * kTriMax;  // (the pivots: only their reciprocals are needed)
+    float* x = w + 4 * kTriMax;  // the FP32 vector, then the corrections
+    const int i0 = lane, i1 = lane + 32;
+    double z0 = (i0 < n) ? double(x[i0]) : 0.0, z1 = (i1 < n) ? double(x[i1]) : 0.0;
+    const double t0 = (i0 < n) ? a[i0] - s0 : 0.0, t1 = (i1 < n) ? a[i1] - s0 : 0.0;
+    const double bl0 = (i0 > 0 && i0 < n) ? b[i0 - 1] : 0.0, br0 = (i0 < n - 1) ? b[i0] : 0.0;
+    const double bl1 = (i1 < n) ? b[i1 - 1] : 0.0, br1 = (i1 < n - 1) ? b[i1] : 0.0;
+    bool good = false;
+    double dth = 0.0;
+    float last = 3.0e38f;
+    for (int it = 0; it < 6; ++it) {
+      if (i0 < n) z[i0] = z0;
+      if (i1 < n) z[i1] = z1;
+      __syncwarp();
+      const double l0 = (i0 > 0 && i0 < n) ? z[i0 - 1] : 0.0, r0 = (i0 < n - 1) ? z[i0 + 1] : 0.0;
+      const double l1 = (i1 < n) ? z[i1 - 1] : 0.0, r1 = (i1 < n - 1) ? z[i1 + 1] : 0.0;
+      const double v0 = fma(t0, z0, fma(bl0, l0, br0 * r0));
+      double v1 = 0.0;
+      if (n > 32) v1 = fma(t1, z1, fma(bl1, l1, br1 * r1));
+      double zv = z0 * v0, zz = z0 * z0;
+      if (n > 32) {
+        zv = fma(z1, v1, zv);
+        zz = fma(z1, z1, zz);
+      }
+      zv = warp_sum_d(zv);
+      zz = warp_sum_d(zz);
+      // |z|^2 is 1 to FP32 accuracy or better: first-order reciprocals
+      dth = zv * (2.0 - zz);
+      const double e0 = fma(-dth, z0, v0), e1 = fma(-dth, z1, v1);
+      const float f0 = float(e0), f1 = float(e1);
+      const float big = warp_max_f(fmaxf(fabsf(f0), fabsf(f1)));
+      if (!(big <= 0.25f * last)) {  // no further gain: at rounding level, or stalled
+        good = big <= 4e-15f * width;
+        break;
+      }
+      last = big;
+      if (big == 0.0f) {
+        good = true;
+        break;
+      }
+      __syncwarp();
+      if (i0 < n) y[i0] = f0 / big;
+      if (i1 < n) y[i1] = f1 / big;
+      __syncwarp();
+      // (T - s) x = residual through the pivots: up, then down (lane 0)
+      if (lane == 0) {
+        float yp = y[n - 1];
+        for (int i = n - 2; i >= 0; --i) {
+          yp = fmaf(-bf[i] * ru[i + 1], yp, y[i]);
+          y[i] = yp;
+        }
+        float xp = y[0] * ru[0];
+        x[0] = xp;
+        for (int i = 1; i < n; ++i) {
+          xp = ru[i] * fmaf(-bf[i - 1], xp, y[i]);
+          x[i] = xp;
+        }
+      }
+      __syncwarp();
+      const float g0 = (i0 < n) ? x[i0] : 0.0f, g1 = (i1 < n) ? x[i1] : 0.0f;
+      const float zf0 = float(z0), zf1 = float(z1);
+      const float along = warp_sum_f(fmaf(zf0, g0, zf1 * g1));
+      const float h0 = fmaf(-along, zf0, g0), h1 = fmaf(-along, zf1, g1);
+      z0 = fma(-double(big), double(h0), z0);
+      z1 = fma(-double(big), double(h1), z1);
+      // unit length again (to first order in |z|^2 - 1)
+      const double sc = fma(-0.5, zz, 1.5);
+      z0 *= sc;
+      z1 *= sc;
+    }
+    if (good) {
+      *theta = s0 + dth;
+      __syncwarp();
+      return conv;
+    }
+  }
+  *theta = warp_lowest_eig(a, b, n, z, work, false, false, 0.0, 0.0);
+  *resid = fabs(bn * z[n - 1]);
+  return *resid <= tol;
 }
 
 }  // namespace lgt

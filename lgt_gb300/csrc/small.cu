@@ -582,24 +582,29 @@ __global__ void __launch_bounds__(kCta, 1) k_lanczos_cta(const SmallProblem* pro
       if (check) {
         unit_sync();
         if (wid == 0) {
-          const double th =
-              fp32 ? warp_lowest_eig_f32(s_alpha, s_beta, n, s_z, s_work, s_zwarm != 0,
-                                         s_zwarm != 0, s_theta, s_resid)
-                   : warp_lowest_eig(s_alpha, s_beta, n, s_z, s_work, s_zwarm != 0,
-                                     s_zwarm != 0, s_theta, s_resid);
+          double th, rr = 0.0;
+          bool conv = false;
+          if constexpr (kDF) {
+            th = warp_lowest_eig_f32(s_alpha, s_beta, n, s_z, s_work, s_zwarm != 0, s_zwarm != 0,
+                                     s_theta, s_resid);
+          } else {
+            conv = warp_check_lowest(s_alpha, s_beta, n, s_beta[n - 1], tol,
+                                     exhausted || j + 1 == m, s_z, s_work, &th, &rr);
+          }
           if (lane == 0) {
-            const double rr = exhausted ? 0.0 : fabs(s_beta[n - 1] * s_z[n - 1]);
+            if constexpr (kDF) rr = fabs(s_beta[n - 1] * s_z[n - 1]);
+            if (exhausted) rr = 0.0;
             // FP32 panels resolve residuals to ~1e-6 |H|: relative floor
             const double tl = fp32 ? fmax(tol, 3e-6 * fmax(fabs(th), 1.0)) : tol;
-            s_flag = (exhausted || rr <= tl) ? 1 : 0;
+            s_flag = (exhausted || (kDF ? rr <= tl : conv)) ? 1 : 0;
             int nxt = n + prm.check_every;
             if (s_pstep > 0 && rr > tl && s_pres > rr) {
-              const double rate = log(rr / s_pres) / double(n - s_pstep);  // < 0
+              const float rate = logf(float(rr) / float(s_pres)) / float(n - s_pstep);  // < 0
               // steps to the tolerance at that rate (a 25% margin measured
               // slower: 121k vs 124.7k GS/s on the 4x2 batch)
-              const double need = log(tl / rr) / rate;                      // > 0 steps
-              if (need < double(prm.check_every)) {
-                const int p = n + ((need > 1.0) ? int(ceil(need)) : 1);
+              const float need = logf(float(tl) / float(rr)) / rate;  // > 0 steps
+              if (need < float(prm.check_every)) {
+                const int p = n + ((need > 1.0f) ? int(ceilf(need)) : 1);
                 if (p < nxt) nxt = p;
               }
             }
