@@ -1006,7 +1006,7 @@ __global__ void k_check_lowest(const double* alpha, const double* beta, int ldT,
     r = fabs(bn * s_z[n - 1]);
     conv = r <= tol;
   } else {
-    conv = warp_check_lowest(s_a, s_b, n, bn, tol, true, s_z, s_work, &th, &r);
+    conv = warp_check_lowest(s_a, s_b, n, bn, tol, true, warm, tp, rp, s_z, s_work, &th, &r);
   }
   for (int i = lane; i < ldT; i += 32) {
     coef[(size_t(k) * ldT + i) * 2 + 0] = (i < n) ? s_z[i] : 0.0;

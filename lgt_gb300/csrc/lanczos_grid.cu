@@ -562,7 +562,8 @@ __global__ void __launch_bounds__(Threads<S>::n, 1) k_lanczos_grid(GridArgs<S> a
               conv = r <= a.tol;
             } else {
               const bool need = j == m || st == kExhausted;
-              conv = warp_check_lowest(s_ta, s_tb, n, bn, a.tol, need, s_tz, s_work, &th, &r);
+              conv = warp_check_lowest(s_ta, s_tb, n, bn, a.tol, need, warm, tp, rp, s_tz, s_work, &th,
+                                       &r);
               vec = conv || need;
             }
             for (int i = lane; i < a.ldT && vec; i += 32) {

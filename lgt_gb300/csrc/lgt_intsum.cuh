@@ -22,6 +22,33 @@ namespace lgt {
 
 constexpr int kMaxIntTerms = 31;
 
+// Whether values whose largest high word (sign cleared) is `top` can be
+// summed in units of that exponent.
+__device__ __forceinline__ bool fix_range(int top) {
+  const int eb = top & 0x7ff00000;
+  return eb >= (100 << 20) && eb <= (0x7ef << 20);
+}
+// v in units of 2^-57 of the exponent eb (a high word's exponent field, no
+// smaller than v's), truncated towards zero; eor flips the sign by its bit 31.
+__device__ __forceinline__ long long fix_of(double v, int eb, uint32_t eor = 0u) {
+  const int hi = __double2hiint(v);
+  const uint32_t lo = uint32_t(__double2loint(v));
+  const int sh = min((eb - (hi & 0x7ff00000)) >> 20, 63);
+  const uint32_t mh = (uint32_t(hi) & 0xfffffu) | 0x100000u;
+  unsigned long long m =
+      (static_cast<unsigned long long>((mh << 5) | (lo >> 27)) << 32) | (lo << 5);
+  m >>= sh;
+  const int neg = int(uint32_t(hi) ^ eor) >> 31;  // 0 or -1
+  const unsigned long long sg = static_cast<unsigned long long>(static_cast<long long>(neg));
+  return static_cast<long long>((m ^ sg) - sg);
+}
+// The FP64 value of a sum t of such terms: t 2^(E - 1080), E the exponent.
+__device__ __forceinline__ double fix_to(long long t, int eb) {
+  if (t == 0) return 0.0;
+  const double d = __ll2double_rn(t);
+  return __hiloint2double(__double2hiint(d) + (eb - (1080 << 20)), __double2loint(d));
+}
+
 // s = sum of the W-column slices load(entry index) of lst[n0 .. n1), U of
 // them in flight; SGN: bit 31 of an entry flips the sign.  At most
 // kMaxIntTerms entries.
@@ -58,30 +85,14 @@ __device__ __forceinline__ void int_sum_part(const uint32_t* lst, int n0, int n1
       acc[e] >>= min(drop, 63);
       top[e] = t;
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int hi = __double2hiint(v[u][e]);
-        const uint32_t lo = uint32_t(__double2loint(v[u][e]));
-        const int sh = min((eb - (hi & 0x7ff00000)) >> 20, 63);
-        const uint32_t mh = (uint32_t(hi) & 0xfffffu) | 0x100000u;
-        unsigned long long m =
-            (static_cast<unsigned long long>((mh << 5) | (lo >> 27)) << 32) | (lo << 5);
-        m >>= sh;
-        const int neg = (SGN ? hi ^ int(ent[u]) : hi) >> 31;  // 0 or -1
-        const unsigned long long sg = static_cast<unsigned long long>(static_cast<long long>(neg));
-        acc[e] += static_cast<long long>((m ^ sg) - sg);
-      }
+      for (int u = 0; u < U; ++u) acc[e] += fix_of(v[u][e], eb, SGN ? ent[u] : 0u);
     }
   }
 #pragma unroll
   for (int e = 0; e < W; ++e) {
-    const int eb = top[e] & 0x7ff00000;
     s[e] = 0.0;
-    if (eb >= (100 << 20) && eb <= (0x7ef << 20)) {
-      // acc 2^(E - 1080) with E the largest exponent field: the field moves
-      if (acc[e] != 0) {
-        const double d = __ll2double_rn(acc[e]);
-        s[e] = __hiloint2double(__double2hiint(d) + (eb - (1080 << 20)), __double2loint(d));
-      }
+    if (fix_range(top[e])) {
+      s[e] = fix_to(acc[e], top[e] & 0x7ff00000);
     } else if (top[e] != 0) {
       for (int n = n0; n < n1; ++n) {
         double v[W];
@@ -92,7 +103,56 @@ __device__ __forceinline__ void int_sum_part(const uint32_t* lst, int n0, int n1
   }
 }
 
-// The same for any number of entries.
+// The sum over a warp of one double per lane (32 terms of 58 bits just fit):
+// every lane gets it.
+__device__ __forceinline__ double warp_sum_int(double v) {
+  const int top = int(__reduce_max_sync(0xffffffffu, uint32_t(__double2hiint(v)) & 0x7fffffffu));
+  if (top == 0) return 0.0;
+  if (!fix_range(top)) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+  }
+  const int eb = top & 0x7ff00000;
+  long long x = fix_of(v, eb);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  return fix_to(x, eb);
+}
+
+// The warp totals of four doubles per lane, value q in lanes 8 q .. 8 q + 7
+// (reduce-scatter: two exchange steps halve the values, three finish them).
+__device__ __forceinline__ double warp_scatter4_int(const double* p, int lane) {
+  const bool b4 = lane & 16, b3 = lane & 8;
+  int top[4];
+  bool ok = true;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    top[q] = int(__reduce_max_sync(0xffffffffu, uint32_t(__double2hiint(p[q])) & 0x7fffffffu));
+    ok = ok && (top[q] == 0 || fix_range(top[q]));
+  }
+  if (!ok) {
+    const double r0 = __shfl_xor_sync(0xffffffffu, b4 ? p[0] : p[2], 16);
+    const double r1 = __shfl_xor_sync(0xffffffffu, b4 ? p[1] : p[3], 16);
+    const double k0 = (b4 ? p[2] : p[0]) + r0, k1 = (b4 ? p[3] : p[1]) + r1;
+    double kk = (b3 ? k1 : k0) + __shfl_xor_sync(0xffffffffu, b3 ? k0 : k1, 8);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) kk += __shfl_xor_sync(0xffffffffu, kk, o);
+    return kk;
+  }
+  long long x[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) x[q] = top[q] == 0 ? 0 : fix_of(p[q], top[q] & 0x7ff00000);
+  const long long r0 = __shfl_xor_sync(0xffffffffu, b4 ? x[0] : x[2], 16);
+  const long long r1 = __shfl_xor_sync(0xffffffffu, b4 ? x[1] : x[3], 16);
+  const long long k0 = (b4 ? x[2] : x[0]) + r0, k1 = (b4 ? x[3] : x[1]) + r1;
+  long long kk = (b3 ? k1 : k0) + __shfl_xor_sync(0xffffffffu, b3 ? k0 : k1, 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) kk += __shfl_xor_sync(0xffffffffu, kk, o);
+  return fix_to(kk, (b4 ? (b3 ? top[3] : top[2]) : (b3 ? top[1] : top[0])) & 0x7ff00000);
+}
+
+// int_sum_part for any number of entries.
 template <int W, int U, bool SGN, class Load>
 __device__ __forceinline__ void int_sum(const uint32_t* lst, int n0, int n1, double (&s)[W],
                                         Load load) {

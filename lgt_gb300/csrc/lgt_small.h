@@ -18,6 +18,7 @@ constexpr int kSmallMaxN = 8192;
 struct Pattern {
   int N = 0;
   int nnz = 0;
+  int max_moves = 0;  // most neighbours a row can have
   uint32_t model = 0;
   int* rowptr = nullptr;
   uint32_t* nbr = nullptr;
@@ -54,7 +55,12 @@ struct SmallParams {
   uint64_t seed;
   int start_given;
   int rows_per_thread = 0;  // launch shape: 0 the smallest R with N <= 512 R
-  int v_smem = 0;           // set by the launcher: Krylov basis in shared memory
+  // set by the launcher: the CTA's rows of the Krylov basis in shared memory
+  // (then the current vector from byte x_off on), and its neighbour lists
+  // (from byte list_off on)
+  int v_smem = 0, x_off = 0;
+  int list_cap = 0, list_off = 0;
+  int max_moves = 0;        // most neighbours a row of the batch can have
 };
 
 // One Hamiltonian's share of a batched launch.

@@ -422,19 +422,60 @@ __device__ __forceinline__ double warp_sum_d(double v) {
   return v;
 }
 
+// Solves (T - s) y = y through the bottom-up pivots (reciprocals ru, couplings
+// bf): up, then down, by lane 0, operands read eight ahead.
+__device__ __forceinline__ void pivot_solve(const float* bf, const float* ru, int n, float* y) {
+  float yp = 0.0f;
+  for (int i1 = n - 1; i1 >= 0; i1 -= 8) {
+    float yc[8], c[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int i = i1 - q;
+      yc[q] = (i >= 0) ? y[i] : 0.0f;
+      c[q] = (i >= 0 && i < n - 1) ? bf[i] * ru[i + 1] : 0.0f;
+    }
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (i1 - q >= 0) {
+        yp = fmaf(-c[q], yp, yc[q]);
+        y[i1 - q] = yp;
+      }
+  }
+  float xp = 0.0f;
+  for (int i0 = 0; i0 < n; i0 += 8) {
+    float yc[8], c[8], r[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int i = i0 + q;
+      yc[q] = (i < n) ? y[i] : 0.0f;
+      r[q] = (i < n) ? ru[i] : 0.0f;
+      c[q] = (i > 0 && i < n) ? bf[i - 1] : 0.0f;
+    }
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (i0 + q < n) {
+        xp = r[q] * fmaf(-c[q], xp, yc[q]);
+        y[i0 + q] = xp;
+      }
+  }
+}
+
 // FP32 part: true when the FP32 data describe T's lowest pair (see above);
 // theta relative to a[0] (*th), the vector's residual factor |z_{n-1}| / |z|
-// (*tail), and in work: d, b, pivots u, reciprocal pivots and the normalised
-// vector (five arrays of kTriMax floats).
+// (*tail), and in work: d, b, b^2, the reciprocal pivots and the normalised
+// vector (five arrays of kTriMax floats).  warm: th_prev, r_prev are an
+// earlier check's theta and residual; the lowest value lies in [th_prev -
+// 2 r_prev, th_prev] unless the counts at its ends say otherwise.
 __device__ inline bool warp_lowest_f32_pivots(const double* a, const double* b, int n,
-                                              float* work, float* th, float* tail,
+                                              float* work, bool warm, double th_prev,
+                                              double r_prev, float* th, float* tail,
                                               float* spread) {
   const int lane = threadIdx.x & 31;
   float* d = work;
   float* bf = d + kTriMax;
-  float* bb = bf + kTriMax;  // then the reciprocal pivots
-  float* u = bb + kTriMax;
-  float* zf = u + kTriMax;
+  float* bb = bf + kTriMax;
+  float* ru = bb + kTriMax;
+  float* zf = ru + kTriMax;
   const double c0 = a[0];
   float R = 0.0f;
   for (int i = lane; i < n; i += 32) {
@@ -460,6 +501,20 @@ __device__ inline bool warp_lowest_f32_pivots(const double* a, const double* b, 
   const float width = hi - lo;
   lo -= 1e-6f * width;
   hi += 1e-6f * width;
+  if (warm) {
+    const float tp = float(th_prev - c0), rp = float(r_prev);
+    const float whi = fminf(hi, tp + 2e-6f * width);
+    const float wlo = fmaxf(lo, tp - fmaxf(2.0f * rp, 4e-6f * width));
+    // the first round's probes include both ends
+    const float step = (whi - wlo) * (1.0f / 31.0f);
+    const float x = (lane == 31) ? whi : wlo + step * float(lane);
+    const unsigned bal = __ballot_sync(0xffffffffu, sturm_below_f(d, bb, n, x) >= 1);
+    if (!(bal & 1u) && (bal >> 31)) {
+      const int L = __ffs(bal) - 1;
+      lo = wlo + step * float(L - 1);
+      hi = (L == 31) ? whi : wlo + step * float(L);
+    }
+  }
   for (int it = 0; it < 12; ++it) {
     if (hi - lo <= 4e-7f * width) break;
     const float step = (hi - lo) * (1.0f / 33.0f);
@@ -476,27 +531,45 @@ __device__ inline bool warp_lowest_f32_pivots(const double* a, const double* b, 
   if (near > 1) return false;
   const float s = lo - 4e-7f * width;
   __syncwarp();
-  // pivots and ratios from the bottom, by lane 0
+  // pivots and ratios from the bottom, by lane 0, operands read eight ahead
   int ok = 1;
   if (lane == 0) {
-    float un = d[n - 1] - s, rn = 1.0f / un;
-    u[n - 1] = un;
-    ok = un > 1e-6f * width || n == 1;
-    for (int i = n - 2; i >= 0; --i) {
-      const float b2 = bf[i] * bf[i];
-      un = (d[i] - s) - b2 * rn;
-      bb[i + 1] = rn;
-      if (i > 0 && !(un > 1e-6f * width)) ok = 0;
-      if (i == 0 && !(un > 1e-7f * width)) un = 1e-7f * width;
-      rn = 1.0f / un;
-      u[i] = un;
+    float rn = 0.0f;
+    const float small = 1e-6f * width;
+    for (int i1 = n - 1; i1 >= 0; i1 -= 8) {
+      float dc[8], bc[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const int i = i1 - q;
+        dc[q] = (i >= 0) ? d[i] - s : 0.0f;
+        bc[q] = (i >= 0) ? bb[i] : 0.0f;
+      }
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const int i = i1 - q;
+        if (i >= 0) {
+          float un = fmaf(-bc[q], rn, dc[q]);
+          if (i > 0 && !(un > small)) ok = 0;
+          if (i == 0) un = fmaxf(un, 0.1f * small);
+          rn = __fdividef(1.0f, un);
+          ru[i] = rn;
+        }
+      }
     }
-    bb[0] = rn;
     float z = 1.0f;
-    zf[0] = 1.0f;
-    for (int i = 1; i < n; ++i) {
-      z = -z * (bf[i - 1] * bb[i]);
-      zf[i] = z;
+    for (int i0 = 0; i0 < n; i0 += 8) {
+      float f[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const int i = i0 + q;
+        f[q] = (i > 0 && i < n) ? bf[i - 1] * ru[i] : 0.0f;
+      }
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const int i = i0 + q;
+        if (i > 0) z = -z * f[q];
+        if (i < n) zf[i] = z;
+      }
     }
   }
   __syncwarp();
@@ -505,9 +578,10 @@ __device__ inline bool warp_lowest_f32_pivots(const double* a, const double* b, 
   for (int i = lane; i < n; i += 32) m = fmaxf(m, fabsf(zf[i]));
   m = warp_max_f(m);
   if (!ok || !(m < 1e15f)) return false;
+  const float im = __fdividef(1.0f, m);
   float q = 0.0f;
-  for (int i = lane; i < n; i += 32) q = fmaf(zf[i] / m, zf[i] / m, q);
-  const float inv = 1.0f / (m * sqrtf(warp_sum_f(q)));
+  for (int i = lane; i < n; i += 32) q = fmaf(zf[i] * im, zf[i] * im, q);
+  const float inv = im * rsqrtf(warp_sum_f(q));
   *tail = fabsf(zf[n - 1]) * inv;
   __syncwarp();
   for (int i = lane; i < n; i += 32) zf[i] *= inv;
@@ -517,18 +591,50 @@ __device__ inline bool warp_lowest_f32_pivots(const double* a, const double* b, 
   return true;
 }
 
+// The mixed path's check: theta to FP32 accuracy of the spread, z (normalised,
+// first component positive, after one inverse iteration with the pivots: the
+// ratios alone carry the shift's distance from theta) and *resid =
+// |bn z_{n-1}|; clusters and ranges FP32 cannot hold through
+// warp_lowest_eig_f32.
+__device__ inline double warp_check_lowest_f32(const double* a, const double* b, int n, double bn,
+                                               bool warm, double th_prev, double r_prev,
+                                               double* z, double* work, double* resid) {
+  const int lane = threadIdx.x & 31;
+  float* w = reinterpret_cast<float*>(work);
+  float th = 0.0f, tail = 0.0f, width = 0.0f;
+  if (n > 1 && warp_lowest_f32_pivots(a, b, n, w, warm, th_prev, r_prev, &th, &tail, &width)) {
+    float* zf = w + 4 * kTriMax;
+    if (lane == 0) pivot_solve(w + kTriMax, w + 3 * kTriMax, n, zf);
+    __syncwarp();
+    float m = 0.0f;
+    for (int i = lane; i < n; i += 32) m = fmaxf(m, fabsf(zf[i]));
+    const float im = __fdividef(1.0f, warp_max_f(m));
+    float q = 0.0f;
+    for (int i = lane; i < n; i += 32) q = fmaf(zf[i] * im, zf[i] * im, q);
+    const float inv = im * rsqrtf(warp_sum_f(q));
+    for (int i = lane; i < n; i += 32) z[i] = double(zf[i] * inv);
+    *resid = fabs(bn) * double(tail);
+    __syncwarp();
+    return a[0] + double(th);
+  }
+  const double t = warp_lowest_eig_f32(a, b, n, z, work, false, false, 0.0, 0.0);
+  *resid = fabs(bn * z[n - 1]);
+  return t;
+}
+
 // The check of the n x n Lanczos tridiagonal (a, b) with beta_n = bn, by one
 // warp: *theta and the residual |bn z_{n-1}| in *resid, and whether it is at
 // most tol.  z (kTriMax doubles) holds the FP64 eigenvector when the check
 // converged or `need` is set (theta is FP64-accurate only then).  work: 3 *
 // kTriMax doubles.
 __device__ inline bool warp_check_lowest(const double* a, const double* b, int n, double bn,
-                                         double tol, bool need, double* z, double* work,
-                                         double* theta, double* resid) {
+                                         double tol, bool need, bool warm, double th_prev,
+                                         double r_prev, double* z, double* work, double* theta,
+                                         double* resid) {
   const int lane = threadIdx.x & 31;
   float* w = reinterpret_cast<float*>(work);
   float th = 0.0f, tail = 0.0f, width = 0.0f;
-  if (n > 1 && warp_lowest_f32_pivots(a, b, n, w, &th, &tail, &width)) {
+  if (n > 1 && warp_lowest_f32_pivots(a, b, n, w, warm, th_prev, r_prev, &th, &tail, &width)) {
     const double r = fabs(bn) * double(tail);
     *resid = r;
     const bool conv = r <= tol;
@@ -538,9 +644,8 @@ __device__ inline bool warp_check_lowest(const double* a, const double* b, int n
       return false;
     }
     const float* bf = w + kTriMax;
-    const float* ru = w + 2 * kTriMax;
-    float* y = w + 3 * kTriMax;  // (the pivots: only their reciprocals are needed)
-    float* x = w + 4 * kTriMax;  // the FP32 vector, then the corrections
+    const float* ru = w + 3 * kTriMax;
+    float* x = w + 4 * kTriMax;  // the FP32 vector, then residuals and corrections
     const int i0 = lane, i1 = lane + 32;
     double z0 = (i0 < n) ? double(x[i0]) : 0.0, z1 = (i1 < n) ? double(x[i1]) : 0.0;
     const double t0 = (i0 < n) ? a[i0] - s0 : 0.0, t1 = (i1 < n) ? a[i1] - s0 : 0.0;
@@ -580,23 +685,11 @@ __device__ inline bool warp_check_lowest(const double* a, const double* b, int n
         break;
       }
       __syncwarp();
-      if (i0 < n) y[i0] = f0 / big;
-      if (i1 < n) y[i1] = f1 / big;
+      const float ib = 1.0f / big;
+      if (i0 < n) x[i0] = f0 * ib;
+      if (i1 < n) x[i1] = f1 * ib;
       __syncwarp();
-      // (T - s) x = residual through the pivots: up, then down (lane 0)
-      if (lane == 0) {
-        float yp = y[n - 1];
-        for (int i = n - 2; i >= 0; --i) {
-          yp = fmaf(-bf[i] * ru[i + 1], yp, y[i]);
-          y[i] = yp;
-        }
-        float xp = y[0] * ru[0];
-        x[0] = xp;
-        for (int i = 1; i < n; ++i) {
-          xp = ru[i] * fmaf(-bf[i - 1], xp, y[i]);
-          x[i] = xp;
-        }
-      }
+      if (lane == 0) pivot_solve(bf, ru, n, x);  // (T - s) x = residual / big
       __syncwarp();
       const float g0 = (i0 < n) ? x[i0] : 0.0f, g1 = (i1 < n) ? x[i1] : 0.0f;
       const float zf0 = float(z0), zf1 = float(z1);

@@ -28,11 +28,13 @@
 #include <mutex>
 #include <string>
 #include <tuple>
+#include <type_traits>
 #include <vector>
 
 #include <cooperative_groups.h>
 
 #include "lgt_dfloat.cuh"
+#include "lgt_intsum.cuh"
 #include "lgt_moves.cuh"
 #include "lgt_rank.cuh"
 #include "lgt_small.h"
@@ -142,83 +144,6 @@ __device__ __forceinline__ double start_normal(uint64_t seed, int k, int64_t row
   return sqrt(-2.0 * log(u1)) * cospi(2.0 * u2);
 }
 
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
-// Block-wide sum of one double per thread (all threads get the result):
-// the values go to shared memory and warp 0 alone adds them (lanes over
-// every 32nd value, then a shuffle tree), so one warp, not all of them,
-// spends FP64 instructions on the reduction (GB300's FP64 pipe is narrow).
-// Thread 0 also calls root(sum) before the block reads the result, for
-// scalars that only depend on it (a norm and its reciprocal, computed once
-// for the block instead of by every thread).  red: blockDim.x doubles.
-template <class Root>
-__device__ double block_sum(double v, double* red, double* out, Root root) {
-  const int tid = threadIdx.x;
-  red[tid] = v;
-  __syncthreads();
-  if (tid < 32) {
-    double s = 0.0;
-    for (int i = tid; i < int(blockDim.x); i += 32) s += red[i];
-    s = warp_sum(s);
-    if (tid == 0) {
-      out[0] = s;
-      root(s);
-    }
-  }
-  __syncthreads();
-  return out[0];
-}
-__device__ double block_sum(double v, double* red, double* out) {
-  return block_sum(v, red, out, [](double) {});
-}
-
-// The sum over a unit's CTAs of one double per thread.  CL = 1: block_sum.
-// CL = 2 (a cluster of two CTAs per unit, rows split between them): each
-// CTA's total goes into slot [par][rank] of both CTAs' `xch`, and after the
-// cluster barrier thread 0 of each CTA adds slot 0 and slot 1 in that order,
-// so both CTAs hold bitwise the same sum (their control flow, which depends
-// only on such sums, stays identical).  `par` flips at every call, so a CTA
-// running ahead never overwrites a slot that its peer has yet to read.
-template <int CL, class Root>
-__device__ double unit_sum(double v, double* red, double* out, double* xch, int& par, Root root) {
-  if constexpr (CL == 1) {
-    return block_sum(v, red, out, root);
-  } else {
-    namespace cg = cooperative_groups;
-    cg::cluster_group cl = cg::this_cluster();
-    const int tid = threadIdx.x;
-    const unsigned cr = cl.block_rank();
-    red[tid] = v;
-    __syncthreads();
-    if (tid < 32) {
-      double s = 0.0;
-      for (int i = tid; i < int(blockDim.x); i += 32) s += red[i];
-      s = warp_sum(s);
-      if (tid == 0) {
-        xch[par * 2 + cr] = s;
-        cl.map_shared_rank(xch, cr ^ 1u)[par * 2 + cr] = s;
-      }
-    }
-    cl.sync();
-    if (tid == 0) {
-      const double s = xch[par * 2] + xch[par * 2 + 1];
-      out[0] = s;
-      root(s);
-    }
-    par ^= 1;
-    __syncthreads();
-    return out[0];
-  }
-}
-template <int CL>
-__device__ double unit_sum(double v, double* red, double* out, double* xch, int& par) {
-  return unit_sum<CL>(v, red, out, xch, par, [](double) {});
-}
-
 __device__ __forceinline__ df shfl_xor_df(df v, int o) {
   return df{__shfl_xor_sync(0xffffffffu, v.hi, o), __shfl_xor_sync(0xffffffffu, v.lo, o)};
 }
@@ -232,10 +157,9 @@ __device__ __forceinline__ void df_sq2(df& x, float h, float l) {
   df_acc(x, p, e);
 }
 
-// The reduce-scatter of four per-lane double-float partial sums over a warp
-// (as the FP64 version in k_lanczos_cta): afterwards lanes 0, 8, 16 and 24
-// hold the warp totals of values 0..3, as doubles.
-__device__ __forceinline__ double warp_scatter4_df(const df* p, int lane) {
+// The warp totals of four double-floats per lane, value q in lanes 8 q ..
+// 8 q + 7 (as warp_scatter4_int).
+__device__ __forceinline__ df warp_scatter4_df(const df* p, int lane) {
   const bool b4 = lane & 16, b3 = lane & 8;
   const df r0 = shfl_xor_df(b4 ? p[0] : p[2], 16);
   const df r1 = shfl_xor_df(b4 ? p[1] : p[3], 16);
@@ -244,100 +168,228 @@ __device__ __forceinline__ double warp_scatter4_df(const df* p, int lane) {
   df kk = df_add(b3 ? k1 : k0, r2);
   kk = df_add(kk, shfl_xor_df(kk, 4));
   kk = df_add(kk, shfl_xor_df(kk, 2));
-  kk = df_add(kk, shfl_xor_df(kk, 1));
-  return widen(kk.hi) + widen(kk.lo);
+  return df_add(kk, shfl_xor_df(kk, 1));
+}
+
+__device__ __forceinline__ df warp_total(df v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = df_add(v, shfl_xor_df(v, o));
+  return v;
+}
+__device__ __forceinline__ double warp_total(double v) { return warp_sum_int(v); }
+__device__ __forceinline__ double as_double(df v) { return widen(v.hi) + widen(v.lo); }
+__device__ __forceinline__ double as_double(double v) { return v; }
+__device__ __forceinline__ float flip_sign(float v, uint32_t ent) {
+  return __uint_as_float(__float_as_uint(v) ^ (ent & 0x80000000u));
+}
+
+// 1 / sqrt(s): an FP32 start and two Newton steps y += y/2 (1 - s y^2) in the
+// range of FP32, rsqrt() outside it; 0 for s <= 0 or NaN.
+__device__ __forceinline__ double inv_sqrt(double s) {
+  const int e = (__double2hiint(s) >> 20);  // negative for s < 0
+  if (e > 1023 - 120 && e < 1023 + 120) {
+    const float r = rsqrtf(narrow(s));
+    double y = widen(r);
+    y = fma(widen(0.5f * r), fma(-s * y, y, 1.0), y);
+    return fma(0.5 * y, fma(-s * y, y, 1.0), y);
+  }
+  return (s > 0.0) ? rsqrt(s) : 0.0;
+}
+
+// Totals over a unit's CTAs of one value per thread.  Every warp adds its
+// lanes and leaves the total in slot [par][rank * warps + warp] of all CTAs of
+// the unit (CL = 2: its own and, through distributed shared memory, its
+// peer's); after one barrier warp 0 of each CTA adds the slots in that order,
+// so both CTAs hold bitwise the same sum (their control flow, which depends
+// only on such sums, stays identical), and its thread 0 calls root(sum)
+// before the block goes on.  `par` flips at every call, so a CTA running
+// ahead never overwrites slots that its peer has yet to read.
+template <int CL, class A, class Root>
+__device__ __forceinline__ void unit_reduce(A v, A (*slots)[CL * kWarpsCta], int& par, Root root) {
+  namespace cg = cooperative_groups;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  v = warp_total(v);
+  if constexpr (CL == 2) {
+    cg::cluster_group cl = cg::this_cluster();
+    const unsigned cr = cl.block_rank();
+    A* at = &slots[par][int(cr) * nw + wid];
+    if (lane == 0) {
+      *at = v;
+      *cl.map_shared_rank(at, cr ^ 1u) = v;
+    }
+    cl.sync();
+  } else {
+    if (lane == 0) slots[par][wid] = v;
+    __syncthreads();
+  }
+  if (wid == 0) {
+    A s;
+    if constexpr (std::is_same<A, df>::value) s = (lane < CL * nw) ? slots[par][lane] : df{0.f, 0.f};
+    else s = (lane < CL * nw) ? slots[par][lane] : 0.0;
+    s = warp_total(s);
+    if (lane == 0) root(as_double(s));
+  }
+  par ^= 1;
+  __syncthreads();
 }
 
 // One ground-state solve per unit of CL CTAs.  S: storage/matvec precision
 // of the Krylov basis (double, or float for the FP32-mixed path); R: rows
 // per thread held in registers (N <= CL * R * 512).  CL = 2 runs a unit on
 // a cluster of two CTAs: CTA rank c owns rows c R nthr .. (c + 1) R nthr - 1,
-// every reduction adds the two CTAs' totals in rank order (unit_sum and the
-// dot exchange), so both CTAs take the same branches at every step; each
-// CTA keeps the whole basis (a new vector's rows are stored into both CTAs'
-// shared memory, or once into the unit's global basis) and the cluster
-// barrier after each store orders it before the next product.
+// every reduction adds the warps' totals of both CTAs in one order
+// (unit_reduce and the dots), so both CTAs take the same branches at every
+// step; a new vector's rows go into both CTAs' copy of the current vector (or
+// once into the unit's global basis), which the cluster barrier after each
+// store orders before the next product.
+//
+// A step is bound by latency: a dependent FP64 operation takes 64 cycles, a
+// cluster barrier about a thousand.  So the sums over lanes and warps run in
+// double-float (mixed) or in integers (FP64: lgt_intsum.cuh), warp totals go
+// to both CTAs without a block barrier of their own, eight dots are reduced
+// together, and for R <= 4 the rows' neighbour lists sit in shared memory and
+// their diagonals in registers for the whole solve.  Cycles a step (4x2,
+// K = 64, clusters of two, R = 1), before -> after: mixed 21.9k -> 17.0k
+// (matvec 2.7 -> 1.2, dots 4.7 -> 4.1, their totals 2.8 -> 1.3, update 2.1 ->
+// 2.6, norm 4.0 -> 3.0, checks 4.0 -> 3.6); FP64 65.3k -> 33.3k (matvec 5.1 ->
+// 3.9, dots 15.8 -> 13.0, totals 4.1 -> 2.1, update 5.5 -> 6.3, norm 3.5 ->
+// 2.6, checks 29.3 -> 4.4).
 template <typename S, int R, int CL>
 __global__ void __launch_bounds__(kCta, 1) k_lanczos_cta(const SmallProblem* probs,
                                                       const SmallUnit* units, SmallParams prm) {
-  extern __shared__ __align__(16) unsigned char s_basis[];  // (m + 1) x N when prm.v_smem
-  __shared__ double s_alpha[kMaxM + 1], s_beta[kMaxM + 1], s_h[kMaxM + 1], s_z[kMaxM + 1];
-  __shared__ double s_part[kMaxM + 1][kWarpsCta];
-  __shared__ double s_red[kCta];
-  __shared__ double s_sum[3];  // block_sum results: sum, sqrt, 1 / sqrt
-  __shared__ int s_exh;        // the step's Krylov space is exhausted
+  // The FP32-mixed path (S = float) keeps the Lanczos residual as
+  // double-float pairs and runs its Gram-Schmidt dots, updates and norms in
+  // double-float arithmetic on the FP32 pipe (lgt_dfloat.cuh): FP64-class
+  // sums without GB300's narrow FP64 pipe.
+  constexpr bool kDF = sizeof(S) == 4;
+  constexpr bool kStage = R <= 4;
+  using A = typename std::conditional<kDF, df, double>::type;
+  extern __shared__ __align__(16) unsigned char s_dyn[];  // prm.v_smem: basis, vector; lists
+  __shared__ double s_alpha[kMaxM + 1], s_beta[kMaxM + 1], s_z[kMaxM + 1];
+  __shared__ A s_part[kMaxM + 2][CL * kWarpsCta];  // dot totals per slot and warp
+  __shared__ A s_nslot[2][CL * kWarpsCta];         // unit_reduce, the step's norms
+  __shared__ double s_dslot[2][CL * kWarpsCta];    // unit_reduce, FP64 sums
+  __shared__ double s_h[kDF ? 1 : kMaxM + 2];      // FP64 coefficients
+  __shared__ float s_hh[kDF ? kMaxM + 2 : 1], s_hl[kDF ? kMaxM + 2 : 1];  // mixed: FP32 pairs
+  __shared__ double s_sum[3];  // unit_reduce results: sum, sqrt, 1 / sqrt
+  __shared__ double s_nb;      // |w|^2 before the latest pass
+  __shared__ double s_thr;     // the step's space is exhausted when beta is not above it
+  __shared__ int s_exh, s_more;  // ... and whether; a further pass is needed
   __shared__ double s_work[3 * kMaxM];
   __shared__ double s_theta, s_resid;
   __shared__ int s_flag, s_zwarm;
   __shared__ int s_next, s_pstep;  // the next check's step; the previous check's step
   __shared__ double s_pres;        // and its residual
-  __shared__ double s_xch[4];                 // unit_sum exchange (CL = 2)
-  __shared__ double s_xh[2][2][kMaxM + 2];    // dot exchange [parity][rank][slot] (CL = 2)
-  int par_sum = 0, par_dot = 0;
+  __shared__ float s_rb[2];        // 1 / beta split into FP32 parts (mixed)
+  int par_n = 0, par_d = 0;
   const SmallUnit U = units[blockIdx.x / CL];
   const SmallProblem P = probs[U.prob];
   const int N = P.N;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int nthr = blockDim.x, nwarps = nthr >> 5;  // rows r = rbase + tid + i * nthr, i < R
   const int m = (prm.m < N) ? prm.m : N;
-  S* V = reinterpret_cast<S*>(prm.v_smem ? static_cast<void*>(s_basis) : U.V);
-  unsigned cr = 0;  // the CTA's rank in its unit
-  S* Vpeer = nullptr;  // the peer CTA's copy of the basis (CL = 2, basis in shared memory)
+  // The basis: in shared memory this CTA's rows alone, [m + 1][nthr R], with
+  // the whole current vector (for the gathers) behind it; else all rows in
+  // the unit's global basis, [m + 1][N].  Row i of this thread is vo + i nthr.
+  const bool vs = prm.v_smem != 0;
+  S* V = reinterpret_cast<S*>(vs ? static_cast<void*>(s_dyn) : U.V);
+  S* s_x = reinterpret_cast<S*>(s_dyn + prm.x_off);
+  unsigned cr = 0;      // the CTA's rank in its unit
+  S* xpeer = nullptr;   // the peer's s_x
+  A* ppeer = nullptr;   // the peer's s_part
   if constexpr (CL == 2) {
     cr = cooperative_groups::this_cluster().block_rank();
-    if (prm.v_smem) Vpeer = cooperative_groups::this_cluster().map_shared_rank(V, cr ^ 1u);
+    if (vs) xpeer = cooperative_groups::this_cluster().map_shared_rank(s_x, cr ^ 1u);
+    ppeer = cooperative_groups::this_cluster().map_shared_rank(&s_part[0][0], cr ^ 1u);
     // both CTAs running before either touches the other's shared memory
     cooperative_groups::this_cluster().sync();
   }
   const int rbase = int(cr) * nthr * R;
-  // a basis entry: into this CTA's basis and, with a split unit keeping the
-  // basis in shared memory, into the peer's copy
-  auto put_v = [&](size_t idx, S val) {
-    V[idx] = val;
-    if (CL == 2 && Vpeer) Vpeer[idx] = val;
+  const int vst = vs ? nthr * R : N;          // elements per basis vector
+  const int vo = (vs ? 0 : rbase) + tid;
+  // entry of basis vector b in this thread's row i (r in the sector)
+  auto put_v = [&](int b, int i, int r, S val) {
+    V[size_t(b) * vst + vo + i * nthr] = val;
+    if (vs) {
+      s_x[r] = val;
+      if (CL == 2) xpeer[r] = val;
+    }
   };
   // orders this unit's stores (basis, X) before any CTA of the unit reads them
   auto unit_sync = [&]() {
     if constexpr (CL == 2) cooperative_groups::this_cluster().sync();
     else __syncthreads();
   };
+  // thread 0's root: the sum, the norm and its reciprocal into s_sum
+  auto norm_root = [&](double sv) {
+    const double rs = inv_sqrt(sv);
+    s_sum[0] = sv;
+    s_sum[1] = sv * rs;
+    s_sum[2] = rs;
+  };
+  auto unit_sum = [&](double v) -> double {
+    unit_reduce<CL>(v, s_dslot, par_d, norm_root);
+    return s_sum[0];
+  };
+  auto zero = []() -> A {
+    if constexpr (kDF) return df{0.f, 0.f};
+    else return 0.0;
+  };
   const S cE = S(U.cE), cm = S(U.cm), ch = S(U.ch), cp = S(U.cp);
-  const bool fp32 = sizeof(S) == 4;
+  const bool fp32 = kDF;
   const double tiny_rel = fp32 ? 1e-6 : 1e-12;
   const double tol = fp32 ? fmax(prm.tol, 2e-5) : prm.tol;
 
-  // The FP32-mixed path (S = float) keeps the Lanczos residual as
-  // double-float pairs and runs its Gram-Schmidt dots, updates and norms in
-  // double-float arithmetic on the FP32 pipe (lgt_dfloat.cuh): FP64-class
-  // sums without GB300's narrow FP64 pipe.  The FP64 path is unchanged.
-  constexpr bool kDF = sizeof(S) == 4;
-  __shared__ float s_hh[kMaxM + 1], s_hl[kMaxM + 1];  // s_h split into FP32 pairs (kDF)
-  __shared__ float s_rb[2];                           // 1 / beta split likewise (kDF)
-  float wh[R], wl[R];  // this thread's residual rows as double-float pairs (kDF)
-  double w[R];  // this thread's rows of the current residual vector
+  // The CTA's neighbour lists: entries index | hop sign << 31, a row's hops
+  // first; rw[i]: the row's start, rn[i]: its hops | entries << 16.
+  const bool staged = kStage && prm.list_cap > 0;
+  uint32_t* s_list = reinterpret_cast<uint32_t*>(s_dyn + prm.list_off);
+  int rw[kStage ? R : 1], rn[kStage ? R : 1];
+  S dg[kStage ? R : 1];
+  if constexpr (kStage) {
+    const int rend = (rbase + nthr * R < N) ? rbase + nthr * R : N;
+    const int q0 = rbase < N ? P.rowptr[rbase] : 0;
+    if (staged && rbase < N) {
+      const int total = P.rowptr[rend] - q0;
+      for (int q = tid; q < total; q += nthr) {
+        const uint32_t e = P.nbr[q0 + q];
+        s_list[q] = (e >> 2) | ((e & 3u) == kHopNeg ? 0x80000000u : 0u);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const int r = rbase + tid + i * nthr;
+      rw[i] = rn[i] = 0;
+      dg[i] = S(0);
+      if (r < N) {
+        const int qa = P.rowptr[r], qb = P.rowptr[r + 1];
+        int nh = 0;
+        while (qa + nh < qb && (P.nbr[qa + nh] & 3u) != kPlaq) ++nh;
+        rw[i] = qa - q0;
+        rn[i] = nh | ((qb - qa) << 16);
+        dg[i] = cE * S(P.e2[r]) + cm * S(P.stag[r]);
+      }
+    }
+  }
+
+  A w[R];  // this thread's rows of the residual (mixed: double-float pairs)
+  double x[R];  // its rows of the start, Ritz and final vectors
   // start vector: normal(seed, k) into V_0, normalised
   double nrm = 0.0;
 #pragma unroll
   for (int i = 0; i < R; ++i) {
     const int r = rbase + tid + i * nthr;
-    w[i] = (r < N) ? (prm.start_given ? U.psi[size_t(r) * U.psi_stride]
+    x[i] = (r < N) ? (prm.start_given ? U.psi[size_t(r) * U.psi_stride]
                                       : start_normal(prm.seed, U.k, r))
                    : 0.0;
-    nrm += w[i] * w[i];
+    nrm += x[i] * x[i];
   }
-  // thread 0's root: the norm and its reciprocal into s_sum[1], s_sum[2]
-  // (one rsqrt: |x| = x^2 * rsqrt(x^2), both within an ulp or two)
-  auto norm_root = [&](double sv) {
-    const double rs = (sv > 0.0) ? rsqrt(sv) : 0.0;
-    s_sum[1] = sv * rs;
-    s_sum[2] = rs;
-  };
-  unit_sum<CL>(nrm, s_red, s_sum, s_xch, par_sum, norm_root);
+  unit_sum(nrm);
   nrm = s_sum[1];
 #pragma unroll
   for (int i = 0; i < R; ++i) {
     const int r = rbase + tid + i * nthr;
-    if (r < N) put_v(size_t(r), S(w[i] / nrm));
+    if (r < N) put_v(0, i, r, S(x[i] / nrm));
   }
   unit_sync();
 
@@ -355,206 +407,198 @@ __global__ void __launch_bounds__(kCta, 1) k_lanczos_cta(const SmallProblem* pro
     }
     __syncthreads();
     for (int j = 0; j < m; ++j) {
-      const S* vj = V + size_t(j) * N;
+      const S* vj = vs ? s_x : V + size_t(j) * N;
       // w = H v_j (matvec in the storage precision)
 #pragma unroll
       for (int i = 0; i < R; ++i) {
         const int r = rbase + tid + i * nthr;
+        S acc = S(0);
         if (r < N) {
-          S acc = (cE * S(P.e2[r]) + cm * S(P.stag[r])) * vj[r];
-          const int q1 = P.rowptr[r + 1];
-          for (int q = P.rowptr[r]; q < q1; ++q) {
-            const uint32_t e = __ldg(P.nbr + q);
-            const uint32_t kind = e & 3u;
-            const S c = (kind == kPlaq) ? cp : ((kind == kHopNeg) ? -ch : ch);
-            acc = fma(c, vj[e >> 2], acc);
+          bool done = false;
+          if constexpr (kStage) {
+            if (staged) {
+              const uint32_t* l = s_list + rw[i];
+              const int nh = rn[i] & 0xffff, n1 = rn[i] >> 16;
+              S sh = S(0), sp = S(0);
+              if constexpr (kDF) {
+                for (int q = 0; q < n1; q += 4) {
+                  uint32_t ent[4];
+                  float v[4];
+#pragma unroll
+                  for (int u = 0; u < 4; ++u) {
+                    ent[u] = (q + u < n1) ? l[q + u] : 0u;
+                    v[u] = (q + u < n1) ? float(vj[ent[u] & 0x7fffffffu]) : 0.f;
+                  }
+#pragma unroll
+                  for (int u = 0; u < 4; ++u) {
+                    if (q + u < nh) sh += flip_sign(v[u], ent[u]);
+                    else sp += v[u];
+                  }
+                }
+              } else {
+                double t[1];
+                auto load = [&](uint32_t e, double(&v)[1]) { v[0] = vj[e]; };
+                int_sum<1, 8, true>(l, 0, nh, t, load);
+                sh = S(t[0]);
+                if (n1 > nh) {
+                  int_sum<1, 8, false>(l, nh, n1, t, load);
+                  sp = S(t[0]);
+                }
+              }
+              acc = fma(ch, sh, dg[i] * vj[r]);
+              if (n1 > nh) acc = fma(cp, sp, acc);
+              done = true;
+            }
           }
-          if constexpr (kDF) {
-            wh[i] = float(acc);
-            wl[i] = 0.f;
-          } else {
-            w[i] = widen(acc);
-          }
-        } else {
-          if constexpr (kDF) {
-            wh[i] = 0.f;
-            wl[i] = 0.f;
-          } else {
-            w[i] = 0.0;
+          if (!done) {
+            acc = (cE * S(P.e2[r]) + cm * S(P.stag[r])) * vj[r];
+            const int q1 = P.rowptr[r + 1];
+            for (int q = P.rowptr[r]; q < q1; ++q) {
+              const uint32_t e = __ldg(P.nbr + q);
+              const uint32_t kind = e & 3u;
+              const S c = (kind == kPlaq) ? cp : ((kind == kHopNeg) ? -ch : ch);
+              acc = fma(c, vj[e >> 2], acc);
+            }
           }
         }
+        if constexpr (kDF) w[i] = df{float(acc), 0.f};
+        else w[i] = acc;
       }
       // Classical Gram-Schmidt against the whole basis V_0..V_j (which also
-      // performs the three-term recurrence), four basis vectors per round so
-      // four independent FP64 chains are in flight.  A further pass (up to
+      // performs the three-term recurrence), eight basis vectors per round so
+      // that their sums over the lanes overlap.  A further pass (up to
       // prm.reorth) runs only when a pass cancels more than two digits,
-      // ||w_after|| < 1e-2 ||w_before||: the rounding error it leaves along the
-      // basis is then above eps * 100 relative to w.
+      // ||w_after||^2 < 1e-4 ||w_before||^2: the rounding error it leaves along
+      // the basis is then above eps * 100 relative to w.
       // ||w||^2 before the first pass comes with that pass's dots: w against
       // itself in slot j + 1 (no separate block reduction)
-      double nb = 0.0, ss = 0.0;
-      for (int pass = 0; pass < prm.reorth; ++pass) {
+      for (int pass = 0;; ++pass) {
         const int jd = (pass == 0) ? j + 1 : j;
-        for (int b0 = 0; b0 <= jd; b0 += 4) {
-          if constexpr (kDF) {
-            df pd[4] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
+        for (int b0 = 0; b0 <= jd; b0 += 8) {
+          A pd[8];
 #pragma unroll
-            for (int i = 0; i < R; ++i) {
-              const int r = rbase + tid + i * nthr;
-              if (r < N) {
-#pragma unroll
-                for (int q = 0; q < 4; ++q)
-                  if (b0 + q <= j)
-                    df_fma2(pd[q], float(V[size_t(b0 + q) * N + r]), wh[i], wl[i]);
-                  else if (b0 + q == jd)
-                    df_sq2(pd[q], wh[i], wl[i]);
-              }
-            }
-            const double kk = warp_scatter4_df(pd, lane);
-            const int qv = lane >> 3;  // lanes 0, 8, 16, 24 hold values 0..3
-            if ((lane & 7) == 0 && b0 + qv <= jd) s_part[b0 + qv][wid] = kk;
-            continue;
-          }
-          double p[4] = {0.0, 0.0, 0.0, 0.0};
+          for (int q = 0; q < 8; ++q) pd[q] = zero();
 #pragma unroll
           for (int i = 0; i < R; ++i) {
             const int r = rbase + tid + i * nthr;
             if (r < N) {
+              S v[8];
 #pragma unroll
-              for (int q = 0; q < 4; ++q)
-                if (b0 + q <= jd) {
-                  const double vq = (b0 + q <= j) ? widen(V[size_t(b0 + q) * N + r]) : w[i];
-                  p[q] = fma(vq, w[i], p[q]);
+              for (int q = 0; q < 8; ++q)
+                v[q] = (b0 + q <= j) ? V[size_t(b0 + q) * vst + vo + i * nthr] : S(0);
+#pragma unroll
+              for (int q = 0; q < 8; ++q) {
+                if constexpr (kDF) {
+                  if (b0 + q <= j) df_fma2(pd[q], v[q], w[i].hi, w[i].lo);
+                  else if (b0 + q == jd) df_sq2(pd[q], w[i].hi, w[i].lo);
+                } else {
+                  if (b0 + q <= j) pd[q] = fma(v[q], w[i], pd[q]);
+                  else if (b0 + q == jd) pd[q] = fma(w[i], w[i], pd[q]);
+                }
+              }
+            }
+          }
+#pragma unroll
+          for (int g = 0; g < 8; g += 4)
+            if (b0 + g <= jd) {
+              A kk;
+              if constexpr (kDF) kk = warp_scatter4_df(pd + g, lane);
+              else kk = warp_scatter4_int(pd + g, lane);
+              const int slot = b0 + g + (lane >> 3);
+              if ((lane & 7) == 0 && slot <= jd) {
+                const int at = int(cr) * nwarps + wid;
+                s_part[slot][at] = kk;
+                if (CL == 2) ppeer[slot * (CL * kWarpsCta) + at] = kk;
+              }
+            }
+        }
+        unit_sync();
+        // eight lanes add a slot's totals of all warps of the unit
+        const int nv = CL * nwarps, ngrp = nthr >> 3, sub = tid & 7;
+        for (int s0 = 0; s0 <= jd; s0 += ngrp) {
+          const int slot = s0 + (tid >> 3);
+          A v = zero();
+          if (slot <= jd)
+            for (int q = sub; q < nv; q += 8) {
+              if constexpr (kDF) v = df_add(v, s_part[slot][q]);
+              else v += s_part[slot][q];
+            }
+#pragma unroll
+          for (int o = 4; o > 0; o >>= 1) {
+            if constexpr (kDF) v = df_add(v, shfl_xor_df(v, o));
+            else v += __shfl_xor_sync(0xffffffffu, v, o);
+          }
+          if (slot <= jd && sub == 0) {
+            if constexpr (kDF) {
+              s_hh[slot] = v.hi;
+              s_hl[slot] = v.lo;
+            } else {
+              s_h[slot] = v;
+            }
+            if (slot == j) s_alpha[j] = (pass == 0) ? as_double(v) : s_alpha[j] + as_double(v);
+            if (slot == j + 1) s_nb = as_double(v);
+          }
+        }
+        __syncthreads();
+        if (tid == nthr - 1) {  // for thread 0 after the next barrier
+          double scl = fabs(s_alpha[j]);
+          if (j > 0) scl = fmax(scl, s_beta[j - 1]);
+          s_thr = tiny_rel * fmax(scl, 1.0);
+        }
+        // w -= sum_b h_b V_b.  Mixed: the leading parts by TwoSum, the
+        // trailing parts apart, renormalised at the end (Dot2 form)
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+          const int r = rbase + tid + i * nthr;
+          if (r < N) {
+            for (int b0 = 0; b0 <= j; b0 += 8) {
+              S v[8];
+#pragma unroll
+              for (int q = 0; q < 8; ++q)
+                v[q] = (b0 + q <= j) ? V[size_t(b0 + q) * vst + vo + i * nthr] : S(0);
+#pragma unroll
+              for (int q = 0; q < 8; ++q)
+                if (b0 + q <= j) {
+                  if constexpr (kDF) {
+                    float p, e, t;
+                    two_prod(s_hh[b0 + q], v[q], p, e);
+                    e = df_fma_rn(s_hl[b0 + q], v[q], e);
+                    two_sum(w[i].hi, -p, w[i].hi, t);
+                    w[i].lo = df_add_rn(w[i].lo, df_sub_rn(t, e));
+                  } else {
+                    w[i] = fma(-s_h[b0 + q], v[q], w[i]);
+                  }
                 }
             }
-          }
-          // reduce-scatter over the warp: after the xor-16 and xor-8 steps
-          // lane l holds value 2 * bit4(l) + bit3(l) summed over 4 lanes, the
-          // last three steps finish it (6 FP64 adds per lane instead of 20)
-          const bool b4 = lane & 16, b3 = lane & 8;
-          const double r0 = __shfl_xor_sync(0xffffffffu, b4 ? p[0] : p[2], 16);
-          const double r1 = __shfl_xor_sync(0xffffffffu, b4 ? p[1] : p[3], 16);
-          const double k0 = (b4 ? p[2] : p[0]) + r0, k1 = (b4 ? p[3] : p[1]) + r1;
-          const double r2 = __shfl_xor_sync(0xffffffffu, b3 ? k0 : k1, 8);
-          double kk = (b3 ? k1 : k0) + r2;
-          kk += __shfl_xor_sync(0xffffffffu, kk, 4);
-          kk += __shfl_xor_sync(0xffffffffu, kk, 2);
-          kk += __shfl_xor_sync(0xffffffffu, kk, 1);
-          const int qv = lane >> 3;  // lanes 0, 8, 16, 24 hold values 0..3
-          if ((lane & 7) == 0 && b0 + qv <= jd) s_part[b0 + qv][wid] = kk;
-        }
-        __syncthreads();
-        if constexpr (CL == 2) {
-          // this CTA's dot totals into slot [par][rank] of both CTAs
-          if (tid <= jd) {
-            double s0 = 0.0, s1 = 0.0;
-            int ww = 0;
-            for (; ww + 1 < nwarps; ww += 2) {
-              s0 += s_part[tid][ww];
-              s1 += s_part[tid][ww + 1];
-            }
-            if (ww < nwarps) s0 += s_part[tid][ww];
-            s_xh[par_dot][cr][tid] = s0 + s1;
-            cooperative_groups::this_cluster().map_shared_rank(&s_xh[par_dot][cr][tid],
-                                                               cr ^ 1u)[0] = s0 + s1;
-          }
-          cooperative_groups::this_cluster().sync();
-        }
-        if (tid <= jd) {
-          double sum;
-          if constexpr (CL == 2) {
-            sum = s_xh[par_dot][0][tid] + s_xh[par_dot][1][tid];
-          } else {
-            double s0 = 0.0, s1 = 0.0;
-            int ww = 0;
-            for (; ww + 1 < nwarps; ww += 2) {
-              s0 += s_part[tid][ww];
-              s1 += s_part[tid][ww + 1];
-            }
-            if (ww < nwarps) s0 += s_part[tid][ww];
-            sum = s0 + s1;
-          }
-          s_h[tid] = sum;
-          if (tid == j) s_alpha[j] = (pass == 0) ? sum : s_alpha[j] + sum;
-          if (kDF) {  // the update's coefficients as FP32 pairs, once per block
-            const float hh = narrow(sum);
-            s_hh[tid] = hh;
-            s_hl[tid] = narrow(sum - widen(hh));
+            if constexpr (kDF) fast_two_sum(w[i].hi, w[i].lo, w[i].hi, w[i].lo);
           }
         }
-        par_dot ^= 1;
-        __syncthreads();
-        if (pass == 0) nb = ss = s_h[j + 1];
-        if constexpr (kDF) {
-          for (int b0 = 0; b0 <= j; b0 += 4) {
-            float hh[4], hl[4];
+        A n2 = zero();
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              hh[q] = (b0 + q <= j) ? s_hh[b0 + q] : 0.f;
-              hl[q] = (b0 + q <= j) ? s_hl[b0 + q] : 0.f;
-            }
-#pragma unroll
-            for (int i = 0; i < R; ++i) {
-              const int r = rbase + tid + i * nthr;
-              if (r < N) {
-                df x{wh[i], wl[i]};
-#pragma unroll
-                for (int q = 0; q < 4; ++q)
-                  if (b0 + q <= j) df_sub_prod(x, hh[q], hl[q], float(V[size_t(b0 + q) * N + r]));
-                wh[i] = x.hi;
-                wl[i] = x.lo;
-              }
-            }
-          }
+        for (int i = 0; i < R; ++i) {
+          if constexpr (kDF) df_sq2(n2, w[i].hi, w[i].lo);
+          else n2 = fma(w[i], w[i], n2);
         }
-        for (int b0 = 0; !kDF && b0 <= j; b0 += 4) {
-          double h4[4];
-#pragma unroll
-          for (int q = 0; q < 4; ++q) h4[q] = (b0 + q <= j) ? s_h[b0 + q] : 0.0;
-#pragma unroll
-          for (int i = 0; i < R; ++i) {
-            const int r = rbase + tid + i * nthr;
-            if (r < N) {
-#pragma unroll
-              for (int q = 0; q < 4; ++q)
-                if (b0 + q <= j) w[i] = fma(-h4[q], widen(V[size_t(b0 + q) * N + r]), w[i]);
-            }
-          }
-        }
-        double s1 = 0.0;
-        if constexpr (kDF) {
-          df n2{0.f, 0.f};
-#pragma unroll
-          for (int i = 0; i < R; ++i) df_sq2(n2, wh[i], wl[i]);
-          s1 = widen(n2.hi) + widen(n2.lo);
-        } else {
-#pragma unroll
-          for (int i = 0; i < R; ++i) s1 = fma(w[i], w[i], s1);
-        }
-        // beta = ||w||, 1 / beta and the exhaustion test of this step, by
-        // thread 0 (alpha_j is final: the pass's reduction synchronised)
-        ss = unit_sum<CL>(s1, s_red, s_sum, s_xch, par_sum, [&](double sv) {
-          const double rs = (sv > 0.0) ? rsqrt(sv) : 0.0;
+        // beta = ||w||, 1 / beta, the exhaustion test of this step and the
+        // need of a further pass, by thread 0
+        unit_reduce<CL>(n2, s_nslot, par_n, [&](double sv) {
+          const double rs = inv_sqrt(sv);
           const double b = sv * rs;
-          s_sum[1] = b;
+          s_beta[j] = b;
           s_sum[2] = rs;
           if (kDF) {
             const float rh = narrow(rs);
             s_rb[0] = rh;
             s_rb[1] = narrow(rs - widen(rh));
           }
-          double scl = fabs(s_alpha[j]);
-          if (j > 0) scl = fmax(scl, s_beta[j - 1]);
-          s_exh = (b > tiny_rel * fmax(scl, 1.0)) ? 0 : 1;
+          s_exh = (b > s_thr) ? 0 : 1;
+          // high words as logarithms: 1e-4 is 13.3 binades
+          s_more = __double2hiint(sv) < __double2hiint(s_nb) - 13933000 ? 1 : 0;
+          s_nb = sv;
         });
-        if (!(ss < 1e-4 * nb)) break;
-        nb = ss;
+        if (!s_more || pass + 1 >= prm.reorth) break;
       }
-      // beta = sqrt(ss) and the exhaustion flag from the last pass's block_sum
-      // (reorth_passes >= 1: at least one pass ran)
-      const double beta = s_sum[1];
       const double rbeta = s_sum[2];
-      if (tid == 0) s_beta[j] = beta;
       n = j + 1;
       ++steps;
       if (s_exh) {
@@ -567,11 +611,11 @@ __global__ void __launch_bounds__(kCta, 1) k_lanczos_cta(const SmallProblem* pro
             // (wh + wl)(rh + rl) to FP32: the leading product and the two
             // cross terms, one final rounding
             if (r < N)
-              put_v(size_t(j + 1) * N + r,
-                    S(df_fma_rn(wh[i], s_rb[0],
-                                df_fma_rn(wh[i], s_rb[1], df_mul_rn(wl[i], s_rb[0])))));
+              put_v(j + 1, i, r,
+                    S(df_fma_rn(w[i].hi, s_rb[0],
+                                df_fma_rn(w[i].hi, s_rb[1], df_mul_rn(w[i].lo, s_rb[0])))));
           } else {
-            if (r < N) put_v(size_t(j + 1) * N + r, to_storage<S>(w[i] * rbeta));
+            if (r < N) put_v(j + 1, i, r, to_storage<S>(w[i] * rbeta));
           }
         }
       }
@@ -585,14 +629,14 @@ __global__ void __launch_bounds__(kCta, 1) k_lanczos_cta(const SmallProblem* pro
           double th, rr = 0.0;
           bool conv = false;
           if constexpr (kDF) {
-            th = warp_lowest_eig_f32(s_alpha, s_beta, n, s_z, s_work, s_zwarm != 0, s_zwarm != 0,
-                                     s_theta, s_resid);
+            th = warp_check_lowest_f32(s_alpha, s_beta, n, s_beta[n - 1], s_zwarm != 0, s_theta,
+                                       s_resid, s_z, s_work, &rr);
           } else {
             conv = warp_check_lowest(s_alpha, s_beta, n, s_beta[n - 1], tol,
-                                     exhausted || j + 1 == m, s_z, s_work, &th, &rr);
+                                     exhausted || j + 1 == m, s_zwarm != 0, s_theta, s_resid, s_z,
+                                     s_work, &th, &rr);
           }
           if (lane == 0) {
-            if constexpr (kDF) rr = fabs(s_beta[n - 1] * s_z[n - 1]);
             if (exhausted) rr = 0.0;
             // FP32 panels resolve residuals to ~1e-6 |H|: relative floor
             const double tl = fp32 ? fmax(tol, 3e-6 * fmax(fabs(th), 1.0)) : tol;
@@ -635,22 +679,23 @@ __global__ void __launch_bounds__(kCta, 1) k_lanczos_cta(const SmallProblem* pro
       const int r = rbase + tid + i * nthr;
       double xv = 0.0;
       if (r < N)
-        for (int b = 0; b < n; ++b) xv = fma(s_z[b], widen(V[size_t(b) * N + r]), xv);
-      w[i] = xv;
+        for (int b = 0; b < n; ++b)
+          xv = fma(s_z[b], widen(V[size_t(b) * vst + vo + i * nthr]), xv);
+      x[i] = xv;
     }
     if (converged || cycle >= prm.maxiter) break;
     // restart from the Ritz vector
     double s2 = 0.0;
 #pragma unroll
-    for (int i = 0; i < R; ++i) s2 = fma(w[i], w[i], s2);
-    unit_sum<CL>(s2, s_red, s_sum, s_xch, par_sum, norm_root);
+    for (int i = 0; i < R; ++i) s2 = fma(x[i], x[i], s2);
+    unit_sum(s2);
     const double xn = s_sum[1];
     // every CTA of the unit has formed its Ritz rows from the old basis
     unit_sync();
 #pragma unroll
     for (int i = 0; i < R; ++i) {
       const int r = rbase + tid + i * nthr;
-      if (r < N) put_v(size_t(r), S(w[i] / xn));
+      if (r < N) put_v(0, i, r, S(x[i] / xn));
     }
     unit_sync();
     ++restarts;
@@ -659,15 +704,15 @@ __global__ void __launch_bounds__(kCta, 1) k_lanczos_cta(const SmallProblem* pro
   // FP64 finish: x normalised, y = H x in FP64, E = <x|y>, ||y - E x||
   double s2 = 0.0;
 #pragma unroll
-  for (int i = 0; i < R; ++i) s2 = fma(w[i], w[i], s2);
-  unit_sum<CL>(s2, s_red, s_sum, s_xch, par_sum, norm_root);
+  for (int i = 0; i < R; ++i) s2 = fma(x[i], x[i], s2);
+  unit_sum(s2);
   const double xn = s_sum[1];
   double* X = U.x;
 #pragma unroll
   for (int i = 0; i < R; ++i) {
     const int r = rbase + tid + i * nthr;
-    w[i] /= xn;
-    if (r < N) X[r] = w[i];
+    x[i] /= xn;
+    if (r < N) X[r] = x[i];
   }
   unit_sync();
   double y[R];
@@ -678,30 +723,48 @@ __global__ void __launch_bounds__(kCta, 1) k_lanczos_cta(const SmallProblem* pro
     y[i] = 0.0;
     if (r < N) {
       double acc = (U.cE * double(P.e2[r]) + U.cm * double(P.stag[r])) * X[r];
-      const int q1 = P.rowptr[r + 1];
-      for (int q = P.rowptr[r]; q < q1; ++q) {
-        const uint32_t e = __ldg(P.nbr + q);
-        const uint32_t kind = e & 3u;
-        const double c = (kind == kPlaq) ? U.cp : ((kind == kHopNeg) ? -U.ch : U.ch);
-        acc = fma(c, X[e >> 2], acc);
+      bool done = false;
+      if constexpr (kStage) {
+        if (staged) {
+          const uint32_t* l = s_list + rw[i];
+          const int nh = rn[i] & 0xffff, n1 = rn[i] >> 16;
+          double t[1];
+          auto load = [&](uint32_t e, double(&v)[1]) { v[0] = X[e]; };
+          int_sum<1, 8, true>(l, 0, nh, t, load);
+          acc = fma(U.ch, t[0], acc);
+          if (n1 > nh) {
+            int_sum<1, 8, false>(l, nh, n1, t, load);
+            acc = fma(U.cp, t[0], acc);
+          }
+          done = true;
+        }
+      }
+      if (!done) {
+        const int q1 = P.rowptr[r + 1];
+        for (int q = P.rowptr[r]; q < q1; ++q) {
+          const uint32_t e = __ldg(P.nbr + q);
+          const uint32_t kind = e & 3u;
+          const double c = (kind == kPlaq) ? U.cp : ((kind == kHopNeg) ? -U.ch : U.ch);
+          acc = fma(c, X[e >> 2], acc);
+        }
       }
       y[i] = acc;
     }
-    ey = fma(w[i], y[i], ey);
+    ey = fma(x[i], y[i], ey);
   }
-  const double Erq = unit_sum<CL>(ey, s_red, s_sum, s_xch, par_sum);
+  const double Erq = unit_sum(ey);
   double rs = 0.0;
 #pragma unroll
   for (int i = 0; i < R; ++i) {
-    const double d = y[i] - Erq * w[i];
+    const double d = y[i] - Erq * x[i];
     rs = fma(d, d, rs);
   }
-  unit_sum<CL>(rs, s_red, s_sum, s_xch, par_sum, norm_root);
+  unit_sum(rs);
   const double rnorm = s_sum[1];
 #pragma unroll
   for (int i = 0; i < R; ++i) {
     const int r = rbase + tid + i * nthr;
-    if (r < N) U.psi[size_t(r) * U.psi_stride] = w[i];
+    if (r < N) U.psi[size_t(r) * U.psi_stride] = x[i];
   }
   if (tid == 0 && cr == 0) {
     U.out[0] = fp32 ? Erq : theta;
@@ -743,14 +806,28 @@ cudaError_t launch_cta(const SmallProblem* probs, const SmallUnit* units, int nu
     int t = ((rowsN + rr - 1) / rr + 31) / 32 * 32;
     return t < 64 ? 64 : t;  // the reduction of step j uses threads 0..j
   };
-  // Krylov basis of every unit in shared memory when the largest fits
+  // shared memory: a CTA's rows of the Krylov basis with the current vector,
+  // and its neighbour lists (R <= 4), each when the largest sector's fit
   SmallParams prm = prm_in;
   const int mmax = (prm.m < maxN) ? prm.m : maxN;
-  const size_t vbytes = size_t(mmax + 1) * size_t(maxN) * sizeof(S);
-  const bool smem = getenv_flag("LGT_CTA_BASIS_SMEM", 1) && vbytes <= size_t(kCtaSmemMax);
-  prm.v_smem = smem ? 1 : 0;
-  const int dyn = smem ? int((vbytes + 15) / 16 * 16) : 0;
+  auto up = [](size_t b) { return (b + 15) / 16 * 16; };
+  auto layout = [&](int rr) -> int {
+    const size_t rows = size_t(threads_for(rr)) * rr;
+    const size_t vb = up(size_t(mmax + 1) * rows * sizeof(S)), xb = up(size_t(maxN) * sizeof(S));
+    const size_t lb =
+        (rr <= 4 && prm.max_moves > 0)
+            ? up(std::min(rows, size_t(maxN)) * size_t(prm.max_moves) * sizeof(uint32_t))
+            : 0;
+    size_t o = 0;
+    prm.v_smem = getenv_flag("LGT_CTA_BASIS_SMEM", 1) && vb + xb <= size_t(kCtaSmemMax) ? 1 : 0;
+    prm.x_off = int(vb);
+    if (prm.v_smem) o = vb + xb;
+    prm.list_cap = lb > 0 && o + lb <= size_t(kCtaSmemMax) ? 1 : 0;
+    prm.list_off = int(o);
+    return int(o + (prm.list_cap ? lb : 0));
+  };
   auto go = [&](auto kern, int rr) -> cudaError_t {
+    const int dyn = layout(rr);
     if (dyn > 0) {  // static + dynamic may pass 48 KB: opt in per device
       cudaError_t ea = lgt::raise_smem_limit(reinterpret_cast<const void*>(kern), kCtaSmemMax);
       if (ea != cudaSuccess) return ea;
@@ -798,6 +875,7 @@ std::string build_pattern(const BasisDev& B, uint32_t model, Pattern* P, cudaStr
   if (N > kSmallMaxN) return "sector too large for the per-CTA solver";
   P->N = int(N);
   P->model = model;
+  P->max_moves = B.G.max_moves > 0 ? B.G.max_moves : 1;
   // Stream-ordered: the neighbour array is sized for the most moves a row can
   // have (at most kSmallMaxN rows, so a few MB at most) instead of reading
   // the exact count back; the fill kernel checks its bounds.
@@ -860,10 +938,13 @@ void free_pattern(Pattern* P, cudaStream_t s) {
   *P = Pattern();
 }
 
-std::string small_ground_states(const std::vector<SmallJob>& jobs, const SmallParams& prm,
+std::string small_ground_states(const std::vector<SmallJob>& jobs, const SmallParams& prm_in,
                                 int mixed, SmallWork* ws, cudaStream_t s, double* seconds,
                                 const int* dev_err, int* err_out,
                                 const std::function<cudaError_t()>& before_sync) {
+  SmallParams prm = prm_in;
+  for (const SmallJob& jb : jobs)
+    prm.max_moves = std::max(prm.max_moves, jb.pattern->max_moves);
   // problems and units, the largest sectors first
   std::vector<SmallProblem> probs;
   std::vector<SmallUnit> units;
