@@ -985,7 +985,8 @@ __global__ void k_check_lowest(const double* alpha, const double* beta, int ldT,
   // count in FP32 (its basis resolves no more), bracket warm-started from
   // this point's previous theta and residual (verified by Sturm counts, so
   // stale values only cost the fallback to the Gershgorin interval)
-  __shared__ double s_a[kMaxDim], s_b[kMaxDim], s_z[kMaxDim], s_work[3 * kMaxDim];
+  __shared__ double s_a[kMaxDim], s_b[kMaxDim], s_z[kMaxDim];
+  __shared__ __align__(16) double s_work[3 * kMaxDim];
   const int k = blockIdx.x, lane = threadIdx.x;
   const int st = status[k];
   if (st >= kConverged) return;

@@ -100,7 +100,8 @@ __global__ void __launch_bounds__(Threads<S>::n, 1) k_lanczos_grid(GridArgs<S> a
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ int s_n, s_bad;
   __shared__ S s_int[256], s_stag[256];  // small integers: conversions to FP64 are slow
-  __shared__ double s_ta[kTriMax], s_tb[kTriMax], s_tz[kTriMax], s_work[3 * kTriMax];
+  __shared__ double s_ta[kTriMax], s_tb[kTriMax], s_tz[kTriMax];
+  __shared__ __align__(16) double s_work[3 * kTriMax];
   const Layout L = layout<S>(a.rpb, a.C, a.m, a.mm, a.list_smem);
   S* s_W = reinterpret_cast<S*>(smem + L.W);
   S* s_lo = s_W + a.rpb * a.C;  // (FP32 only)

@@ -120,36 +120,45 @@ __device__ __forceinline__ double warp_sum_int(double v) {
   return fix_to(x, eb);
 }
 
-// The warp totals of four doubles per lane, value q in lanes 8 q .. 8 q + 7
-// (reduce-scatter: two exchange steps halve the values, three finish them).
-__device__ __forceinline__ double warp_scatter4_int(const double* p, int lane) {
-  const bool b4 = lane & 16, b3 = lane & 8;
-  int top[4];
+// The warp totals of eight values per lane, value q in lanes 4 q .. 4 q + 3:
+// three exchange steps halve the values, two finish them.  add(x, y), and
+// shfl(x, lane mask), of type A.
+template <class A, class Add, class Shfl>
+__device__ __forceinline__ A warp_scatter8(const A* p, int lane, Add add, Shfl shfl) {
+  const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
+  A k[4], h[2];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) k[q] = add(b4 ? p[q + 4] : p[q], shfl(b4 ? p[q] : p[q + 4], 16));
+#pragma unroll
+  for (int q = 0; q < 2; ++q) h[q] = add(b3 ? k[q + 2] : k[q], shfl(b3 ? k[q] : k[q + 2], 8));
+  A v = add(b2 ? h[1] : h[0], shfl(b2 ? h[0] : h[1], 4));
+  v = add(v, shfl(v, 2));
+  return add(v, shfl(v, 1));
+}
+
+// The same for doubles, by integers where their ranges allow.
+__device__ __forceinline__ double warp_scatter8_int(const double* p, int lane) {
+  int top[8];
   bool ok = true;
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
+  for (int q = 0; q < 8; ++q) {
     top[q] = int(__reduce_max_sync(0xffffffffu, uint32_t(__double2hiint(p[q])) & 0x7fffffffu));
     ok = ok && (top[q] == 0 || fix_range(top[q]));
   }
-  if (!ok) {
-    const double r0 = __shfl_xor_sync(0xffffffffu, b4 ? p[0] : p[2], 16);
-    const double r1 = __shfl_xor_sync(0xffffffffu, b4 ? p[1] : p[3], 16);
-    const double k0 = (b4 ? p[2] : p[0]) + r0, k1 = (b4 ? p[3] : p[1]) + r1;
-    double kk = (b3 ? k1 : k0) + __shfl_xor_sync(0xffffffffu, b3 ? k0 : k1, 8);
+  if (!ok)
+    return warp_scatter8<double>(
+        p, lane, [](double x, double y) { return x + y; },
+        [](double x, int o) { return __shfl_xor_sync(0xffffffffu, x, o); });
+  long long x[8];
 #pragma unroll
-    for (int o = 4; o > 0; o >>= 1) kk += __shfl_xor_sync(0xffffffffu, kk, o);
-    return kk;
-  }
-  long long x[4];
+  for (int q = 0; q < 8; ++q) x[q] = top[q] == 0 ? 0 : fix_of(p[q], top[q] & 0x7ff00000);
+  const long long v = warp_scatter8<long long>(
+      x, lane, [](long long y, long long z) { return y + z; },
+      [](long long y, int o) { return __shfl_xor_sync(0xffffffffu, y, o); });
+  int t = top[0];
 #pragma unroll
-  for (int q = 0; q < 4; ++q) x[q] = top[q] == 0 ? 0 : fix_of(p[q], top[q] & 0x7ff00000);
-  const long long r0 = __shfl_xor_sync(0xffffffffu, b4 ? x[0] : x[2], 16);
-  const long long r1 = __shfl_xor_sync(0xffffffffu, b4 ? x[1] : x[3], 16);
-  const long long k0 = (b4 ? x[2] : x[0]) + r0, k1 = (b4 ? x[3] : x[1]) + r1;
-  long long kk = (b3 ? k1 : k0) + __shfl_xor_sync(0xffffffffu, b3 ? k0 : k1, 8);
-#pragma unroll
-  for (int o = 4; o > 0; o >>= 1) kk += __shfl_xor_sync(0xffffffffu, kk, o);
-  return fix_to(kk, (b4 ? (b3 ? top[3] : top[2]) : (b3 ? top[1] : top[0])) & 0x7ff00000);
+  for (int q = 1; q < 8; ++q) t = (lane >> 2) == q ? top[q] : t;
+  return fix_to(v, t & 0x7ff00000);
 }
 
 // int_sum_part for any number of entries.

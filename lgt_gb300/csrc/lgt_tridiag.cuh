@@ -401,11 +401,16 @@ __device__ inline double warp_lowest_eig_f32(const double* a64, const double* b6
 //     even a tail component of 1e-13 has a few FP32 ulps per factor, and the
 //     residual |beta_n z_n| is known to about 1e-5 of itself.
 // Only a converged check, or one that must hand out the vector, goes on to
-// FP64: defect correction, the residual (T - theta) z in FP64 by all lanes,
+// FP64: one inverse iteration in FP32, then defect correction, the residual (T - theta) z in FP64 by all lanes,
 // the correction from the FP32 pivots (projected against z), about six digits
 // a round.  Clustered lowest eigenvalues (a second one within 4e-6 of the
-// spread), ranges FP32 cannot hold and corrections that stall take
-// warp_lowest_eig instead.
+// spread), a start vector with less than 1e-5 of the state (the ratios' tail
+// is 10 % low there), ranges FP32 cannot hold and corrections that stall take
+// warp_lowest_eig instead, at 260k (n = 33) to 440k cycles (n = 60), so none
+// of these may be common: among 64 points of random start vectors one in two
+// batches has a share below 1e-3 (whose pivots FP32 rounds to 10 % and the
+// inverse iteration puts right).  A check (n = 25, warm): not converged 7.6k
+// cycles (15.1k with the branching count), converged 28k; mixed 9.8k (18.2k).
 __device__ __forceinline__ float warp_max_f(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
@@ -460,55 +465,94 @@ __device__ __forceinline__ void pivot_solve(const float* bf, const float* ru, in
   }
 }
 
+// Whether the tridiagonal with diagonal d and squared couplings e (e[i]
+// between i - 1 and i, e[0] = 0) has an eigenvalue below x: some leading minor
+// of T - x is negative.  Arrays padded to a multiple of four with d = 8, e = 0
+// and scaled to a spread of 1 to 2, so that four steps stay in range between
+// the exact rescalings; no branches (the general count took 100 cycles a row).
+__device__ __forceinline__ bool below_scaled(const float* d, const float* e, int n, float x) {
+  float p0 = 0.0f, p1 = 1.0f;
+  int neg = 0;
+  for (int i = 0; i < n; i += 4) {
+    const float4 D = *reinterpret_cast<const float4*>(d + i);
+    const float4 E = *reinterpret_cast<const float4*>(e + i);
+    const float q0 = fmaf(D.x - x, p1, -E.x * p0);
+    const float q1 = fmaf(D.y - x, q0, -E.y * p1);
+    p0 = fmaf(D.z - x, q1, -E.z * q0);
+    p1 = fmaf(D.w - x, p0, -E.w * q1);
+    neg |= __float_as_int(q0) | __float_as_int(q1) | __float_as_int(p0) | __float_as_int(p1);
+    const int m =
+        max(__float_as_int(p0) & 0x7f800000, __float_as_int(p1) & 0x7f800000);
+    const float sc = __int_as_float(0x7f000000 - m);
+    p0 *= sc;
+    p1 *= sc;
+  }
+  return neg < 0;
+}
+
 // FP32 part: true when the FP32 data describe T's lowest pair (see above);
 // theta relative to a[0] (*th), the vector's residual factor |z_{n-1}| / |z|
-// (*tail), and in work: d, b, b^2, the reciprocal pivots and the normalised
-// vector (five arrays of kTriMax floats).  warm: th_prev, r_prev are an
-// earlier check's theta and residual; the lowest value lies in [th_prev -
-// 2 r_prev, th_prev] unless the counts at its ends say otherwise.
+// (*tail), the power of two (*scale) that the FP32 matrix is T - a[0] times,
+// and in work (16-byte aligned): its diagonal, squared couplings, couplings,
+// reciprocal pivots and the normalised vector (five arrays of kTriMax
+// floats).  warm: th_prev, r_prev are an earlier check's theta and residual;
+// the lowest value lies in [th_prev - 2 r_prev, th_prev] unless the counts at
+// its ends say otherwise.
 __device__ inline bool warp_lowest_f32_pivots(const double* a, const double* b, int n,
                                               float* work, bool warm, double th_prev,
                                               double r_prev, float* th, float* tail,
-                                              float* spread) {
+                                              float* spread, float* scale) {
   const int lane = threadIdx.x & 31;
   float* d = work;
-  float* bf = d + kTriMax;
-  float* bb = bf + kTriMax;
-  float* ru = bb + kTriMax;
+  float* ee = d + kTriMax;
+  float* bf = ee + kTriMax;
+  float* ru = bf + kTriMax;
   float* zf = ru + kTriMax;
   const double c0 = a[0];
-  float R = 0.0f;
-  for (int i = lane; i < n; i += 32) {
-    const float di = float(a[i] - c0);
-    const float bi = (i < n - 1) ? float(b[i]) : 0.0f;
-    d[i] = di;
-    bf[i] = bi;
-    bb[i] = bi * bi;
-    R = fmaxf(R, fabsf(di) + 2.0f * fabsf(bi));
+  // rows lane and lane + 32: diagonal and the couplings on both sides
+  float dv[2], bl[2], br[2];
+  float lo = 3.0e38f, hi = -3.0e38f;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int i = lane + 32 * h;
+    dv[h] = (i < n) ? float(a[i] - c0) : 0.0f;
+    br[h] = (i < n - 1) ? float(b[i]) : 0.0f;
+    bl[h] = (i > 0 && i < n) ? float(b[i - 1]) : 0.0f;
+    if (i < n) {
+      const float r = fabsf(bl[h]) + fabsf(br[h]);
+      lo = fminf(lo, dv[h] - r);
+      hi = fmaxf(hi, dv[h] + r);
+    }
+  }
+  lo = -warp_max_f(-lo);  // Gershgorin
+  hi = warp_max_f(hi);
+  float width = hi - lo;
+  if (!(width > 1e-15f && width < 1e15f && fabsf(lo) < 1e15f)) return false;
+  *spread = width;
+  const float sc = __int_as_float(0x7f000000 - (__float_as_int(width) & 0x7f800000));
+  *scale = sc;
+  lo *= sc;
+  hi *= sc;
+  width *= sc;  // in [1, 2)
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int i = lane + 32 * h;
+    const float l = bl[h] * sc;
+    d[i] = (i < n) ? dv[h] * sc : 8.0f;
+    ee[i] = l * l;
+    bf[i] = br[h] * sc;
   }
   __syncwarp();
-  R = warp_max_f(R);
-  if (!(R > 1e-15f && R < 1e15f)) return false;
-  // Gershgorin by rows
-  float lo = 3.0e38f, hi = -3.0e38f;
-  for (int i = lane; i < n; i += 32) {
-    const float r = ((i > 0) ? fabsf(bf[i - 1]) : 0.0f) + fabsf(bf[i]);
-    lo = fminf(lo, d[i] - r);
-    hi = fmaxf(hi, d[i] + r);
-  }
-  lo = -warp_max_f(-lo);
-  hi = warp_max_f(hi);
-  const float width = hi - lo;
   lo -= 1e-6f * width;
   hi += 1e-6f * width;
   if (warm) {
-    const float tp = float(th_prev - c0), rp = float(r_prev);
+    const float tp = float(th_prev - c0) * sc, rp = float(r_prev) * sc;
     const float whi = fminf(hi, tp + 2e-6f * width);
     const float wlo = fmaxf(lo, tp - fmaxf(2.0f * rp, 4e-6f * width));
     // the first round's probes include both ends
     const float step = (whi - wlo) * (1.0f / 31.0f);
     const float x = (lane == 31) ? whi : wlo + step * float(lane);
-    const unsigned bal = __ballot_sync(0xffffffffu, sturm_below_f(d, bb, n, x) >= 1);
+    const unsigned bal = __ballot_sync(0xffffffffu, below_scaled(d, ee, n, x));
     if (!(bal & 1u) && (bal >> 31)) {
       const int L = __ffs(bal) - 1;
       lo = wlo + step * float(L - 1);
@@ -519,18 +563,14 @@ __device__ inline bool warp_lowest_f32_pivots(const double* a, const double* b, 
     if (hi - lo <= 4e-7f * width) break;
     const float step = (hi - lo) * (1.0f / 33.0f);
     const float x = lo + step * float(lane + 1);
-    const unsigned bal = __ballot_sync(0xffffffffu, sturm_below_f(d, bb, n, x) >= 1);
+    const unsigned bal = __ballot_sync(0xffffffffu, below_scaled(d, ee, n, x));
     const int L = bal ? __ffs(bal) - 1 : 32;
     const float nlo = lo + step * float(L), nhi = (L < 32) ? lo + step * float(L + 1) : hi;
     if (!(nhi < hi) && !(nlo > lo)) break;
     if (L > 0) lo = nlo;
     hi = nhi;
   }
-  // one eigenvalue only near the bracket
-  const int near = sturm_below_f(d, bb, n, hi + 4e-6f * width);
-  if (near > 1) return false;
   const float s = lo - 4e-7f * width;
-  __syncwarp();
   // pivots and ratios from the bottom, by lane 0, operands read eight ahead
   int ok = 1;
   if (lane == 0) {
@@ -542,15 +582,18 @@ __device__ inline bool warp_lowest_f32_pivots(const double* a, const double* b, 
       for (int q = 0; q < 8; ++q) {
         const int i = i1 - q;
         dc[q] = (i >= 0) ? d[i] - s : 0.0f;
-        bc[q] = (i >= 0) ? bb[i] : 0.0f;
+        bc[q] = (i >= 0 && i < n - 1) ? ee[i + 1] : 0.0f;
       }
 #pragma unroll
       for (int q = 0; q < 8; ++q) {
         const int i = i1 - q;
         if (i >= 0) {
           float un = fmaf(-bc[q], rn, dc[q]);
-          if (i > 0 && !(un > small)) ok = 0;
-          if (i == 0) un = fmaxf(un, 0.1f * small);
+          // below the spectrum every pivot is positive; one of rounding size
+          // (a start vector with little of the lowest state) moves the matrix
+          // by no more than rounding when it is raised
+          if (!(un > -small)) ok = 0;
+          un = fmaxf(un, 0.1f * small);
           rn = __fdividef(1.0f, un);
           ru[i] = rn;
         }
@@ -586,33 +629,69 @@ __device__ inline bool warp_lowest_f32_pivots(const double* a, const double* b, 
   __syncwarp();
   for (int i = lane; i < n; i += 32) zf[i] *= inv;
   __syncwarp();
-  *th = 0.5f * (lo + hi);
-  *spread = width;
+  // No second eigenvalue near the bracket.  It is above the lowest one of the
+  // matrix without any one row (interlacing), here the row of the largest
+  // component; if that is near too, by count.
+  // (a start vector with less than 1e-5 of the state: the ratios are off)
+  if (!(zf[0] > 1e-5f)) return false;
+  const float top = 0.99f * m * inv;
+  const unsigned b0 = __ballot_sync(0xffffffffu, lane < n && fabsf(zf[lane]) >= top);
+  const unsigned b1 = __ballot_sync(0xffffffffu, lane + 32 < n && fabsf(zf[lane + 32]) >= top);
+  const int row = b0 ? __ffs(b0) - 1 : (b1 ? __ffs(b1) + 31 : 0);
+  const float x = hi + 4e-6f * width;
+  const float od = d[row], oe = ee[row], on = (row + 1 < n) ? ee[row + 1] : 0.0f;
+  __syncwarp();
+  if (lane == 0) {
+    d[row] = 8.0f;
+    ee[row] = 0.0f;
+    if (row + 1 < n) ee[row + 1] = 0.0f;
+  }
+  __syncwarp();
+  if (below_scaled(d, ee, n, x)) {
+    __syncwarp();
+    if (lane == 0) {
+      d[row] = od;
+      ee[row] = oe;
+      if (row + 1 < n) ee[row + 1] = on;
+    }
+    __syncwarp();
+    if (sturm_below_f(d, ee + 1, n, x) > 1) return false;
+  }
+  *th = 0.5f * (lo + hi) / sc;
   return true;
 }
 
+// One inverse iteration on the vector of warp_lowest_f32_pivots with its
+// pivots (the ratios alone are the solution for the right-hand side e_0: they
+// carry the shift's distance from theta over the start vector's share of the
+// lowest state); unit length again.
+__device__ __forceinline__ void improve_f32(float* work, int n) {
+  const int lane = threadIdx.x & 31;
+  float* zf = work + 4 * kTriMax;
+  if (lane == 0) pivot_solve(work + 2 * kTriMax, work + 3 * kTriMax, n, zf);
+  __syncwarp();
+  const float f0 = (lane < n) ? zf[lane] : 0.0f, f1 = (lane + 32 < n) ? zf[lane + 32] : 0.0f;
+  const float im = __fdividef(1.0f, warp_max_f(fmaxf(fabsf(f0), fabsf(f1))));
+  const float g0 = f0 * im, g1 = f1 * im;
+  const float inv = rsqrtf(warp_sum_f(fmaf(g0, g0, g1 * g1)));
+  if (lane < n) zf[lane] = g0 * inv;
+  if (lane + 32 < n) zf[lane + 32] = g1 * inv;
+  __syncwarp();
+}
+
 // The mixed path's check: theta to FP32 accuracy of the spread, z (normalised,
-// first component positive, after one inverse iteration with the pivots: the
-// ratios alone carry the shift's distance from theta) and *resid =
-// |bn z_{n-1}|; clusters and ranges FP32 cannot hold through
-// warp_lowest_eig_f32.
+// first component positive) and *resid = |bn z_{n-1}|; what the FP32 pivots
+// cannot do through warp_lowest_eig_f32.
 __device__ inline double warp_check_lowest_f32(const double* a, const double* b, int n, double bn,
                                                bool warm, double th_prev, double r_prev,
                                                double* z, double* work, double* resid) {
   const int lane = threadIdx.x & 31;
   float* w = reinterpret_cast<float*>(work);
-  float th = 0.0f, tail = 0.0f, width = 0.0f;
-  if (n > 1 && warp_lowest_f32_pivots(a, b, n, w, warm, th_prev, r_prev, &th, &tail, &width)) {
-    float* zf = w + 4 * kTriMax;
-    if (lane == 0) pivot_solve(w + kTriMax, w + 3 * kTriMax, n, zf);
-    __syncwarp();
-    float m = 0.0f;
-    for (int i = lane; i < n; i += 32) m = fmaxf(m, fabsf(zf[i]));
-    const float im = __fdividef(1.0f, warp_max_f(m));
-    float q = 0.0f;
-    for (int i = lane; i < n; i += 32) q = fmaf(zf[i] * im, zf[i] * im, q);
-    const float inv = im * rsqrtf(warp_sum_f(q));
-    for (int i = lane; i < n; i += 32) z[i] = double(zf[i] * inv);
+  float th = 0.0f, tail = 0.0f, width = 0.0f, sc = 1.0f;
+  if (n > 1 &&
+      warp_lowest_f32_pivots(a, b, n, w, warm, th_prev, r_prev, &th, &tail, &width, &sc)) {
+    improve_f32(w, n);
+    for (int i = lane; i < n; i += 32) z[i] = double(w[4 * kTriMax + i]);
     *resid = fabs(bn) * double(tail);
     __syncwarp();
     return a[0] + double(th);
@@ -633,8 +712,9 @@ __device__ inline bool warp_check_lowest(const double* a, const double* b, int n
                                          double* resid) {
   const int lane = threadIdx.x & 31;
   float* w = reinterpret_cast<float*>(work);
-  float th = 0.0f, tail = 0.0f, width = 0.0f;
-  if (n > 1 && warp_lowest_f32_pivots(a, b, n, w, warm, th_prev, r_prev, &th, &tail, &width)) {
+  float th = 0.0f, tail = 0.0f, width = 0.0f, sc = 1.0f;
+  if (n > 1 &&
+      warp_lowest_f32_pivots(a, b, n, w, warm, th_prev, r_prev, &th, &tail, &width, &sc)) {
     const double r = fabs(bn) * double(tail);
     *resid = r;
     const bool conv = r <= tol;
@@ -643,7 +723,8 @@ __device__ inline bool warp_check_lowest(const double* a, const double* b, int n
       *theta = s0;
       return false;
     }
-    const float* bf = w + kTriMax;
+    improve_f32(w, n);
+    const float* bf = w + 2 * kTriMax;
     const float* ru = w + 3 * kTriMax;
     float* x = w + 4 * kTriMax;  // the FP32 vector, then residuals and corrections
     const int i0 = lane, i1 = lane + 32;
@@ -695,8 +776,9 @@ __device__ inline bool warp_check_lowest(const double* a, const double* b, int n
       const float zf0 = float(z0), zf1 = float(z1);
       const float along = warp_sum_f(fmaf(zf0, g0, zf1 * g1));
       const float h0 = fmaf(-along, zf0, g0), h1 = fmaf(-along, zf1, g1);
-      z0 = fma(-double(big), double(h0), z0);
-      z1 = fma(-double(big), double(h1), z1);
+      const float ds = big * sc;  // the FP32 matrix is sc (T - a_0)
+      z0 -= double(ds * h0);
+      z1 -= double(ds * h1);
       // unit length again (to first order in |z|^2 - 1)
       const double sc = fma(-0.5, zz, 1.5);
       z0 *= sc;
@@ -705,7 +787,8 @@ __device__ inline bool warp_check_lowest(const double* a, const double* b, int n
     if (good) {
       *theta = s0 + dth;
       __syncwarp();
-      return conv;
+      *resid = fabs(bn * z[n - 1]);
+      return *resid <= tol;
     }
   }
   *theta = warp_lowest_eig(a, b, n, z, work, false, false, 0.0, 0.0);

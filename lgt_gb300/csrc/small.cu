@@ -157,18 +157,10 @@ __device__ __forceinline__ void df_sq2(df& x, float h, float l) {
   df_acc(x, p, e);
 }
 
-// The warp totals of four double-floats per lane, value q in lanes 8 q ..
-// 8 q + 7 (as warp_scatter4_int).
-__device__ __forceinline__ df warp_scatter4_df(const df* p, int lane) {
-  const bool b4 = lane & 16, b3 = lane & 8;
-  const df r0 = shfl_xor_df(b4 ? p[0] : p[2], 16);
-  const df r1 = shfl_xor_df(b4 ? p[1] : p[3], 16);
-  const df k0 = df_add(b4 ? p[2] : p[0], r0), k1 = df_add(b4 ? p[3] : p[1], r1);
-  const df r2 = shfl_xor_df(b3 ? k0 : k1, 8);
-  df kk = df_add(b3 ? k1 : k0, r2);
-  kk = df_add(kk, shfl_xor_df(kk, 4));
-  kk = df_add(kk, shfl_xor_df(kk, 2));
-  return df_add(kk, shfl_xor_df(kk, 1));
+// warp_scatter8 of double-floats.
+__device__ __forceinline__ df warp_scatter8_df(const df* p, int lane) {
+  return warp_scatter8<df>(p, lane, [](df x, df y) { return df_add(x, y); },
+                           [](df x, int o) { return shfl_xor_df(x, o); });
 }
 
 __device__ __forceinline__ df warp_total(df v) {
@@ -249,11 +241,11 @@ __device__ __forceinline__ void unit_reduce(A v, A (*slots)[CL * kWarpsCta], int
 // to both CTAs without a block barrier of their own, eight dots are reduced
 // together, and for R <= 4 the rows' neighbour lists sit in shared memory and
 // their diagonals in registers for the whole solve.  Cycles a step (4x2,
-// K = 64, clusters of two, R = 1), before -> after: mixed 21.9k -> 17.0k
-// (matvec 2.7 -> 1.2, dots 4.7 -> 4.1, their totals 2.8 -> 1.3, update 2.1 ->
-// 2.6, norm 4.0 -> 3.0, checks 4.0 -> 3.6); FP64 65.3k -> 33.3k (matvec 5.1 ->
-// 3.9, dots 15.8 -> 13.0, totals 4.1 -> 2.1, update 5.5 -> 6.3, norm 3.5 ->
-// 2.6, checks 29.3 -> 4.4).
+// K = 64, clusters of two, R = 1), before -> after: mixed 21.9k -> 15.1k
+// (matvec 2.7 -> 1.2, dots 4.7 -> 3.7, their totals 2.8 -> 1.3, update 2.1 ->
+// 2.6, norm 4.0 -> 3.0, checks 4.0 -> 2.4); FP64 65.3k -> 32k (matvec 5.1 ->
+// 4.0, dots 15.8 -> 12.8, totals 4.1 -> 2.2, update 5.5 -> 6.3, norm 3.5 ->
+// 2.6, checks 29.3 -> 3.2).
 template <typename S, int R, int CL>
 __global__ void __launch_bounds__(kCta, 1) k_lanczos_cta(const SmallProblem* probs,
                                                       const SmallUnit* units, SmallParams prm) {
@@ -275,7 +267,7 @@ __global__ void __launch_bounds__(kCta, 1) k_lanczos_cta(const SmallProblem* pro
   __shared__ double s_nb;      // |w|^2 before the latest pass
   __shared__ double s_thr;     // the step's space is exhausted when beta is not above it
   __shared__ int s_exh, s_more;  // ... and whether; a further pass is needed
-  __shared__ double s_work[3 * kMaxM];
+  __shared__ __align__(16) double s_work[3 * kMaxM];
   __shared__ double s_theta, s_resid;
   __shared__ int s_flag, s_zwarm;
   __shared__ int s_next, s_pstep;  // the next check's step; the previous check's step
@@ -498,19 +490,15 @@ __global__ void __launch_bounds__(kCta, 1) k_lanczos_cta(const SmallProblem* pro
               }
             }
           }
-#pragma unroll
-          for (int g = 0; g < 8; g += 4)
-            if (b0 + g <= jd) {
-              A kk;
-              if constexpr (kDF) kk = warp_scatter4_df(pd + g, lane);
-              else kk = warp_scatter4_int(pd + g, lane);
-              const int slot = b0 + g + (lane >> 3);
-              if ((lane & 7) == 0 && slot <= jd) {
-                const int at = int(cr) * nwarps + wid;
-                s_part[slot][at] = kk;
-                if (CL == 2) ppeer[slot * (CL * kWarpsCta) + at] = kk;
-              }
-            }
+          A kk;
+          if constexpr (kDF) kk = warp_scatter8_df(pd, lane);
+          else kk = warp_scatter8_int(pd, lane);
+          const int slot = b0 + (lane >> 2);
+          if ((lane & 3) == 0 && slot <= jd) {
+            const int at = int(cr) * nwarps + wid;
+            s_part[slot][at] = kk;
+            if (CL == 2) ppeer[slot * (CL * kWarpsCta) + at] = kk;
+          }
         }
         unit_sync();
         // eight lanes add a slot's totals of all warps of the unit
