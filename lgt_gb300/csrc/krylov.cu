@@ -1478,6 +1478,9 @@ template <typename S>
 cudaError_t apply_h(const OpDev& op, const S* x, const int* xsel, size_t xstride, S* y, int ncomp,
                     cudaStream_t s, int nslots = 1);
 
+// Panels above this are visited in the table's order of tiles.
+constexpr size_t kTileOrderBytes = size_t(48) << 20;
+
 template <typename S>
 void set_table(const OpDev& op, HpsiArgs<S>* a) {
   const bool ord = op.krylov_order && op.table_ord && op.table_ord->state == 1;
@@ -1488,6 +1491,8 @@ void set_table(const OpDev& op, HpsiArgs<S>* a) {
   a->t_off = T->tile_off;
   a->t_nbr = T->nbr;
   a->t_mm = T->mm;
+  // a panel that L2 holds gains nothing from the order of its tiles
+  if (!ord && size_t(a->N) * a->C * sizeof(S) > kTileOrderBytes) a->t_tile = T->tile_ord;
   a->use_table = 1;
 }
 
@@ -1798,19 +1803,30 @@ bool ensure_table(OpDev* op, cudaStream_t s) {
     T->state = -1;
     return false;
   }
-  // the renumbered copy for the Krylov drivers, when a second table fits the
-  // same budget: mask segments in breadth-first order (default),
-  // LGT_TABLE_ORDER=row the row-level order, LGT_TABLE_ORDER=0 none
+  // the order of the mask segments for products in the reference order, and
+  // the renumbered copy for the Krylov drivers when a second table fits the
+  // same budget (LGT_TABLE_ORDER=row: in the row-level order,
+  // LGT_TABLE_ORDER=0: neither)
   NbrTable* T2 = op->table_ord;
+  const char* eo = getenv("LGT_TABLE_ORDER");
+  const bool none = eo && eo[0] == '0';
+  const bool rows = eo && eo[0] == 'r';
+  SegmentOrder so;
+  std::string es;
+  if (!none && !rows) {
+    es = segment_order(op->G, op->R, &so, s);
+    if (es.empty() && !build_tile_order(so, T, s).empty()) {
+      cudaFree(T->tile_ord);
+      T->tile_ord = nullptr;
+    }
+  }
   if (T2 && T2->state == 0) {
-    const char* eo = getenv("LGT_TABLE_ORDER");
-    const bool none = eo && eo[0] == '0';
-    const bool rows = eo && eo[0] == 'r';
     if (none || 2 * bound > cap) {
       T2->state = -1;
     } else {
-      const std::string e2 = rows ? build_table_order(*T, T2, s)
-                                  : build_table_mask_order(*T, op->G, op->R, T2, s);
+      const std::string e2 = rows          ? build_table_order(*T, T2, s)
+                             : es.empty() ? build_table_mask_order(*T, so, T2, s)
+                                          : es;
       if (!e2.empty()) {
         free_nbr_table(T2);
         T2->state = -1;

@@ -1,6 +1,8 @@
 // lgt_hpsi.h -- launch interface of the H*psi and CSR-export kernels.
 #pragma once
 
+#include <vector>
+
 #include <string>
 
 #include "lgt_internal.h"
@@ -36,6 +38,7 @@ struct HpsiArgs {
   const uint32_t* t_off = nullptr;
   const uint32_t* t_nbr = nullptr;
   int t_mm = 0;           // most entries a row can have
+  const int* t_tile = nullptr;  // the order of the 32-row tiles (null: ascending)
   int use_table = 0;
   // the panels are in the table's own row order (a renumbered table): only
   // the table kernel may run; anything else is an error, not a fallback
@@ -66,6 +69,14 @@ struct NbrTable {
   // row, iperm[old] = new row.
   int* perm = nullptr;
   int* iperm = nullptr;
+  // The order in which a product visits the 32-row tiles (null: ascending).
+  int* tile_ord = nullptr;
+};
+
+// The mask segments of a basis in an order that keeps a product's gathers
+// local: segment i of it is rows [first[i], last[i]) (order.cu).
+struct SegmentOrder {
+  std::vector<uint32_t> first, last;
 };
 
 // Whether the basis fits the table format (N < 2^31, fewer than 2^32
@@ -80,10 +91,12 @@ void free_nbr_table(NbrTable* T);
 // T2 receives the renumbered table with its perm / iperm.  One-time cost per
 // Hamiltonian (a host read per search level).
 std::string build_table_order(const NbrTable& T, NbrTable* T2, cudaStream_t s);
-// The same with the fermion-mask segments ordered breadth-first over the
-// mask graph and the rows of a segment kept in order (order.cu).
-std::string build_table_mask_order(const NbrTable& T, const Geom& G, const RankView& R,
-                                   NbrTable* T2, cudaStream_t s);
+std::string segment_order(const Geom& G, const RankView& R, SegmentOrder* o, cudaStream_t s);
+// T renumbered to the segments in that order, the rows of one kept in order.
+std::string build_table_mask_order(const NbrTable& T, const SegmentOrder& o, NbrTable* T2,
+                                   cudaStream_t s);
+// T->tile_ord in that order of segments.
+std::string build_tile_order(const SegmentOrder& o, NbrTable* T, cudaStream_t s);
 
 // Whether the table kernel serves these arguments (table present, vector-
 // aligned panels) and its widest load mode (as hpsi_fixed_applies).

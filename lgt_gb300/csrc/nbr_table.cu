@@ -181,8 +181,10 @@ __global__ void __launch_bounds__(kTabThreads, PLAQ || sizeof(T) == 8 ? LGT_TABL
   }
   __syncthreads();
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int64_t warp_row0 = (int64_t(blockIdx.x) * kTabWarps + wid) * 32;
-  if (warp_row0 >= a.N) return;
+  int64_t tile = int64_t(blockIdx.x) * kTabWarps + wid;
+  if (tile * 32 >= a.N) return;
+  if (a.t_tile) tile = __ldg(a.t_tile + tile);
+  const int64_t warp_row0 = tile * 32;
   const int64_t row = warp_row0 + lane;
   const uint32_t m = (row < a.N) ? __ldcs(a.t_meta + row) : 0u;
   const int cnt = int(m & 255u);
@@ -292,6 +294,7 @@ void free_nbr_table(NbrTable* T) {
   cudaFree(T->nbr);
   cudaFree(T->perm);
   cudaFree(T->iperm);
+  cudaFree(T->tile_ord);
   *T = NbrTable();
 }
 

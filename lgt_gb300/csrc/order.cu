@@ -22,14 +22,13 @@
 // The row-level order above scatters the gathers of neighbouring lanes
 // (the rows a warp handles no longer have structured neighbours), and the
 // table kernel is bound by L1/TEX transactions more than by DRAM misses; so
-// the default is the same search one level up: the fermion-mask segments
-// (whose rows keep their reference order inside) are ordered breadth-first
-// over the mask graph, two masks being adjacent when one hop moves a
-// fermion across a bond between them (LRU model: 2.1 misses per row at
-// 100 MB against 4.3).  LGT_TABLE_ORDER=row selects the row-level order,
-// LGT_TABLE_ORDER=0 none.
+// the default orders the fermion-mask segments (whose rows keep their
+// reference order inside): segment_order.  LGT_TABLE_ORDER=row selects the
+// row-level order, LGT_TABLE_ORDER=0 none.  A product whose panels are in the
+// reference order visits its tiles of rows in the same order
+// (build_tile_order).
 //
-// Everything runs on the device, level-synchronous: per level one pass
+// The row-level search runs on the device, level-synchronous: per level one pass
 // claims the undiscovered neighbours of the level's rows (the smallest
 // (discoverer position, entry slot) key wins), one counts each row's claimed
 // children, a scan turns the counts into offsets and one pass places the
@@ -402,73 +401,116 @@ std::string build_table_order(const NbrTable& T, NbrTable* T2, cudaStream_t s) {
   finish(T, T2);
   return std::string();
 }
-std::string build_table_mask_order(const NbrTable& T, const Geom& G, const RankView& R,
-                                   NbrTable* T2, cudaStream_t s) {
-  const int64_t N = T.N;
-  if (T.state != 1 || N <= 0) return "no neighbour table to reorder";
-  if (G.ns > 26) return "too many sites for the host mask search";
-  free_nbr_table(T2);
+// The order of the sector's mask segments: by the masks' dipole P = sum of
+// x + y over the fermions, within a level by sum of y and then the mask, every
+// other level backwards.  A hop changes P by one, so a segment's neighbours
+// lie in the two levels around its own, and the turn keeps the last ones of a
+// level near the first of the next.  Exact LRU model of the 4x4 sector at
+// K = 8 complex FP32 (x 548 MB; a 75 MB cache fits the measured reads of the
+// other two orders): 1.35 GB of x against 2.05 breadth-first and 2.85 in the
+// basis order.
+std::string segment_order(const Geom& G, const RankView& R, SegmentOrder* o, cudaStream_t s) {
+  if (G.ns > 26) return "too many sites for the host mask order";
   // the sector's masks, ascending (the segment order of the basis)
-  std::vector<uint32_t> masks;
-  for (uint32_t m = 0; m < (1u << G.ns); ++m)
-    if (__builtin_popcount(m) == G.nf_target) masks.push_back(m);
-  if (int64_t(masks.size()) != int64_t(R.nmasks)) return "mask count differs from the basis";
-  std::vector<uint32_t> segc(masks.size() + 1);
+  std::vector<std::pair<uint64_t, uint32_t>> key;  // sort key, segment
+  for (uint32_t m = 0; m < (1u << G.ns); ++m) {
+    if (__builtin_popcount(m) != G.nf_target) continue;
+    uint64_t p = 0, y = 0;
+    for (uint32_t t = m; t; t &= t - 1) {
+      const int site = __builtin_ctz(t);
+      p += uint64_t(site % G.nx + site / G.nx);
+      y += uint64_t(site / G.nx);
+    }
+    constexpr uint64_t kLow = (1ull << 48) - 1;
+    const uint64_t in = (y << 32) | uint64_t(~m);
+    key.push_back({(p << 48) | ((p & 1) ? kLow - in : in), uint32_t(key.size())});
+  }
+  if (int64_t(key.size()) != int64_t(R.nmasks)) return "mask count differs from the basis";
+  std::vector<uint32_t> segc(key.size() + 1);
   OCK(cudaMemcpyAsync(segc.data(), R.segc, sizeof(uint32_t) * segc.size(),
                       cudaMemcpyDeviceToHost, s));
   OCK(cudaStreamSynchronize(s));
-  // bonds (site pairs) of the lattice: a hop across one moves a fermion
-  std::vector<std::pair<int, int>> bonds;
-  for (int iy = 0; iy < G.ny; ++iy)
-    for (int ix = 0; ix + 1 < G.nx; ++ix) bonds.push_back({iy * G.nx + ix, iy * G.nx + ix + 1});
-  for (int iy = 0; iy + 1 < G.ny; ++iy)
-    for (int ix = 0; ix < G.nx; ++ix) bonds.push_back({iy * G.nx + ix, (iy + 1) * G.nx + ix});
-  const size_t M = masks.size();
-  std::vector<int> order;
-  order.reserve(M);
-  std::vector<char> seen(M, 0);
-  for (size_t start = 0; start < M; ++start) {  // every component, first mask first
-    if (seen[start]) continue;
-    seen[start] = 1;
-    size_t head = order.size();
-    order.push_back(int(start));
-    while (head < order.size()) {
-      const uint32_t m = masks[order[head++]];
-      for (const auto& b : bonds) {
-        const uint32_t ba = 1u << b.first, bb = 1u << b.second;
-        if (((m & ba) != 0) == ((m & bb) != 0)) continue;
-        const uint32_t n = m ^ ba ^ bb;
-        const size_t q = size_t(std::lower_bound(masks.begin(), masks.end(), n) - masks.begin());
-        if (q < M && masks[q] == n && !seen[q]) {
-          seen[q] = 1;
-          order.push_back(int(q));
-        }
-      }
-    }
+  if (int64_t(segc.back()) != R.dim) return "mask segments do not cover the basis";
+  std::sort(key.begin(), key.end());
+  o->first.resize(key.size());
+  o->last.resize(key.size());
+  for (size_t i = 0; i < key.size(); ++i) {
+    o->first[i] = segc[key[i].second];
+    o->last[i] = segc[key[i].second + 1];
   }
-  std::vector<int> hperm;
-  hperm.reserve(size_t(N));
-  for (int q : order)
-    for (uint32_t r = segc[q]; r < segc[q + 1]; ++r) hperm.push_back(int(r));
-  if (int64_t(hperm.size()) != N) return "mask segments do not cover the basis";
+  return std::string();
+}
+
+// Ranges [first[i], last[i]) placed one after another: at[first + j] in perm
+// is from[i] + j, and iperm (when given) its inverse.  One block a range.
+__global__ void k_place_ranges(const uint32_t* first, const uint32_t* last, const uint32_t* at,
+                               int* perm, int* iperm) {
+  const uint32_t f = first[blockIdx.x], n = last[blockIdx.x] - f, to = at[blockIdx.x];
+  for (uint32_t j = threadIdx.x; j < n; j += blockDim.x) {
+    perm[to + j] = int(f + j);
+    if (iperm) iperm[f + j] = int(to + j);
+  }
+}
+
+std::string place_ranges(const std::vector<uint32_t>& first, const std::vector<uint32_t>& last,
+                         int64_t total, int* perm, int* iperm, cudaStream_t s) {
+  const size_t M = first.size();
+  std::vector<uint32_t> h(first);
+  h.insert(h.end(), last.begin(), last.end());
+  uint64_t at = 0;
+  for (size_t i = 0; i < M; ++i) {
+    h.push_back(uint32_t(at));
+    at += last[i] - first[i];
+  }
+  if (int64_t(at) != total) return "the ranges of the row order do not cover the basis";
+  uint32_t* d = nullptr;
+  OCK(dev_alloc_n(&d, h.size(), s));
+  OCK(cudaMemcpyAsync(d, h.data(), sizeof(uint32_t) * h.size(), cudaMemcpyHostToDevice, s));
+  k_place_ranges<<<unsigned(M), 128, 0, s>>>(d, d + M, d + 2 * M, perm, iperm),
+      lgt::note_launch();
+  OCK(cudaGetLastError());
+  OCK(cudaStreamSynchronize(s));  // h is copied
+  OCK(dev_free(d, s));
+  return std::string();
+}
+
+std::string build_table_mask_order(const NbrTable& T, const SegmentOrder& o, NbrTable* T2,
+                                   cudaStream_t s) {
+  const int64_t N = T.N;
+  if (T.state != 1 || N <= 0) return "no neighbour table to reorder";
+  free_nbr_table(T2);
   int *perm = nullptr, *iperm = nullptr;
   uint32_t* row_off = nullptr;
   OCK(cudaMalloc(&perm, sizeof(int) * N));
   T2->perm = perm;
   OCK(cudaMalloc(&iperm, sizeof(int) * N));
   T2->iperm = iperm;
-  OCK(cudaMemcpyAsync(perm, hperm.data(), sizeof(int) * N, cudaMemcpyHostToDevice, s));
+  std::string e = place_ranges(o.first, o.last, N, perm, iperm, s);
+  if (!e.empty()) return e;
   const unsigned nblk = unsigned((N + kOT - 1) / kOT);
-  k_invert<<<nblk, kOT, 0, s>>>(perm, N, iperm), lgt::note_launch();
   OCK(dev_alloc_n(&row_off, size_t(N), s));
   k_row_offsets<<<nblk, kOT, 0, s>>>(T.meta, T.tile_off, N, row_off), lgt::note_launch();
   OCK(cudaGetLastError());
-  std::string e = renumber(T, perm, iperm, row_off, T2, s);
+  e = renumber(T, perm, iperm, row_off, T2, s);
   if (!e.empty()) return e;
   OCK(dev_free(row_off, s));
   OCK(cudaStreamSynchronize(s));
   finish(T, T2);
   return std::string();
+}
+
+// The 32-row tiles of the reference order, each in the place of its first
+// row's segment.
+std::string build_tile_order(const SegmentOrder& o, NbrTable* T, cudaStream_t s) {
+  const int64_t tiles = (T->N + 31) / 32;
+  std::vector<uint32_t> first(o.first.size()), last(o.last.size());
+  for (size_t i = 0; i < first.size(); ++i) {
+    first[i] = uint32_t((uint64_t(o.first[i]) + 31) / 32);
+    last[i] = uint32_t((uint64_t(o.last[i]) + 31) / 32);
+  }
+  OCK(cudaMalloc(&T->tile_ord, sizeof(int) * tiles));
+  T->bytes += sizeof(int) * size_t(tiles);
+  return place_ranges(first, last, tiles, T->tile_ord, nullptr, s);
 }
 
 }  // namespace lgt
