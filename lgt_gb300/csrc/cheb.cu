@@ -10,10 +10,16 @@
 // earlier vectors per product, 55 % of a 4x4 K = 8 step): a product reads
 // T_n (gathered) and T_{n-1} once and writes T_{n+1}, and one pass at the end
 // sums the stored panels.  Measured against the Krylov step, observables
-// included: 4x4 K = 8 mixed, two steps of dt = 0.05, 114.6 -> 40.9 ms; 4x4
-// K = 3 FP64 with plaquettes, one step, 85.1 -> 62.2 ms (bound by the FP64
-// pipe of the products); 3x4 K = 1 FP64, ten steps, 13.5 -> 4.0 ms; the
+// included: 4x4 K = 8 mixed, two steps of dt = 0.05, 114.6 -> 35.1 ms; 4x4
+// K = 3 FP64 with plaquettes, one step, 85.1 -> 37.9 ms (bound by the FP64
+// pipe of the products); 3x4 K = 1 FP64, ten steps, 13.5 -> 2.9 ms; the
 // error against exact propagation is unchanged (5.7e-8, 4.4e-15, 7.6e-15).
+//
+// The products apply H's couplings as they are and multiply the finished sum
+// by 2 / d; c and 1 / d are taken as FP32 numbers.  (Couplings divided by d
+// and then rounded to FP32 shift every energy by up to 6e-8 of itself; the 4x4
+// K = 8 mixed quench, two steps, is now off by 2.5e-8 - 3.0e-8 of the FP64
+// state, the Krylov steps by 3.0e-8 - 3.7e-8.)
 //
 // The bounds are Gershgorin's, per point, from the table's row meta words
 // (diagonal and entry counts) in FP32, widened by 1e-5 of their size.  The
@@ -310,9 +316,10 @@ std::string run(const OpDev& op, ChebWork* w, const NbrTable& T, int n_steps,
   double* a_rho = a_phase + 2 * K;
   double* a_rho0 = a_rho + K;
   double* a_drift = a_rho0 + K;
-  S* a_c1 = reinterpret_cast<S*>(a_drift + K);  // [5][K]: the first product's couplings
-  S* a_c2 = a_c1 + 5 * size_t(K);               // the others' (twice those)
-  const size_t host_n = size_t(terms) * K + 5 * size_t(K) + 10 * size_t(K);
+  // [6][K]: couplings, shift and scale of the first product; of the others
+  S* a_c1 = reinterpret_cast<S*>(a_drift + K);
+  S* a_c2 = a_c1 + 6 * size_t(K);
+  const size_t host_n = size_t(terms) * K + 5 * size_t(K) + 12 * size_t(K);
   int* a_fail = reinterpret_cast<int*>(a_coef + host_n);
   double* a_part = a_coef + host_n + 1;
   std::vector<double> h(host_n + 1, 0.0);
@@ -320,7 +327,7 @@ std::string run(const OpDev& op, ChebWork* w, const NbrTable& T, int n_steps,
   CCK(cudaMemcpyAsync(cc.data(), op.cE_d, sizeof(double) * 4 * K, cudaMemcpyDeviceToHost, s));
   CCK(cudaStreamSynchronize(s));
   S* h1 = reinterpret_cast<S*>(h.data() + size_t(terms) * K + 5 * size_t(K));
-  S* h2 = h1 + 5 * size_t(K);
+  S* h2 = h1 + 6 * size_t(K);
   for (int k = 0; k < K; ++k) {
     for (size_t n = 0; n < J[k].size(); ++n) {
       const double j = (n == 0 ? 1.0 : 2.0) * J[k][n];
@@ -329,11 +336,10 @@ std::string run(const OpDev& op, ChebWork* w, const NbrTable& T, int n_steps,
     const double ph = -c[k] * dt * double(n_steps);
     h[size_t(terms) * K + 2 * k] = std::cos(ph);
     h[size_t(terms) * K + 2 * k + 1] = std::sin(ph);
-    for (int q = 0; q < 5; ++q) {
-      const double v = (q < 4 ? cc[size_t(q) * K + k] : -c[k]) / d[k];
-      h1[size_t(q) * K + k] = S(v);
-      h2[size_t(q) * K + k] = S(2.0 * v);
-    }
+    for (int q = 0; q < 5; ++q)
+      h1[size_t(q) * K + k] = h2[size_t(q) * K + k] = S(q < 4 ? cc[size_t(q) * K + k] : -c[k]);
+    h1[5 * size_t(K) + k] = S(1.0 / d[k]);  // exact in S, like the shift
+    h2[5 * size_t(K) + k] = S(2.0 / d[k]);
   }
   // (a copy from pageable memory has staged the host data when it returns)
   CCK(cudaMemcpyAsync(a_coef, h.data(), sizeof(double) * h.size(), cudaMemcpyHostToDevice, s));
@@ -445,7 +451,7 @@ std::string cheb_expm(const OpDev& op, const KrylovParams& p, ChebWork* w, doubl
   // the buffers beside the panels, sized for the longest expansion
   const int nmax = p.krylovdim;
   int64_t rpb = 1;
-  const size_t aux = sizeof(double) * (size_t(nmax + 1) * K + 16 * size_t(K) + 2 +
+  const size_t aux = sizeof(double) * (size_t(nmax + 1) * K + 18 * size_t(K) + 2 +
                                        size_t(blocks_for(N, K, &rpb)) * K) +
                      sizeof(float2) * size_t(kBoundBlocks + 1) * K + 256;
   if (w->aux_bytes < aux) {
@@ -469,10 +475,12 @@ std::string cheb_expm(const OpDev& op, const KrylovParams& p, ChebWork* w, doubl
   std::vector<std::vector<double>> J(K);
   for (int k = 0; k < K; ++k) {
     const double lo = b[k].x, hi = b[k].y;
-    if (!std::isfinite(lo) || !std::isfinite(hi) || std::fmax(std::fabs(lo), std::fabs(hi)) > 1e30)
+    if (!std::isfinite(lo) || !std::isfinite(hi) || std::fmax(std::fabs(lo), std::fabs(hi)) > 1e30 ||
+        !(std::fmax(std::fabs(lo), std::fabs(hi)) > 1e-25))
       return std::string();
-    c[k] = 0.5 * (lo + hi);
+    c[k] = double(float(0.5 * (lo + hi)));
     d[k] = 0.5 * (hi - lo) + 1e-5 * std::fmax(std::fabs(lo), std::fabs(hi)) + 1e-30;
+    d[k] = 1.0 / double(std::nextafterf(float(1.0 / d[k]), 0.0f));
     J[k] = cheb_bessel(d[k] * dt, eps, nmax);
     if (J[k].empty()) return std::string();
   }

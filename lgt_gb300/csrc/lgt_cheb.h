@@ -31,7 +31,7 @@ std::string cheb_expm(const OpDev& op, const KrylovParams& p, ChebWork* w, doubl
 std::vector<double> cheb_bessel(double z, double eps, int nmax);
 
 // The products of the expansion from the stored table (one translation unit
-// per precision): y = coef-scaled H x (- prev), coef = [5][K].
+// per precision): y = scale (H + shift) x (- prev), coef = [6][K].
 cudaError_t launch_cheb_product(const NbrTable& T, uint32_t model, int64_t N, int K, const float* x,
                                 float* y, const float* prev, const float* coef, cudaStream_t s);
 cudaError_t launch_cheb_product(const NbrTable& T, uint32_t model, int64_t N, int K,

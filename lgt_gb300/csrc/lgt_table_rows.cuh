@@ -8,8 +8,7 @@
 // width divides into slices (W = 1 where C is odd).
 //
 //   plain  y = (cE e2 + cm stag) x + ch sum_hops (+-) x_j + cp sum_plaq x_j
-//   Cheb   y = that with the scaled couplings of (H - c) / d and the shift
-//          cs added to the diagonal, minus `prev` where it is given:
+//   Cheb   y = scale ((H + shift) x), minus `prev` where it is given:
 //          T_{n+1} = 2 H~ T_n - T_{n-1}  (cheb.cu)
 // (finite_ed.jl:265-318; matter_gauge_entanglement_pjw.jl:82-147).
 #pragma once
@@ -35,7 +34,7 @@ struct Args {
   const T* x;
   T* y;
   const T* prev;          // Cheb: subtracted when not null
-  const T* coef;          // [4][K] cE, cm, ch, cp (Cheb: [5][K], then cs)
+  const T* coef;          // Cheb: [6][K] cE, cm, ch, cp, shift, scale
   const T* cE;            // plain: the four coupling arrays
   const T* cm;
   const T* ch;
@@ -121,7 +120,7 @@ __device__ __forceinline__ void sum_entries(const T* x, int C, int col0, const u
     sum_slices<T, W, U, SGN>(x, C, col0, lst, n0, n1, s);
 }
 
-__host__ __device__ inline int coef_words(bool cheb, int K) { return (cheb ? 5 : 4) * K; }
+__host__ __device__ inline int coef_words(bool cheb, int K) { return (cheb ? 6 : 4) * K; }
 
 template <typename T>
 __host__ __device__ inline int smem_bytes(bool cheb, int K, int mm) {
@@ -139,7 +138,8 @@ __device__ __forceinline__ int incl_scan(int v, int lane) {
 }
 
 template <typename T, int W, int U, bool PLAQ, bool JW, bool CHEB>
-__global__ void __launch_bounds__(kThreads, PLAQ || sizeof(T) == 8 ? 4 : 5) k_table_rows(Args<T> a) {
+__global__ void __launch_bounds__(kThreads, PLAQ || JW || sizeof(T) == 8 ? 4 : 5)
+    k_table_rows(Args<T> a) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int K = a.K, C = a.C;
   T* s_coef = reinterpret_cast<T*>(smem);
@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(kThreads, PLAQ || sizeof(T) == 8 ? 4 : 5) k_ta
   uint32_t* s_off = s_meta + kThreads;
   uint32_t* s_list = s_off + kThreads;
   if constexpr (CHEB) {
-    for (int i = threadIdx.x; i < 5 * K; i += kThreads) s_coef[i] = a.coef[i];
+    for (int i = threadIdx.x; i < 6 * K; i += kThreads) s_coef[i] = a.coef[i];
   } else {
     for (int i = threadIdx.x; i < K; i += kThreads) {
       s_coef[i] = a.cE[i];
@@ -191,8 +191,8 @@ __global__ void __launch_bounds__(kThreads, PLAQ || sizeof(T) == 8 ? 4 : 5) k_ta
 #pragma unroll
     for (int e = 0; e < W; ++e) {
       const int k = a.ncomp == 2 ? (col0 + e) >> 1 : col0 + e;
-      T cd = fma(s_coef[k], e2, s_coef[K + k] * stag);
-      if (CHEB) cd += s_coef[4 * K + k];
+      const T cd = CHEB ? fma(s_coef[k], e2, fma(s_coef[K + k], stag, s_coef[4 * K + k]))
+                        : fma(s_coef[k], e2, s_coef[K + k] * stag);
       out[e] = fma(s_coef[2 * K + k], ah[e], cd * xd[e]);
     }
     if (PLAQ) {
@@ -203,10 +203,15 @@ __global__ void __launch_bounds__(kThreads, PLAQ || sizeof(T) == 8 ? 4 : 5) k_ta
         out[e] = fma(s_coef[3 * K + k], ah[e], out[e]);
       }
     }
-    if (CHEB && a.prev) {
-      ld_cols<T, W>(a.prev + at, ah);
+    if (CHEB) {
 #pragma unroll
-      for (int e = 0; e < W; ++e) out[e] -= ah[e];
+      for (int e = 0; e < W; ++e) ah[e] = T(0);
+      if (a.prev) ld_cols<T, W>(a.prev + at, ah);
+#pragma unroll
+      for (int e = 0; e < W; ++e) {
+        const int k = a.ncomp == 2 ? (col0 + e) >> 1 : col0 + e;
+        out[e] = fma(s_coef[5 * K + k], out[e], -ah[e]);
+      }
     }
     st_cols<T, W>(a.y + at, out);
   }

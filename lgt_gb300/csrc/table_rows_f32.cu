@@ -5,7 +5,10 @@
 
 namespace lgt {
 
-// Slices of 32, 16 or 8 bytes: the widest that divides the panel row.
+// Slices of 16 bytes where they divide the panel row, else of 8.  (32-byte
+// ones take half the instructions, but the lanes wait on L2 and have more rows
+// in flight with the smaller ones: 4x4 K = 8 quench, FP32-mixed, 35.9 ms a run
+// with 32-byte slices, 35.1 with 16, 40.5 with 8.)
 cudaError_t launch_cheb_product(const NbrTable& T, uint32_t model, int64_t N, int K, const float* x,
                                 float* y, const float* prev, const float* coef, cudaStream_t s) {
   rows::Args<float> a = {};
@@ -21,7 +24,6 @@ cudaError_t launch_cheb_product(const NbrTable& T, uint32_t model, int64_t N, in
   a.y = y;
   a.prev = prev;
   a.coef = coef;
-  if (a.C % 8 == 0) return rows::launch_model<float, 8, 4, true>(a, model, s);
   if (a.C % 4 == 0) return rows::launch_model<float, 4, 8, true>(a, model, s);
   return rows::launch_model<float, 2, 8, true>(a, model, s);
 }
