@@ -775,7 +775,7 @@ lgt_status lgt_ground_state_observe(lgt_ham* h, const lgt_krylov_opts* opts, dou
   const int nf = observe_nfeat(G);
   int nblk;
   int64_t rpb;
-  observe_plan(N, &nblk, &rpb);
+  observe_plan(N, h->K, &nblk, &rpb);
   CUDA_OR_FAIL(h->part.need(sizeof(double) * size_t(nblk) * h->K * nf, s));
   CUDA_OR_FAIL(h->out.need(sizeof(double) * size_t(h->K) * nf, s));
   const size_t n = size_t(h->K) * nf;
@@ -924,7 +924,7 @@ lgt_status observe_dev(lgt_ham* h, const T* x, int ncomp, std::vector<double>* f
   const int nf = observe_nfeat(G);
   int nblk;
   int64_t rpb;
-  observe_plan(h->b->B.dim, &nblk, &rpb);
+  observe_plan(h->b->B.dim, h->K, &nblk, &rpb);
   CUDA_OR_FAIL(h->part.need(sizeof(double) * size_t(nblk) * h->K * nf, h->b->B.stream));
   CUDA_OR_FAIL(h->out.need(sizeof(double) * size_t(h->K) * nf, h->b->B.stream));
   cudaStream_t s = h->b->B.stream;

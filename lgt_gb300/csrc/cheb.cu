@@ -12,7 +12,7 @@
 // sums the stored panels.  Measured against the Krylov step, observables
 // included: 4x4 K = 8 mixed, two steps of dt = 0.05, 114.6 -> 35.1 ms; 4x4
 // K = 3 FP64 with plaquettes, one step, 85.1 -> 37.9 ms (bound by the FP64
-// pipe of the products); 3x4 K = 1 FP64, ten steps, 13.5 -> 2.9 ms; the
+// pipe of the products); 3x4 K = 1 FP64, ten steps, 13.5 -> 2.3 ms; the
 // error against exact propagation is unchanged (5.7e-8, 4.4e-15, 7.6e-15).
 //
 // The products apply H's couplings as they are and multiply the finished sum
@@ -282,7 +282,9 @@ __global__ void __launch_bounds__(kT) k_cheb_combine(const S* __restrict__ V, si
 
 int blocks_for(int64_t N, int K, int64_t* rpb) {
   const int RG = kT / K;
-  int64_t b = (N + 4 * RG - 1) / (4 * RG);  // four rows a thread at least
+  // two rows a thread at least (four: 2.69 ms for 3x4 K = 1 FP64, ten steps;
+  // two 2.59, one 2.60)
+  int64_t b = (N + 2 * RG - 1) / (2 * RG);
   if (b > kMaxBlocks) b = kMaxBlocks;
   if (b < 1) b = 1;
   *rpb = (N + b - 1) / b;

@@ -7,8 +7,8 @@ namespace lgt {
 
 // Number of features per point: n_f per site, E^2 per site, plaquettes, norm.
 int observe_nfeat(const Geom& G);
-// Block partition of the observables reduction for N rows.
-void observe_plan(int64_t N, int* nblk, int64_t* rpb);
+// Block partition of the observables reduction for N rows of K points.
+void observe_plan(int64_t N, int K, int* nblk, int64_t* rpb);
 
 // out[k * nfeat + f] for the K points of panel x ([N][K][ncomp]); part must
 // hold nblk * K * nfeat doubles (observe_plan).

@@ -100,7 +100,7 @@ lgt_status lgt_observe_noalloc(const lgt_ham* h, const void* psi, int32_t ncomp,
   if (e != cudaSuccess) return fail_na(LGT_ERR_CUDA, std::string("scratch set-up: ") + cudaGetErrorString(e));
   int nblk;
   int64_t rpb;
-  lgt::observe_plan(b->B.dim, &nblk, &rpb);
+  lgt::observe_plan(b->B.dim, K, &nblk, &rpb);
   const int fit = int((kScratchDoubles - fixed) / per_block);
   if (nblk > fit) {
     nblk = fit;

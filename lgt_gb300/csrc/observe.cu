@@ -982,11 +982,15 @@ cudaError_t launch_obs2(const Geom& G, const RankView& R, const T* x, int K, int
 
 int observe_nfeat(const Geom& G) { return 2 * G.ns + G.nP + 1; }
 
-void observe_plan(int64_t N, int* nblk, int64_t* rpb) {
-  // at least 4 rows per block (a K = 64 batch of N = 645 spreads over 162
-  // blocks: the per-row FP64 feature sums are the work), at most four
-  // blocks per SM
-  int64_t want = (N + 3) / 4;
+void observe_plan(int64_t N, int K, int* nblk, int64_t* rpb) {
+  // At least two rows for each of a block's kT / K groups of threads (the
+  // block's reduction of all features costs as much as some rows: 3x4 K = 1,
+  // eleven measurements in a run of 2.69 ms, 119 rows a block for 256 groups;
+  // two rows a group 2.39 ms, one 2.46, four 2.31, which leaves K = 64 batches
+  // of N = 645 with 40 blocks), at most four blocks per SM.
+  int64_t least = (K < 1 || K > kT) ? 4 : 2 * int64_t(kT / K);
+  if (least < 4) least = 4;
+  int64_t want = (N + least - 1) / least;
   if (want > 152 * 4) want = 152 * 4;
   if (want < 1) want = 1;
   int64_t r = (N + want - 1) / want;
@@ -1003,7 +1007,7 @@ cudaError_t launch_observe(const Geom& G, const RankView& R, const T* x, int K, 
   if (nfeat > 96) return cudaErrorInvalidValue;
   int nblk;
   int64_t rpb;
-  observe_plan(R.dim, &nblk, &rpb);
+  observe_plan(R.dim, K, &nblk, &rpb);
   cudaError_t e = (ncomp == 1)
                       ? launch_obs2<T, 1>(G, R, x, K, nfeat, nblk, rpb, part, err, s)
                       : launch_obs2<T, 2>(G, R, x, K, nfeat, nblk, rpb, part, err, s);
