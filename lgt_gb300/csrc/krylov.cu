@@ -1815,7 +1815,8 @@ bool ensure_table(OpDev* op, cudaStream_t s) {
   std::string es;
   if (!none && !rows) {
     es = segment_order(op->G, op->R, &so, s);
-    if (es.empty() && !build_tile_order(so, T, s).empty()) {
+    // (a basis whose widest usual panels L2 holds needs no order of its tiles)
+    if (es.empty() && T->N >= (int64_t(1) << 17) && !build_tile_order(so, T, s).empty()) {
       cudaFree(T->tile_ord);
       T->tile_ord = nullptr;
     }

@@ -23,8 +23,8 @@ struct OpDev {
   int vpl = 0;            // fixed-shape H*psi: vector loads per lane (0: by width)
   NbrTable* table = nullptr;  // the Hamiltonian's neighbour table (built on demand)
   int use_table = 0;          // H*psi from the stored table
-  // The table renumbered to its breadth-first row order (order.cu), built
-  // with the table; the Krylov drivers keep their basis vectors in that
+  // The table renumbered to its own row order (order.cu), built with the
+  // table; the Krylov drivers keep their basis vectors in that
   // order (krylov_order = 1) when the table kernel is chosen.
   NbrTable* table_ord = nullptr;
   int krylov_order = 0;

@@ -36,7 +36,10 @@ constexpr int kTabWarps = 8;
 constexpr int kTabThreads = kTabWarps * 32;
 // Resident blocks per SM the register budget must allow.  Measured on the
 // 4x4 lattice, K = 8 complex FP32: 5 blocks with 8 rows in flight beat 6
-// with 4 (0.714 vs 0.757 ms); 8 blocks (32 registers) spill.
+// with 4 (0.714 vs 0.757 ms); 8 blocks (32 registers) spill.  With the tiles
+// in the order of the mask segments one vector a lane is the best load mode
+// (0.694 ms; two vectors 0.726, one 32-byte access 0.745): nothing but the
+// gathers' traffic from L2, 7.3 GB, is near a limit.
 #ifndef LGT_TABLE_MINB
 #define LGT_TABLE_MINB 5
 #endif

@@ -221,11 +221,6 @@ __global__ void k_place_unplaced(const int* level, int64_t N, const uint32_t* of
   }
 }
 
-__global__ void k_invert(const int* perm, int64_t N, int* iperm) {
-  const int64_t n = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (n < N) iperm[perm[n]] = int(n);
-}
-
 __global__ void k_seed(int* perm, int* iperm, int* level, int64_t at, int row, int L) {
   perm[at] = row;
   iperm[row] = int(at);
