@@ -42,10 +42,10 @@ G_LO, G_HI, T_HOP, MASS = 0.5, 2.0, 1.0, 0.5
 RF_NX, RF_NY, RF_K = 4, 4, 8          # roofline panel (4x4 quench, K = 8 complex)
 # DRAM bytes of one such launch (FP32, reference model) per kernel family,
 # measured by ncu (dram__bytes_read.sum + dram__bytes_write.sum, one launch
-# of each kernel on this panel; the ordered table in the mask-BFS row order)
+# of each kernel on this panel; the ordered table in its own row order)
 RF_TRAFFIC_BYTES = {"fixed": int((2.903165 + 0.533069) * 1e9),
-                    "table": int((3.236144 + 0.532940) * 1e9),
-                    "table_ordered": int((2.525915 + 0.527390) * 1e9)}
+                    "table": int((2.063974 + 0.532940) * 1e9),
+                    "table_ordered": int((1.962439 + 0.527390) * 1e9)}
 L2_FLUSH_BYTES = 512 << 20            # > 129 MB L2
 METRIC = "ground states/s, batched FP32-mixed Lanczos at |dE|/|E|<=1e-10"
 
@@ -604,9 +604,9 @@ def roofline(L, C, lib, torch, stream, dev, reps=10, only=None):
     gs = np.random.default_rng(0).uniform(0.5, 1.5, RF_K)
     out = {"N": N, "basis_build_s": basis_s}
     # variants: the autotuner's choice, and each kernel family forced
-    # (LGT_HPSI_VARIANT: 3 fixed shape, 6 stored table, two vectors per lane;
-    # 8 stored table with the neighbour rows gathered by the copy engine)
-    forced = {"": None, "_generic": None, "_fixed": "3", "_table": "6", "_table_ordered": "6",
+    # (LGT_HPSI_VARIANT: 3 fixed shape, two vectors per lane; 5 stored table,
+    # one vector; 8 stored table with the rows gathered by the copy engine)
+    forced = {"": None, "_generic": None, "_fixed": "3", "_table": "5", "_table_ordered": "5",
               "_gather": "8", "_gather_ordered": "8"}
     models, precs = ("ref", "pjw"), (("fp64", torch.float64, 16), ("fp32", torch.float32, 8))
     if only is not None:
@@ -658,9 +658,9 @@ def roofline(L, C, lib, torch, stream, dev, reps=10, only=None):
                 elif var == "8":
                     kernel = "table_gather_ordered" if ordered else "table_gather"
                 elif ordered:
-                    kernel = "table_ordered_vpl2"
+                    kernel = "table_ordered_vpl1"
                 elif var is not None:
-                    kernel = "fixed_vpl2" if var == "3" else "table_vpl2"
+                    kernel = "fixed_vpl2" if var == "3" else "table_vpl1"
                 else:  # the autotuner's kernel for this shape (chosen at the first call)
                     tune = C.Tuning()
                     C.check(lib.lgt_autotune(H.handle, 2, code, ctypes_byref(tune)))

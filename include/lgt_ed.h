@@ -211,9 +211,9 @@ LGT_API lgt_status lgt_matvec(const lgt_ham* h, const void* x, void* y, int32_t 
                       uint32_t flags);
 
 /* The locality row order of the stored-table H*psi (no counterpart in the
-   reference): the rows in breadth-first order of the Hamiltonian's hop
-   graph, which the Krylov drivers use internally for their basis vectors
-   (the x gathers of a product then mostly hit L2).  Builds the neighbour
+   reference): the fermion-mask segments by the masks' dipole sum(x + y),
+   which the panel drivers use internally for their vectors (half of a
+   product's gathers then hit L2).  Builds the neighbour
    table and its renumbered copy on first use (LGT_ERR_UNSUPPORTED where the
    table is not available).  perm: N int32 (may be NULL), perm[n] = the
    0-based basis index of row n of that order.  lgt_matvec with
@@ -252,7 +252,7 @@ LGT_API lgt_status lgt_ground_state_batch(int32_t nham, lgt_ham* const* hams,
                                           void* const* psi, double* const* residual,
                                           uint32_t flags, lgt_info* info);
 
-/* evolve_ED! (finite_ed.jl:405-431): n_steps Krylov steps
+/* evolve_ED! (finite_ed.jl:405-431): n_steps exponential steps
    psi <- exp(-i H dt) psi, each followed by renormalisation, for all K
    points.  psi: complex double panel [N][K][2], updated in place.  obs:
    (n_steps + 1) * K records (t = step * dt), filled every step, or NULL.

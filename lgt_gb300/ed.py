@@ -364,9 +364,9 @@ class Hamiltonian:
         return y.reshape(xin.shape)
 
     def row_order(self) -> np.ndarray:
-        """The locality row order of the stored-table product (rows in
-        breadth-first order of the hop graph): perm[n] is the basis index of
-        row n of that order.  The Krylov drivers keep their vectors in it."""
+        """The locality row order of the stored-table product (mask
+        segments by the masks' dipole): perm[n] is the basis index of row n
+        of that order.  The panel drivers keep their vectors in it."""
         perm = np.zeros(self.basis.dim, np.int32)
         C.check(C.load().lgt_ham_row_order(self._h, _p(perm)))
         return perm
