@@ -291,24 +291,37 @@ int blocks_for(int64_t N, int K, int64_t* rpb) {
   return int((N + *rpb - 1) / *rpb);
 }
 
+// Dynamic shared memory of k_cheb_combine.
+size_t comb_smem(int terms, int K) { return sizeof(double) * size_t(terms) * K; }
+
+// Device memory and shared memory for an expansion of `terms` panels of `vs`
+// elements; false (with nothing held) where they cannot be had.
+template <typename S>
+bool reserve(ChebWork* w, int terms, int K, size_t vs, cudaStream_t s) {
+  const size_t need = sizeof(S) * vs * size_t(terms) + 256;
+  cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(k_cheb_combine<S>),
+                                   int(comb_smem(terms, K)));
+  if (e == cudaSuccess && w->v_bytes < need) {
+    dev_free(w->V, s);
+    w->V = nullptr;
+    w->v_bytes = 0;
+    e = dev_alloc(&w->V, need, s);
+    if (e == cudaSuccess) w->v_bytes = need;
+  }
+  if (e == cudaSuccess) return true;
+  cudaGetLastError();
+  w->release(s);
+  return false;
+}
+
 template <typename S>
 std::string run(const OpDev& op, ChebWork* w, const NbrTable& T, int n_steps,
                 const std::vector<std::vector<double>>& J, const std::vector<double>& c,
-                const std::vector<double>& d, double dt, double* Xd, double* drift,
+                const std::vector<double>& d, int terms, double dt, double* Xd, double* drift,
                 StepObserver* obs, cudaStream_t s, KrylovReport* rep, double tail) {
   const int64_t N = op.R.dim;
   const int K = op.K;
-  int terms = 1;
-  for (const auto& j : J) terms = int(j.size()) > terms ? int(j.size()) : terms;
   const size_t vs = size_t(N) * 2 * K;
-  const size_t need = sizeof(S) * vs * size_t(terms) + 256;
-  if (w->v_bytes < need) {
-    CCK(dev_free(w->V, s));
-    w->V = nullptr;
-    w->v_bytes = 0;
-    CCK(dev_alloc(&w->V, need, s));
-    w->v_bytes = need;
-  }
   S* V = static_cast<S*>(w->V);
   int64_t rpb = 1;
   const int nblk = blocks_for(N, K, &rpb);
@@ -348,9 +361,8 @@ std::string run(const OpDev& op, ChebWork* w, const NbrTable& T, int n_steps,
 
   double2* X = reinterpret_cast<double2*>(Xd);
   const int* perm = T.perm;
-  const size_t sh = sizeof(double) * size_t(terms) * K;
+  const size_t sh = comb_smem(terms, K);
   auto comb = k_cheb_combine<S>;
-  CCK(raise_smem_limit(reinterpret_cast<const void*>(comb), int(sh)));
   const int RG = kT / K;
   int64_t gs = (N + RG - 1) / RG;
   if (gs > 152 * 16) gs = 152 * 16;
@@ -457,10 +469,14 @@ std::string cheb_expm(const OpDev& op, const KrylovParams& p, ChebWork* w, doubl
                                        size_t(blocks_for(N, K, &rpb)) * K) +
                      sizeof(float2) * size_t(kBoundBlocks + 1) * K + 256;
   if (w->aux_bytes < aux) {
-    CCK(dev_free(w->aux, s));
+    dev_free(w->aux, s);
     w->aux = nullptr;
     w->aux_bytes = 0;
-    CCK(dev_alloc(&w->aux, aux, s));
+    if (dev_alloc(&w->aux, aux, s) != cudaSuccess) {
+      cudaGetLastError();
+      w->release(s);
+      return std::string();
+    }
     w->aux_bytes = aux;
   }
   float2* part = static_cast<float2*>(w->aux);
@@ -486,9 +502,14 @@ std::string cheb_expm(const OpDev& op, const KrylovParams& p, ChebWork* w, doubl
     J[k] = cheb_bessel(d[k] * dt, eps, nmax);
     if (J[k].empty()) return std::string();
   }
+  int terms = 1;
+  for (const auto& j : J) terms = int(j.size()) > terms ? int(j.size()) : terms;
+  const size_t vs = size_t(N) * 2 * K;
+  if (!(p.mixed ? reserve<float>(w, terms, K, vs, s) : reserve<double>(w, terms, K, vs, s)))
+    return std::string();
   *done = true;
-  return p.mixed ? run<float>(op, w, *T, n_steps, J, c, d, dt, X, drift, obs, s, rep, eps)
-                 : run<double>(op, w, *T, n_steps, J, c, d, dt, X, drift, obs, s, rep, eps);
+  return p.mixed ? run<float>(op, w, *T, n_steps, J, c, d, terms, dt, X, drift, obs, s, rep, eps)
+                 : run<double>(op, w, *T, n_steps, J, c, d, terms, dt, X, drift, obs, s, rep, eps);
 }
 
 }  // namespace lgt

@@ -2622,16 +2622,19 @@ std::string krylov_expm(const OpDev& op, const KrylovParams& p, KrylovCache* cac
                         int n_steps, double* X, double* norm_drift, StepObserver* obs,
                         cudaStream_t s, KrylovReport* rep) {
   if (op.K * 2 > kT) return "at most 128 complex points per panel";
-  // A step whose Chebyshev expansion takes at most krylovdim products runs as
-  // one (4x4 K = 8 mixed: see cheb.cu); longer steps, a forced H*psi kernel
-  // or LGT_EXPM=krylov (cross-checks) take the Krylov space, which halves
-  // the step until its space is large enough.
+  // A step whose Chebyshev expansion takes at most as many products as the
+  // Krylov space may have vectors (krylovdim, at most kMaxDim - 1) runs as one
+  // (4x4 K = 8 mixed: see cheb.cu); longer steps, panels that do not fit the
+  // memory, a forced H*psi kernel or LGT_EXPM=krylov (cross-checks) take the
+  // Krylov space, which halves the step until its space is large enough.
   const char* ex = getenv("LGT_EXPM");
   if (!(ex && ex[0] == 'k') && !hpsi_forced()) {
     OpDev o = op;
+    KrylovParams q = p;
+    if (q.krylovdim > kMaxDim - 1) q.krylovdim = kMaxDim - 1;
     bool done = false;
     if (dt > 0.0 && n_steps > 0 && ensure_table(&o, s)) {
-      const std::string err = cheb_expm(o, p, p.mixed ? &cache->cheb_f : &cache->cheb_d, dt,
+      const std::string err = cheb_expm(o, q, p.mixed ? &cache->cheb_f : &cache->cheb_d, dt,
                                         n_steps, X, norm_drift, obs, s, rep, &done);
       if (done || !err.empty()) return err;
     }

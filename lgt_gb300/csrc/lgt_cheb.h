@@ -20,8 +20,9 @@ struct ChebWork {
 
 // psi <- exp(-i H dt) psi, n_steps times with renormalisation after each, on
 // the complex panel X (as krylov_expm).  Runs when the table of `op` is
-// built, dt > 0 and the expansion needs at most p.krylovdim products a step;
-// otherwise *done stays false and nothing was changed.
+// built, dt > 0, the expansion needs at most p.krylovdim products a step and
+// its panels can be allocated; otherwise *done stays false and nothing was
+// changed.
 std::string cheb_expm(const OpDev& op, const KrylovParams& p, ChebWork* w, double dt, int n_steps,
                       double* X, double* drift, StepObserver* obs, cudaStream_t s,
                       KrylovReport* rep, bool* done);
