@@ -1,19 +1,19 @@
-// lgt_table_rows.cuh -- row-pull products from the stored neighbour table
-// for any panel width, with an optional three-term epilogue.
+// lgt_table_rows.cuh -- the products of the Chebyshev expansion (cheb.cu) from
+// the stored neighbour table:
+//
+//   y = scale ((H + shift) x), minus `prev` where it is given,
+//   H x = (cE e2 + cm stag) x + ch sum_hops (+-) x_j + cp sum_plaq x_j
+// (T_{n+1} = 2 H~ T_n - T_{n-1}; finite_ed.jl:265-318,
+// matter_gauge_entanglement_pjw.jl:82-147).  A panel row holds (re, im) of K
+// points.
 //
 // A warp copies the meta words and entries of its 32 rows into shared memory
 // (coalesced, evict-first) and runs its lanes over (row, W-column slice): a
 // lane sums the slices of the row's neighbours and applies the couplings
-// once.  W columns of T are one 4-, 8-, 16- or 32-byte access, so every
-// width divides into slices (W = 1 where C is odd).
-//
-//   plain  y = (cE e2 + cm stag) x + ch sum_hops (+-) x_j + cp sum_plaq x_j
-//   Cheb   y = scale ((H + shift) x), minus `prev` where it is given:
-//          T_{n+1} = 2 H~ T_n - T_{n-1}  (cheb.cu)
-// (finite_ed.jl:265-318; matter_gauge_entanglement_pjw.jl:82-147).
+// once.  A slice is one 8-, 16- or 32-byte access.
 #pragma once
 
-#include "lgt_hpsi.h"
+#include "lgt_cheb.h"
 #include "lgt_hpsi_gather.cuh"
 #include "lgt_intsum.cuh"
 
@@ -30,17 +30,11 @@ struct Args {
   const uint32_t* nbr;
   int mm;
   int64_t N;
-  int C, ncomp, K;
+  int K;
   const T* x;
   T* y;
-  const T* prev;          // Cheb: subtracted when not null
-  const T* coef;          // Cheb: [6][K] cE, cm, ch, cp, shift, scale
-  const T* cE;            // plain: the four coupling arrays
-  const T* cm;
-  const T* ch;
-  const T* cp;
-  const int* xsel;        // x + *xsel * xstride when not null
-  size_t xstride;
+  const T* prev;          // subtracted when not null
+  const T* coef;          // [6][K] cE, cm, ch, cp, shift, scale
 };
 
 template <typename T, int W>
@@ -54,11 +48,10 @@ __device__ __forceinline__ void ld_cols(const T* p, T (&r)[W]) {
   } else if constexpr (B == 16) {
     const double2 v = __ldg(reinterpret_cast<const double2*>(p));
     r[0] = v.x, r[1] = v.y;
-  } else if constexpr (B == 8 && sizeof(T) == 4) {
+  } else {
+    static_assert(B == 8 && sizeof(T) == 4, "slices of 8, 16 or 32 bytes");
     const float2 v = __ldg(reinterpret_cast<const float2*>(p));
     r[0] = v.x, r[1] = v.y;
-  } else {
-    r[0] = __ldg(p);
   }
 }
 
@@ -71,10 +64,9 @@ __device__ __forceinline__ void st_cols(T* p, const T (&r)[W]) {
     __stcs(reinterpret_cast<float4*>(p), make_float4(r[0], r[1], r[2], r[3]));
   } else if constexpr (B == 16) {
     __stcs(reinterpret_cast<double2*>(p), make_double2(r[0], r[1]));
-  } else if constexpr (B == 8 && sizeof(T) == 4) {
-    __stcs(reinterpret_cast<float2*>(p), make_float2(r[0], r[1]));
   } else {
-    __stcs(p, r[0]);
+    static_assert(B == 8 && sizeof(T) == 4, "slices of 8, 16 or 32 bytes");
+    __stcs(reinterpret_cast<float2*>(p), make_float2(r[0], r[1]));
   }
 }
 
@@ -120,12 +112,9 @@ __device__ __forceinline__ void sum_entries(const T* x, int C, int col0, const u
     sum_slices<T, W, U, SGN>(x, C, col0, lst, n0, n1, s);
 }
 
-__host__ __device__ inline int coef_words(bool cheb, int K) { return (cheb ? 6 : 4) * K; }
-
 template <typename T>
-__host__ __device__ inline int smem_bytes(bool cheb, int K, int mm) {
-  return (coef_words(cheb, K) * int(sizeof(T)) + 15) / 16 * 16 + 2 * kThreads * 4 +
-         kThreads * mm * 4;
+__host__ __device__ inline int smem_bytes(int K, int mm) {
+  return (6 * K * int(sizeof(T)) + 15) / 16 * 16 + 2 * kThreads * 4 + kThreads * mm * 4;
 }
 
 __device__ __forceinline__ int incl_scan(int v, int lane) {
@@ -137,26 +126,18 @@ __device__ __forceinline__ int incl_scan(int v, int lane) {
   return v;
 }
 
-template <typename T, int W, int U, bool PLAQ, bool JW, bool CHEB>
+template <typename T, int W, int U, bool PLAQ, bool JW>
 __global__ void __launch_bounds__(kThreads, PLAQ || JW || sizeof(T) == 8 ? 4 : 5)
-    k_table_rows(Args<T> a) {
+    k_cheb_product(Args<T> a) {
+  static_assert(W % 2 == 0, "a slice holds whole points");
   extern __shared__ __align__(16) unsigned char smem[];
-  const int K = a.K, C = a.C;
+  const int K = a.K, C = 2 * K;
   T* s_coef = reinterpret_cast<T*>(smem);
   uint32_t* s_meta =
-      reinterpret_cast<uint32_t*>(smem + (coef_words(CHEB, K) * int(sizeof(T)) + 15) / 16 * 16);
+      reinterpret_cast<uint32_t*>(smem + (6 * K * int(sizeof(T)) + 15) / 16 * 16);
   uint32_t* s_off = s_meta + kThreads;
   uint32_t* s_list = s_off + kThreads;
-  if constexpr (CHEB) {
-    for (int i = threadIdx.x; i < 6 * K; i += kThreads) s_coef[i] = a.coef[i];
-  } else {
-    for (int i = threadIdx.x; i < K; i += kThreads) {
-      s_coef[i] = a.cE[i];
-      s_coef[K + i] = a.cm[i];
-      s_coef[2 * K + i] = a.ch[i];
-      s_coef[3 * K + i] = a.cp[i];
-    }
-  }
+  for (int i = threadIdx.x; i < 6 * K; i += kThreads) s_coef[i] = a.coef[i];
   __syncthreads();
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int64_t row0 = (int64_t(blockIdx.x) * kWarps + wid) * 32;
@@ -172,7 +153,7 @@ __global__ void __launch_bounds__(kThreads, PLAQ || JW || sizeof(T) == 8 ? 4 : 5
   for (int i = lane; i < total; i += 32) lst[i] = __ldcs(src + i);
   __syncwarp();
 
-  const T* __restrict__ x = a.xsel ? a.x + size_t(*a.xsel) * a.xstride : a.x;
+  const T* __restrict__ x = a.x;
   const int lpr = C / W;
   const int items = 32 * lpr;
   for (int it = lane; it < items; it += 32) {
@@ -185,42 +166,34 @@ __global__ void __launch_bounds__(kThreads, PLAQ || JW || sizeof(T) == 8 ? 4 : 5
     const T e2 = T(int((mw >> 16) & 255u)), stag = T(int(mw >> 24) - 128);
     const uint32_t* l = lst + s_off[wid * 32 + rl];
     const size_t at = size_t(row) * C + col0;
+    const T* cf = s_coef + (col0 >> 1);  // the slice's points
     T xd[W], ah[W], out[W];
     ld_cols<T, W>(x + at, xd);
     sum_entries<T, W, U, JW>(x, C, col0, l, 0, nh, ah);
 #pragma unroll
     for (int e = 0; e < W; ++e) {
-      const int k = a.ncomp == 2 ? (col0 + e) >> 1 : col0 + e;
-      const T cd = CHEB ? fma(s_coef[k], e2, fma(s_coef[K + k], stag, s_coef[4 * K + k]))
-                        : fma(s_coef[k], e2, s_coef[K + k] * stag);
-      out[e] = fma(s_coef[2 * K + k], ah[e], cd * xd[e]);
+      const int k = e >> 1;
+      const T cd = fma(cf[k], e2, fma(cf[K + k], stag, cf[4 * K + k]));
+      out[e] = fma(cf[2 * K + k], ah[e], cd * xd[e]);
     }
     if (PLAQ) {
       sum_entries<T, W, U, false>(x, C, col0, l, nh, n1, ah);
 #pragma unroll
-      for (int e = 0; e < W; ++e) {
-        const int k = a.ncomp == 2 ? (col0 + e) >> 1 : col0 + e;
-        out[e] = fma(s_coef[3 * K + k], ah[e], out[e]);
-      }
+      for (int e = 0; e < W; ++e) out[e] = fma(cf[3 * K + (e >> 1)], ah[e], out[e]);
     }
-    if (CHEB) {
 #pragma unroll
-      for (int e = 0; e < W; ++e) ah[e] = T(0);
-      if (a.prev) ld_cols<T, W>(a.prev + at, ah);
+    for (int e = 0; e < W; ++e) ah[e] = T(0);
+    if (a.prev) ld_cols<T, W>(a.prev + at, ah);
 #pragma unroll
-      for (int e = 0; e < W; ++e) {
-        const int k = a.ncomp == 2 ? (col0 + e) >> 1 : col0 + e;
-        out[e] = fma(s_coef[5 * K + k], out[e], -ah[e]);
-      }
-    }
+    for (int e = 0; e < W; ++e) out[e] = fma(cf[5 * K + (e >> 1)], out[e], -ah[e]);
     st_cols<T, W>(a.y + at, out);
   }
 }
 
-template <typename T, int W, int U, bool PLAQ, bool JW, bool CHEB>
+template <typename T, int W, int U, bool PLAQ, bool JW>
 cudaError_t launch(const Args<T>& a, cudaStream_t s) {
-  auto kern = k_table_rows<T, W, U, PLAQ, JW, CHEB>;
-  const int bytes = smem_bytes<T>(CHEB, a.K, a.mm);
+  auto kern = k_cheb_product<T, W, U, PLAQ, JW>;
+  const int bytes = smem_bytes<T>(a.K, a.mm);
   const cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(kern), bytes);
   if (e != cudaSuccess) return e;
   const int64_t blocks = (a.N + kThreads - 1) / kThreads;
@@ -229,13 +202,30 @@ cudaError_t launch(const Args<T>& a, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-template <typename T, int W, int U, bool CHEB>
+template <typename T, int W, int U>
 cudaError_t launch_model(const Args<T>& a, uint32_t model, cudaStream_t s) {
   const bool plaq = model & kModelPlaq, jw = model & kModelJW;
-  if (plaq && jw) return launch<T, W, U, true, true, CHEB>(a, s);
-  if (plaq) return launch<T, W, U, true, false, CHEB>(a, s);
-  if (jw) return launch<T, W, U, false, true, CHEB>(a, s);
-  return launch<T, W, U, false, false, CHEB>(a, s);
+  if (plaq && jw) return launch<T, W, U, true, true>(a, s);
+  if (plaq) return launch<T, W, U, true, false>(a, s);
+  if (jw) return launch<T, W, U, false, true>(a, s);
+  return launch<T, W, U, false, false>(a, s);
+}
+
+template <typename T>
+Args<T> args(const NbrTable& t, int64_t N, int K, const T* x, T* y, const T* prev,
+             const T* coef) {
+  Args<T> a = {};
+  a.meta = t.meta;
+  a.off = t.tile_off;
+  a.nbr = t.nbr;
+  a.mm = t.mm;
+  a.N = N;
+  a.K = K;
+  a.x = x;
+  a.y = y;
+  a.prev = prev;
+  a.coef = coef;
+  return a;
 }
 
 }  // namespace rows

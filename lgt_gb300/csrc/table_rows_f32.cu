@@ -1,6 +1,5 @@
-// table_rows_f32.cu -- FP32 instances of the table products of
-// lgt_table_rows.cuh.
-#include "lgt_cheb.h"
+// table_rows_f32.cu -- FP32 instances of the expansion's products
+// (lgt_table_rows.cuh).
 #include "lgt_table_rows.cuh"
 
 namespace lgt {
@@ -11,21 +10,9 @@ namespace lgt {
 // with 32-byte slices, 35.1 with 16, 40.5 with 8.)
 cudaError_t launch_cheb_product(const NbrTable& T, uint32_t model, int64_t N, int K, const float* x,
                                 float* y, const float* prev, const float* coef, cudaStream_t s) {
-  rows::Args<float> a = {};
-  a.meta = T.meta;
-  a.off = T.tile_off;
-  a.nbr = T.nbr;
-  a.mm = T.mm;
-  a.N = N;
-  a.C = 2 * K;
-  a.ncomp = 2;
-  a.K = K;
-  a.x = x;
-  a.y = y;
-  a.prev = prev;
-  a.coef = coef;
-  if (a.C % 4 == 0) return rows::launch_model<float, 4, 8, true>(a, model, s);
-  return rows::launch_model<float, 2, 8, true>(a, model, s);
+  const rows::Args<float> a = rows::args(T, N, K, x, y, prev, coef);
+  if (K % 2 == 0) return rows::launch_model<float, 4, 8>(a, model, s);
+  return rows::launch_model<float, 2, 8>(a, model, s);
 }
 
 }  // namespace lgt
