@@ -10,16 +10,21 @@
 // earlier vectors per product, 55 % of a 4x4 K = 8 step): a product reads
 // T_n (gathered) and T_{n-1} once and writes T_{n+1}, and one pass at the end
 // sums the stored panels.  Measured against the Krylov step, observables
-// included: 4x4 K = 8 mixed, two steps of dt = 0.05, 114.6 -> 35.1 ms; 4x4
-// K = 3 FP64 with plaquettes, one step, 85.1 -> 37.9 ms (bound by the FP64
-// pipe of the products); 3x4 K = 1 FP64, ten steps, 13.5 -> 2.3 ms; the
-// error against exact propagation is unchanged (5.7e-8, 4.4e-15, 7.6e-15).
+// included: 4x4 K = 8 mixed, two steps of dt = 0.05, 114.6 -> 36.4 ms; 4x4
+// K = 3 FP64 with plaquettes, one step, 85.1 -> 36.5 ms (bound by the FP64
+// pipe of the products); 3x4 K = 1 FP64, ten steps, 13.5 -> 2.3 ms.
 //
-// The products apply H's couplings as they are and multiply the finished sum
-// by 2 / d; c and 1 / d are taken as FP32 numbers.  (Couplings divided by d
-// and then rounded to FP32 shift every energy by up to 6e-8 of itself; the 4x4
-// K = 8 mixed quench, two steps, is now off by 2.5e-8 - 3.0e-8 of the FP64
-// state, the Krylov steps by 3.0e-8 - 3.7e-8.)
+// Errors.  FP64: that of the Krylov steps (3e-15 to 9e-15).  Mixed: every T_n is
+// rounded to FP32 once, when it is stored.  The couplings of the products are
+// scaled on the host and kept as pairs of FP32 numbers (pair_coefs), the
+// neighbours are added pairwise, and of T_1, which a short step is made of
+// beside T_0, the part that the rounding drops is kept too.  The state's
+// distance from the FP64 one, against that of the Krylov steps (three sets of
+// points each): 4x4 K = 8, two steps of 0.05: 1.3e-8 - 1.6e-8 (3.5e-8); 4x3
+// K = 2 with plaquettes, the same: 1.0e-8 - 1.1e-8 (1.7e-8 - 3.3e-8); 3x4
+// K = 2, six steps of 0.1: 6.9e-8 - 8.1e-8 (8.5e-8 - 9.4e-8); 3x3, one step of
+// 0.03: 2.1e-10 - 2.7e-10 (2.0e-9).  (With FP32 couplings, the scale apart and
+// one chain of sums it was 3.0e-8 - 3.9e-8 for the first of these.)
 //
 // The bounds are Gershgorin's, per point, from the table's row meta words
 // (diagonal and entry counts) in FP32, widened by 1e-5 of their size.  The
@@ -183,10 +188,13 @@ __global__ void __launch_bounds__(kT) k_cheb_start(double2* X, S* V, int64_t N, 
 // partial sums of the new norms.  coef[n][k] = +-J_n (2 - [n = 0]): an even n
 // adds coef T_n, an odd one -i coef T_n, to (re, im).  FP32 panels: double-
 // float sums (coefficients split into FP32 pairs once per block) beside the
-// FP64 first term, which is taken from X itself; FP64 panels: FP64 sums.
-// Bound by the panels' bytes (terms S 2 N K read once) in FP32.
+// FP64 first term, which is taken from X itself, and the part of T_1 that FP32
+// drops from `low` (a short step is little more than its first two terms);
+// FP64 panels: FP64 sums.  Bound by the panels' bytes ((terms + 1) S 2 N K read
+// once) in FP32.
 template <typename S>
 __global__ void __launch_bounds__(kT) k_cheb_combine(const S* __restrict__ V, size_t vstride,
+                                                     const S* __restrict__ low,
                                                      const double* coef, int terms, double2* X,
                                                      int64_t N, int K, int64_t rpb,
                                                      const int* perm, double* part) {
@@ -246,6 +254,12 @@ __global__ void __launch_bounds__(kT) k_cheb_combine(const S* __restrict__ V, si
               }
             }
         }
+        if (terms > 1) {
+          const float2 t =
+              __ldcs(reinterpret_cast<const float2*>(low + (size_t(r) * K + k) * 2));
+          ar.lo = df_fma_rn(s_hi[K + k], t.y, ar.lo);
+          ai.lo = df_fma_rn(-s_hi[K + k], t.x, ai.lo);
+        }
         re = fma(a0, x0.x, widen(ar.hi) + widen(ar.lo));
         im = fma(a0, x0.y, widen(ai.hi) + widen(ai.lo));
       } else {
@@ -291,14 +305,37 @@ int blocks_for(int64_t N, int K, int64_t* rpb) {
   return int((N + *rpb - 1) / *rpb);
 }
 
+// The FP32 products' coefficients (PairCoef) of one point: out[q * K].  cc:
+// cE, cm, ch, cp at [q * K].  The leading parts of the diagonal's three terms
+// are multiples of a unit of which no sum of them reaches 2^24: a row's
+// diagonal is then exact in FP32, however its terms are added.
+void pair_coefs(const Geom& G, const double* cc, int K, double shift, double scale, float* out) {
+  const double el = scale * cc[0], mass = scale * cc[K], sh = scale * shift;
+  const double most = std::fabs(el) * double((G.nR + G.nU) * G.dg * G.dg) +
+                      std::fabs(mass) * double(G.ns) + std::fabs(sh);
+  int e = 0;
+  std::frexp(most, &e);  // most < 2^e
+  const double unit = std::ldexp(1.0, e - 23);
+  auto put = [&](int q, double v, double hi) {
+    out[size_t(q) * K] = float(hi);
+    out[size_t(q + 1) * K] = float(v - double(float(hi)));
+  };
+  put(kElHi, el, std::nearbyint(el / unit) * unit);
+  put(kMassHi, mass, std::nearbyint(mass / unit) * unit);
+  put(kShiftHi, sh, std::nearbyint(sh / unit) * unit);
+  put(kHopHi, scale * cc[2 * K], scale * cc[2 * K]);
+  put(kPlaqHi, scale * cc[3 * K], scale * cc[3 * K]);
+}
+
 // Dynamic shared memory of k_cheb_combine.
 size_t comb_smem(int terms, int K) { return sizeof(double) * size_t(terms) * K; }
 
 // Device memory and shared memory for an expansion of `terms` panels of `vs`
-// elements; false (with nothing held) where they cannot be had.
+// elements (FP32: and T_1's dropped part behind them); false (with nothing
+// held) where they cannot be had.
 template <typename S>
 bool reserve(ChebWork* w, int terms, int K, size_t vs, cudaStream_t s) {
-  const size_t need = sizeof(S) * vs * size_t(terms) + 256;
+  const size_t need = sizeof(S) * vs * size_t(terms + (sizeof(S) == 4 ? 1 : 0)) + 256;
   cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(k_cheb_combine<S>),
                                    int(comb_smem(terms, K)));
   if (e == cudaSuccess && w->v_bytes < need) {
@@ -323,6 +360,7 @@ std::string run(const OpDev& op, ChebWork* w, const NbrTable& T, int n_steps,
   const int K = op.K;
   const size_t vs = size_t(N) * 2 * K;
   S* V = static_cast<S*>(w->V);
+  S* low = V + size_t(terms) * vs;  // (FP32 only)
   int64_t rpb = 1;
   const int nblk = blocks_for(N, K, &rpb);
   // aux (the bounds in it have been read): coefficients, norms, partial sums
@@ -331,9 +369,10 @@ std::string run(const OpDev& op, ChebWork* w, const NbrTable& T, int n_steps,
   double* a_rho = a_phase + 2 * K;
   double* a_rho0 = a_rho + K;
   double* a_drift = a_rho0 + K;
-  // [6][K]: couplings, shift and scale of the first product; of the others
+  // coefficients of the first product; of the others
+  constexpr int kCoefs = sizeof(S) == 4 ? int(kPairCoefs) : 6;  // (12 K doubles hold both)
   S* a_c1 = reinterpret_cast<S*>(a_drift + K);
-  S* a_c2 = a_c1 + 6 * size_t(K);
+  S* a_c2 = a_c1 + kCoefs * size_t(K);
   const size_t host_n = size_t(terms) * K + 5 * size_t(K) + 12 * size_t(K);
   int* a_fail = reinterpret_cast<int*>(a_coef + host_n);
   double* a_part = a_coef + host_n + 1;
@@ -342,7 +381,7 @@ std::string run(const OpDev& op, ChebWork* w, const NbrTable& T, int n_steps,
   CCK(cudaMemcpyAsync(cc.data(), op.cE_d, sizeof(double) * 4 * K, cudaMemcpyDeviceToHost, s));
   CCK(cudaStreamSynchronize(s));
   S* h1 = reinterpret_cast<S*>(h.data() + size_t(terms) * K + 5 * size_t(K));
-  S* h2 = h1 + 6 * size_t(K);
+  S* h2 = h1 + kCoefs * size_t(K);
   for (int k = 0; k < K; ++k) {
     for (size_t n = 0; n < J[k].size(); ++n) {
       const double j = (n == 0 ? 1.0 : 2.0) * J[k][n];
@@ -351,10 +390,16 @@ std::string run(const OpDev& op, ChebWork* w, const NbrTable& T, int n_steps,
     const double ph = -c[k] * dt * double(n_steps);
     h[size_t(terms) * K + 2 * k] = std::cos(ph);
     h[size_t(terms) * K + 2 * k + 1] = std::sin(ph);
-    for (int q = 0; q < 5; ++q)
-      h1[size_t(q) * K + k] = h2[size_t(q) * K + k] = S(q < 4 ? cc[size_t(q) * K + k] : -c[k]);
-    h1[5 * size_t(K) + k] = S(1.0 / d[k]);  // exact in S, like the shift
-    h2[5 * size_t(K) + k] = S(2.0 / d[k]);
+    const double* ck = cc.data() + k;
+    if constexpr (sizeof(S) == 4) {
+      pair_coefs(op.G, ck, K, -c[k], 1.0 / d[k], h1 + k);
+      pair_coefs(op.G, ck, K, -c[k], 2.0 / d[k], h2 + k);
+    } else {
+      for (int q = 0; q < 5; ++q)
+        h1[size_t(q) * K + k] = h2[size_t(q) * K + k] = q < 4 ? ck[size_t(q) * K] : -c[k];
+      h1[5 * size_t(K) + k] = 1.0 / d[k];
+      h2[5 * size_t(K) + k] = 2.0 / d[k];
+    }
   }
   // (a copy from pageable memory has staged the host data when it returns)
   CCK(cudaMemcpyAsync(a_coef, h.data(), sizeof(double) * h.size(), cudaMemcpyHostToDevice, s));
@@ -378,10 +423,18 @@ std::string run(const OpDev& op, ChebWork* w, const NbrTable& T, int n_steps,
   k_cheb_start<S><<<unsigned(gs), kT, 0, s>>>(X, V, N, K, a_rho0, nullptr, perm), note_launch();
   CCK(cudaGetLastError());
   for (int step = 1; step <= n_steps; ++step) {
-    for (int n = 1; n < terms; ++n)
-      CCK(launch_cheb_product(T, op.model, N, K, V + size_t(n - 1) * vs, V + size_t(n) * vs,
-                              n > 1 ? V + size_t(n - 2) * vs : nullptr, n > 1 ? a_c2 : a_c1, s));
-    comb<<<nblk, kT, sh, s>>>(V, vs, a_coef, terms, X, N, K, rpb, perm, a_part), note_launch();
+    for (int n = 1; n < terms; ++n) {
+      const S* x = V + size_t(n - 1) * vs;
+      S* y = V + size_t(n) * vs;
+      const S* prev = n > 1 ? V + size_t(n - 2) * vs : nullptr;
+      const S* cf = n > 1 ? a_c2 : a_c1;
+      if constexpr (sizeof(S) == 4)
+        CCK(launch_cheb_product(T, op.model, N, K, x, y, prev, n == 1 ? low : nullptr, cf, s));
+      else
+        CCK(launch_cheb_product(T, op.model, N, K, x, y, prev, cf, s));
+    }
+    comb<<<nblk, kT, sh, s>>>(V, vs, low, a_coef, terms, X, N, K, rpb, perm, a_part),
+        note_launch();
     k_cheb_finish<<<K, 32, 0, s>>>(a_part, nblk, K, a_rho, step == 1 ? a_rho0 : nullptr, a_drift,
                                    a_fail), note_launch();
     const bool last = step == n_steps;

@@ -31,10 +31,20 @@ std::string cheb_expm(const OpDev& op, const KrylovParams& p, ChebWork* w, doubl
 // 2 sum_{m > n} |J_m(z)| is below eps; empty when n would pass nmax.
 std::vector<double> cheb_bessel(double z, double eps, int nmax);
 
+// Rows of the FP32 products' coefficients: the couplings times the scale, each
+// as a leading and a trailing FP32 number (cheb.cu).
+enum PairCoef : int {
+  kElHi, kElLo, kMassHi, kMassLo, kShiftHi, kShiftLo, kHopHi, kHopLo, kPlaqHi, kPlaqLo,
+  kPairCoefs
+};
+
 // The products of the expansion from the stored table (one translation unit
-// per precision): y = scale (H + shift) x (- prev), coef = [6][K].
+// per precision): y = scale (H + shift) x (- prev).  FP64: coef = [6][K].
+// FP32: coef = [kPairCoefs][K]; the part of y that its rounding drops goes to
+// `low` when that is given.
 cudaError_t launch_cheb_product(const NbrTable& T, uint32_t model, int64_t N, int K, const float* x,
-                                float* y, const float* prev, const float* coef, cudaStream_t s);
+                                float* y, const float* prev, float* low, const float* coef,
+                                cudaStream_t s);
 cudaError_t launch_cheb_product(const NbrTable& T, uint32_t model, int64_t N, int K,
                                 const double* x, double* y, const double* prev,
                                 const double* coef, cudaStream_t s);

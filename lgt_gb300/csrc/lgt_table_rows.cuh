@@ -11,9 +11,19 @@
 // (coalesced, evict-first) and runs its lanes over (row, W-column slice): a
 // lane sums the slices of the row's neighbours and applies the couplings
 // once.  A slice is one 8-, 16- or 32-byte access.
+//
+// FP32 panels: A x + B sum_hops + C sum_plaq - prev with the scale folded into
+// the couplings, these as pairs of FP32 numbers (PairCoef below), and the
+// neighbours added pairwise, so that a new entry sees about three roundings
+// of its own size (errors: cheb.cu).  The 4x4 K = 8 quench takes 36.4 ms a run
+// with them, 35.2 with FP32 couplings, one chain of sums and the scale apart;
+// with every error carried by TwoSum and TwoProduct 48.0 (and two thirds of
+// the state's error).  Where `low` is given, an entry's products and their sum
+// carry their errors and what its rounding drops is stored.
 #pragma once
 
 #include "lgt_cheb.h"
+#include "lgt_dfloat.cuh"
 #include "lgt_hpsi_gather.cuh"
 #include "lgt_intsum.cuh"
 
@@ -34,7 +44,8 @@ struct Args {
   const T* x;
   T* y;
   const T* prev;          // subtracted when not null
-  const T* coef;          // [6][K] cE, cm, ch, cp, shift, scale
+  T* low;                 // FP32: the dropped part of y when not null
+  const T* coef;          // FP64: [6][K] cE, cm, ch, cp, shift, scale; FP32: PairCoef
 };
 
 template <typename T, int W>
@@ -70,51 +81,59 @@ __device__ __forceinline__ void st_cols(T* p, const T (&r)[W]) {
   }
 }
 
-// s = the sum of the slices of entries lst[n0 .. n1), U of them in flight (the
-// last trip adds zeros for the entries it lacks); SGN: bit 31 of an entry
-// flips the sign.
-template <typename T, int W, int U, bool SGN>
-__device__ __forceinline__ void sum_slices(const T* x, int C, int col0, const uint32_t* lst,
-                                           int n0, int n1, T (&s)[W]) {
+// s = the sum of the slices of entries lst[n0 .. n1), eight of them in flight
+// and added pairwise (the last trip adds zeros for the entries it lacks); SGN:
+// bit 31 of an entry flips the sign.
+template <int W, bool SGN>
+__device__ __forceinline__ void sum_slices(const float* x, int C, int col0, const uint32_t* lst,
+                                           int n0, int n1, float (&s)[W]) {
 #pragma unroll
-  for (int e = 0; e < W; ++e) s[e] = T(0);
-  for (int n = n0; n < n1; n += U) {
-    T v[U][W];
-    uint32_t ent[U];
+  for (int e = 0; e < W; ++e) s[e] = 0.f;
+  for (int n = n0; n < n1; n += 8) {
+    float v[8][W];
+    uint32_t ent[8];
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
+    for (int u = 0; u < 8; ++u) {
       if (n + u < n1) {
         ent[u] = lst[n + u];
-        ld_cols<T, W>(x + size_t(ent[u] & 0x7fffffffu) * C + col0, v[u]);
+        ld_cols<float, W>(x + size_t(ent[u] & 0x7fffffffu) * C + col0, v[u]);
       } else {
         ent[u] = 0u;
 #pragma unroll
-        for (int e = 0; e < W; ++e) v[u][e] = T(0);
+        for (int e = 0; e < W; ++e) v[u][e] = 0.f;
       }
     }
+    float sg[8];
 #pragma unroll
-    for (int u = 0; u < U; ++u)
+    for (int u = 0; u < 8; ++u) sg[u] = (ent[u] >> 31) ? -1.f : 1.f;
 #pragma unroll
-      for (int e = 0; e < W; ++e)
-        s[e] = SGN ? fma((ent[u] >> 31) ? T(-1) : T(1), v[u][e], s[e]) : s[e] + v[u][e];
+    for (int e = 0; e < W; ++e) {
+      float t[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        t[u] = SGN ? fmaf(sg[2 * u], v[2 * u][e], sg[2 * u + 1] * v[2 * u + 1][e])
+                   : v[2 * u][e] + v[2 * u + 1][e];
+      s[e] += (t[0] + t[1]) + (t[2] + t[3]);
+    }
   }
 }
 
-// A row's sum over entries lst[n0 .. n1) in T: FP64 by integers.
-template <typename T, int W, int U, bool SGN>
-__device__ __forceinline__ void sum_entries(const T* x, int C, int col0, const uint32_t* lst,
-                                            int n0, int n1, T (&s)[W]) {
-  if constexpr (sizeof(T) == 8)
-    int_sum<W, U, SGN>(lst, n0, n1, s, [&](uint32_t j, double(&v)[W]) {
-      ld_cols<double, W>(x + size_t(j) * C + col0, v);
-    });
-  else
-    sum_slices<T, W, U, SGN>(x, C, col0, lst, n0, n1, s);
+// h + l += (c + d) s
+__device__ __forceinline__ void add_prod(float c, float d, float s, float& h, float& l) {
+  float p, e, q;
+  two_prod(c, s, p, e);
+  e = df_fma_rn(d, s, e);
+  two_sum(h, p, h, q);
+  l = df_add_rn(l, df_add_rn(q, e));
 }
 
 template <typename T>
+__host__ __device__ constexpr int coef_rows() { return sizeof(T) == 4 ? kPairCoefs : 6; }
+
+template <typename T>
 __host__ __device__ inline int smem_bytes(int K, int mm) {
-  return (6 * K * int(sizeof(T)) + 15) / 16 * 16 + 2 * kThreads * 4 + kThreads * mm * 4;
+  return (coef_rows<T>() * K * int(sizeof(T)) + 15) / 16 * 16 + 2 * kThreads * 4 +
+         kThreads * mm * 4;
 }
 
 __device__ __forceinline__ int incl_scan(int v, int lane) {
@@ -126,6 +145,16 @@ __device__ __forceinline__ int incl_scan(int v, int lane) {
   return v;
 }
 
+// The scaled and shifted diagonal of a row: the leading parts are multiples of
+// one unit, so their sum is exact (cheb.cu).
+__device__ __forceinline__ float diag_hi(const float* c, int K, float e2, float stag) {
+  return fmaf(c[kElHi * K], e2, fmaf(c[kMassHi * K], stag, c[kShiftHi * K]));
+}
+__device__ __forceinline__ float diag_lo(const float* c, int K, float e2, float stag) {
+  return fmaf(c[kElLo * K], e2, fmaf(c[kMassLo * K], stag, c[kShiftLo * K]));
+}
+
+// U: entries in flight (FP64; FP32 has eight).
 template <typename T, int W, int U, bool PLAQ, bool JW>
 __global__ void __launch_bounds__(kThreads, PLAQ || JW || sizeof(T) == 8 ? 4 : 5)
     k_cheb_product(Args<T> a) {
@@ -134,10 +163,10 @@ __global__ void __launch_bounds__(kThreads, PLAQ || JW || sizeof(T) == 8 ? 4 : 5
   const int K = a.K, C = 2 * K;
   T* s_coef = reinterpret_cast<T*>(smem);
   uint32_t* s_meta =
-      reinterpret_cast<uint32_t*>(smem + (6 * K * int(sizeof(T)) + 15) / 16 * 16);
+      reinterpret_cast<uint32_t*>(smem + (coef_rows<T>() * K * int(sizeof(T)) + 15) / 16 * 16);
   uint32_t* s_off = s_meta + kThreads;
   uint32_t* s_list = s_off + kThreads;
-  for (int i = threadIdx.x; i < 6 * K; i += kThreads) s_coef[i] = a.coef[i];
+  for (int i = threadIdx.x; i < coef_rows<T>() * K; i += kThreads) s_coef[i] = a.coef[i];
   __syncthreads();
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int64_t row0 = (int64_t(blockIdx.x) * kWarps + wid) * 32;
@@ -167,25 +196,66 @@ __global__ void __launch_bounds__(kThreads, PLAQ || JW || sizeof(T) == 8 ? 4 : 5
     const uint32_t* l = lst + s_off[wid * 32 + rl];
     const size_t at = size_t(row) * C + col0;
     const T* cf = s_coef + (col0 >> 1);  // the slice's points
-    T xd[W], ah[W], out[W];
+    T xd[W], out[W];
     ld_cols<T, W>(x + at, xd);
-    sum_entries<T, W, U, JW>(x, C, col0, l, 0, nh, ah);
+    if constexpr (sizeof(T) == 8) {
+      T ah[W];
+      auto load = [&](uint32_t j, double(&v)[W]) {
+        ld_cols<double, W>(x + size_t(j) * C + col0, v);
+      };
+      int_sum<W, U, JW>(l, 0, nh, ah, load);
 #pragma unroll
-    for (int e = 0; e < W; ++e) {
-      const int k = e >> 1;
-      const T cd = fma(cf[k], e2, fma(cf[K + k], stag, cf[4 * K + k]));
-      out[e] = fma(cf[2 * K + k], ah[e], cd * xd[e]);
+      for (int e = 0; e < W; ++e) {
+        const int k = e >> 1;
+        const T cd = fma(cf[k], e2, fma(cf[K + k], stag, cf[4 * K + k]));
+        out[e] = fma(cf[2 * K + k], ah[e], cd * xd[e]);
+      }
+      if (PLAQ) {
+        int_sum<W, U, false>(l, nh, n1, ah, load);
+#pragma unroll
+        for (int e = 0; e < W; ++e) out[e] = fma(cf[3 * K + (e >> 1)], ah[e], out[e]);
+      }
+#pragma unroll
+      for (int e = 0; e < W; ++e) ah[e] = T(0);
+      if (a.prev) ld_cols<T, W>(a.prev + at, ah);
+#pragma unroll
+      for (int e = 0; e < W; ++e) out[e] = fma(cf[5 * K + (e >> 1)], out[e], -ah[e]);
+    } else {
+      T ah[W], ap[W], pv[W];
+      sum_slices<W, JW>(x, C, col0, l, 0, nh, ah);
+      if (PLAQ) sum_slices<W, false>(x, C, col0, l, nh, n1, ap);
+#pragma unroll
+      for (int e = 0; e < W; ++e) pv[e] = 0.f;
+      if (a.prev) ld_cols<T, W>(a.prev + at, pv);
+      if (a.low) {
+        T low[W];
+#pragma unroll
+        for (int e = 0; e < W; ++e) {
+          const float* c = cf + (e >> 1);
+          out[e] = -pv[e];
+          low[e] = 0.f;
+          add_prod(diag_hi(c, K, e2, stag), diag_lo(c, K, e2, stag), xd[e], out[e], low[e]);
+          add_prod(c[kHopHi * K], c[kHopLo * K], ah[e], out[e], low[e]);
+          if (PLAQ) add_prod(c[kPlaqHi * K], c[kPlaqLo * K], ap[e], out[e], low[e]);
+          fast_two_sum(out[e], low[e], out[e], low[e]);
+        }
+        st_cols<T, W>(a.low + at, low);
+      } else {
+#pragma unroll
+        for (int p = 0; p < W / 2; ++p) {
+          const float* c = cf + p;
+          const float dh = diag_hi(c, K, e2, stag), dl = diag_lo(c, K, e2, stag);
+#pragma unroll
+          for (int e = 2 * p; e < 2 * p + 2; ++e) {
+            // the small terms first, T_{n-1} last
+            float t = fmaf(dl, xd[e], c[kHopLo * K] * ah[e]);
+            if (PLAQ) t = fmaf(c[kPlaqHi * K], ap[e], fmaf(c[kPlaqLo * K], ap[e], t));
+            t = fmaf(c[kHopHi * K], ah[e], t);
+            out[e] = fmaf(dh, xd[e], t) - pv[e];
+          }
+        }
+      }
     }
-    if (PLAQ) {
-      sum_entries<T, W, U, false>(x, C, col0, l, nh, n1, ah);
-#pragma unroll
-      for (int e = 0; e < W; ++e) out[e] = fma(cf[3 * K + (e >> 1)], ah[e], out[e]);
-    }
-#pragma unroll
-    for (int e = 0; e < W; ++e) ah[e] = T(0);
-    if (a.prev) ld_cols<T, W>(a.prev + at, ah);
-#pragma unroll
-    for (int e = 0; e < W; ++e) out[e] = fma(cf[5 * K + (e >> 1)], out[e], -ah[e]);
     st_cols<T, W>(a.y + at, out);
   }
 }
@@ -212,7 +282,7 @@ cudaError_t launch_model(const Args<T>& a, uint32_t model, cudaStream_t s) {
 }
 
 template <typename T>
-Args<T> args(const NbrTable& t, int64_t N, int K, const T* x, T* y, const T* prev,
+Args<T> args(const NbrTable& t, int64_t N, int K, const T* x, T* y, const T* prev, T* low,
              const T* coef) {
   Args<T> a = {};
   a.meta = t.meta;
@@ -224,6 +294,7 @@ Args<T> args(const NbrTable& t, int64_t N, int K, const T* x, T* y, const T* pre
   a.x = x;
   a.y = y;
   a.prev = prev;
+  a.low = low;
   a.coef = coef;
   return a;
 }

@@ -9,8 +9,9 @@ namespace lgt {
 // in flight with the smaller ones: 4x4 K = 8 quench, FP32-mixed, 35.9 ms a run
 // with 32-byte slices, 35.1 with 16, 40.5 with 8.)
 cudaError_t launch_cheb_product(const NbrTable& T, uint32_t model, int64_t N, int K, const float* x,
-                                float* y, const float* prev, const float* coef, cudaStream_t s) {
-  const rows::Args<float> a = rows::args(T, N, K, x, y, prev, coef);
+                                float* y, const float* prev, float* low, const float* coef,
+                                cudaStream_t s) {
+  const rows::Args<float> a = rows::args(T, N, K, x, y, prev, low, coef);
   if (K % 2 == 0) return rows::launch_model<float, 4, 8>(a, model, s);
   return rows::launch_model<float, 2, 8>(a, model, s);
 }

@@ -8,7 +8,7 @@ namespace lgt {
 cudaError_t launch_cheb_product(const NbrTable& T, uint32_t model, int64_t N, int K,
                                 const double* x, double* y, const double* prev,
                                 const double* coef, cudaStream_t s) {
-  const rows::Args<double> a = rows::args(T, N, K, x, y, prev, coef);
+  const rows::Args<double> a = rows::args<double>(T, N, K, x, y, prev, nullptr, coef);
   if (K % 2 == 0) return rows::launch_model<double, 4, 2>(a, model, s);
   return rows::launch_model<double, 2, 4>(a, model, s);
 }
