@@ -2147,6 +2147,16 @@ GridPlan plan_grid(OpDev* op, int64_t N, int C, int m, cudaStream_t s) {
   return g;
 }
 
+// SM cycles that the cycle's barriers wait (~4 s: a kernel of another stream
+// may hold SMs).  LGT_PANEL_GRID_SPIN: another number (tests).
+long long grid_spin() {
+  const char* e = getenv("LGT_PANEL_GRID_SPIN");
+  return e && e[0] ? atoll(e) : 8000000000LL;
+}
+
+// *steps is negative where a barrier's wait ran out (the basis panels and the
+// points' states are then undefined, V_0 and X as they were) or where the
+// launch is not to be had (no memory, not all blocks at once).
 template <typename S>
 std::string run_grid_cycle(const OpDev& op, Work<S>& w, const KrylovParams& p, const GridPlan& g,
                            double tol, double tiny_rel, cudaStream_t s, int* steps) {
@@ -2156,7 +2166,12 @@ std::string run_grid_cycle(const OpDev& op, Work<S>& w, const KrylovParams& p, c
     cudaFree(w.gbuf);
     w.gbuf = nullptr;
     w.gbuf_n = 0;
-    KCK(cudaMalloc(&w.gbuf, sizeof(double) * need));
+    if (cudaMalloc(&w.gbuf, sizeof(double) * need) != cudaSuccess) {
+      cudaGetLastError();
+      w.gbuf = nullptr;
+      *steps = -1;
+      return std::string();
+    }
     w.gbuf_n = need;
   }
   GridArgs<S> a = {};
@@ -2193,11 +2208,15 @@ std::string run_grid_cycle(const OpDev& op, Work<S>& w, const KrylovParams& p, c
   a.h = w.gbuf + 2;
   a.npart = a.h + (size_t(w.m) + 1) * w.C;
   a.part = a.npart + per;
-  a.err = op.err;
+  a.spin = grid_spin();
   a.list_smem = g.list_smem;
   KCK(cudaMemsetAsync(w.gbuf, 0, sizeof(double), s));
   KCK(cudaMemsetAsync(w.gbuf + 1, 0xff, sizeof(double), s));  // -1: a cycle that was cut short
-  KCK(launch_lanczos_grid<S>(a, g.bytes, s));
+  if (launch_lanczos_grid<S>(a, g.bytes, s) != cudaSuccess) {
+    cudaGetLastError();
+    *steps = -1;
+    return std::string();
+  }
   KCK(cudaMemcpyAsync(steps, a.steps, sizeof(int), cudaMemcpyDeviceToHost, s));
   return std::string();
 }
@@ -2218,18 +2237,26 @@ std::string ground_state_impl(const OpDev& op_in, const KrylovParams& p, Work<S>
     w.release();
     return err;
   }
-  const GridPlan grid = plan_grid<S>(&op, N, C, m, s);
+  GridPlan grid = plan_grid<S>(&op, N, C, m, s);
+  const int* perm = nullptr;
+  auto multi_launch = [&]() -> std::string {
+    const std::string e = autotune<S>(&op, w, s, nullptr);
+    if (!e.empty()) return e;
+    // the Krylov vectors in the table's row order when its kernel was chosen
+    // and serves these panels: X is gathered into V_0 and the combinations
+    // scattered back
+    op.krylov_order = (use_krylov_order(op) && table_serves(op, w)) ? 1 : 0;
+    perm = op.krylov_order ? op.table_ord->perm : nullptr;
+    return std::string();
+  };
   if (grid.on) {
     op.use_table = 1;  // the FP64 finish
+    op.krylov_order = 0;
+    perm = grid.T->perm;
   } else {
-    err = autotune<S>(&op, w, s, nullptr);
+    err = multi_launch();
     if (!err.empty()) return err;
   }
-  // the Krylov vectors in the table's row order when its kernel was chosen
-  // and serves these panels: X is gathered into V_0 and the combinations
-  // scattered back
-  op.krylov_order = (!grid.on && use_krylov_order(op) && table_serves(op, w)) ? 1 : 0;
-  const int* perm = grid.on ? grid.T->perm : op.krylov_order ? op.table_ord->perm : nullptr;
   const bool fp32 = sizeof(S) == 4;
   const double tiny_rel = fp32 ? 1e-6 : 1e-12;
   // FP32 panels cannot resolve residuals much below 1e-6 |H|: the inner
@@ -2252,7 +2279,7 @@ std::string ground_state_impl(const OpDev& op_in, const KrylovParams& p, Work<S>
   err = start_from<S>(w, X, s, perm);
   if (!err.empty()) return err;
 
-  std::vector<int> st(K);
+  std::vector<int> st(K), st0(K, kActive);  // st0: when the cycle began
   int j = 0, restarts = 0;
   int64_t matvecs = 0;
   bool noconv = false;
@@ -2273,7 +2300,20 @@ std::string ground_state_impl(const OpDev& op_in, const KrylovParams& p, Work<S>
     KCK(cudaGetLastError());
     KCK(cudaMemcpyAsync(st.data(), w.status, sizeof(int) * K, cudaMemcpyDeviceToHost, s));
     KCK(cudaStreamSynchronize(s));
-    if (cycle < 0) return "a bounded wait of the Lanczos cycle expired";
+    if (cycle < 0) {
+      // the cycle did not run to its end: again from X by single launches
+      grid.on = false;
+      op.use_table = 0;
+      err = multi_launch();
+      if (!err.empty()) return err;
+      KCK(cudaMemcpyAsync(w.status, st0.data(), sizeof(int) * K, cudaMemcpyHostToDevice, s));
+      err = reset_cycle<S>(w, s);
+      if (!err.empty()) return err;
+      err = start_from<S>(w, X, s, perm);
+      if (!err.empty()) return err;
+      j = 0;
+      continue;
+    }
     matvecs += cycle;
     bool all = true;
     for (int k = 0; k < K; ++k) all = all && (st[k] >= kConverged);
@@ -2295,6 +2335,7 @@ std::string ground_state_impl(const OpDev& op_in, const KrylovParams& p, Work<S>
       if (!err.empty()) return err;
       err = start_from<S>(w, X, s, perm);
       if (!err.empty()) return err;
+      for (int k = 0; k < K; ++k) st0[k] = st[k] >= kConverged ? int(kWritten) : st[k];
       j = 0;
       ++restarts;
     }

@@ -23,7 +23,8 @@
 // decisions from the same values.
 //
 // The grid barrier counts arrivals in one word; its wait is bounded by the
-// SM clock and raises kDevErrSpin (all blocks then leave).
+// SM clock (GridArgs::spin).  Where it runs out, the blocks leave and no step
+// count is written; the driver then takes the multi-launch steps.
 #include <type_traits>
 
 #include "lgt_dfloat.cuh"
@@ -48,7 +49,6 @@ struct Threads {
 };
 constexpr int kQ = 8;               // basis vectors per dot chunk
 constexpr int kSmemMax = 214 * 1024;  // beside the static arrays
-constexpr long long kGridSpinCycles = 8000000000LL;  // ~4 s: another kernel may hold SMs
 
 enum : int { kActive = 0, kExhausted = 1, kConverged = 2 };  // as krylov.cu
 
@@ -147,8 +147,7 @@ __global__ void __launch_bounds__(Threads<S>::n, 1) k_lanczos_grid(GridArgs<S> a
       atomicAdd(a.bar, 1u);
       const long long t0 = clock64();
       while (int(ld_acquire(a.bar) - target) < 0)
-        if (clock64() - t0 > kGridSpinCycles) {
-          atomicOr(a.err, kDevErrSpin);
+        if (clock64() - t0 > a.spin) {
           s_bad = 1;
           break;
         }

@@ -28,8 +28,8 @@ struct GridArgs {
   double* h;              // [m + 1][C]
   double* npart;          // [C][nblk]
   unsigned* bar;          // zero at launch
-  int* steps;             // steps taken
-  int* err;
+  int* steps;             // steps taken; untouched where a wait ran out
+  long long spin;         // SM cycles that a barrier waits at the most
   int list_smem;          // the blocks' neighbour lists sit in shared memory
 };
 
