@@ -2140,10 +2140,14 @@ GridPlan plan_grid(OpDev* op, int64_t N, int C, int m, cudaStream_t s) {
   const char* e = getenv("LGT_PANEL_GRID");
   if ((e && e[0] == '0') || hpsi_forced() || (sizeof(S) == 4 && !df_reductions_enabled()))
     return g;
-  if (!ensure_table(op, s)) return g;
+  // (no table is built for panels that the cycle cannot take)
+  if (!lanczos_grid_plan<S>(N, C, m, table_row_moves(op->G, op->model), &g.rpb, &g.nblk,
+                            &g.list_smem, &g.bytes) ||
+      !ensure_table(op, s))
+    return g;
   g.T = op->table_ord && op->table_ord->state == 1 && op->table_ord->perm ? op->table_ord
                                                                           : op->table;
-  g.on = lanczos_grid_plan<S>(N, C, m, g.T->mm, &g.rpb, &g.nblk, &g.list_smem, &g.bytes);
+  g.on = true;
   return g;
 }
 

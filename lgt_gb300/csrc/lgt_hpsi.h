@@ -82,6 +82,7 @@ struct SegmentOrder {
 // Whether the basis fits the table format (N < 2^31, fewer than 2^32
 // entries, counts and sum of e^2 below 256); *bytes: an upper bound of the
 // table's size.
+int table_row_moves(const Geom& G, uint32_t model);  // most entries a row can have
 bool nbr_table_eligible(const Geom& G, int64_t N, uint32_t model, size_t* bytes);
 std::string build_nbr_table(const Geom& G, const RankView& R, uint32_t model, int* err,
                             NbrTable* T, cudaStream_t s);

@@ -1,5 +1,6 @@
 """How the panel solver chooses between its one-launch cycle and the single
-launches: a cycle whose barrier wait runs out is done again by single launches.
+launches: a cycle whose barrier wait runs out is done again by single launches,
+and panels that the cycle cannot take cost no table.
 
 Bars as for every solver: energies 1e-10 relative, states 1e-8 (FP64) and 1e-3
 (FP32-mixed, residual 2e-5)."""
@@ -42,4 +43,22 @@ def test_expired_wait_falls_back(monkeypatch, precision, nx, ny, K, kd):
         assert np.max(np.abs(got[0] - single[0]) / np.abs(single[0])) <= 1e-10
         assert np.max(np.linalg.norm(got[1] - single[1], axis=0)) <= bar
         assert np.all(np.isfinite(got[3]))
+    b.close()
+
+
+def test_no_table_for_panels_the_cycle_cannot_take(monkeypatch):
+    """4x3, K = 64 in FP64: a block's rows do not fit, and with the tuner off
+    the single launches need no table."""
+    monkeypatch.setenv("LGT_AUTOTUNE", "0")
+    b, _ = lgt.build_basis(4, 3, 1, lgt.staggered_charges(4, 3))
+    n = {}
+    for env in ("0", "1"):
+        monkeypatch.setenv("LGT_PANEL_GRID", env)
+        H = lgt.build_hamiltonian(b, g=np.geomspace(0.5, 2.0, 64), t=1.0, m=0.4)
+        n0 = C.launch_count()
+        with pytest.raises(lgt.NotConverged):
+            lgt.find_ground_state(H, solver="panel", krylovdim=10, maxiter=0, as_complex=False)
+        n[env] = C.launch_count() - n0
+        H.close()
+    assert n["1"] == n["0"]
     b.close()
