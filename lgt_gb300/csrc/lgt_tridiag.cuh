@@ -398,12 +398,17 @@ __device__ inline double warp_lowest_eig_f32(const double* a64, const double* b6
 //   * the bottom-up pivots u_i = d_i - s - b_i^2 / u_{i+1} at the lower end s
 //     of the bracket (all positive but the top one) give the eigenvector by
 //     its ratios z_i / z_{i-1} = -b_{i-1} / u_i: products, no differences, so
-//     even a tail component of 1e-13 has a few FP32 ulps per factor, and the
-//     residual |beta_n z_n| is known to about 1e-5 of itself.
-// Only a converged check, or one that must hand out the vector, goes on to
-// FP64: one inverse iteration in FP32, then defect correction, the residual (T - theta) z in FP64 by all lanes,
-// the correction from the FP32 pivots (projected against z), about six digits
-// a round.  Clustered lowest eigenvalues (a second one within 4e-6 of the
+//     even a tail component of 1e-13 has a few FP32 ulps per factor.  The
+//     shift lies up to 1e-6 of the spread below the eigenvalue: the residual
+//     |beta_n z_n| is known to 3e-4 of itself where the start vector holds
+//     1e-3 of the state or more, to 4e-3 at 1e-4 and a tenth at 2e-5; one
+//     inverse iteration leaves 4e-6 (300 levels, the second one 1/38 of the
+//     spread above).
+// "Not converged" is decided by that residual (a wrong one costs steps, not
+// accuracy).  A converged check, or one that must hand out the vector, goes on
+// to FP64: one inverse iteration in FP32, then defect correction, the residual
+// (T - theta) z in FP64 by all lanes, the correction from the FP32 pivots
+// (projected against z), about six digits a round.  Clustered lowest eigenvalues (a second one within 4e-6 of the
 // spread), a start vector with less than 1e-5 of the state (the ratios' tail
 // is 10 % low there), ranges FP32 cannot hold and corrections that stall take
 // warp_lowest_eig instead, at 260k (n = 33) to 440k cycles (n = 60), so none
@@ -692,8 +697,8 @@ __device__ inline double warp_check_lowest_f32(const double* a, const double* b,
       warp_lowest_f32_pivots(a, b, n, w, warm, th_prev, r_prev, &th, &tail, &width, &sc)) {
     improve_f32(w, n);
     for (int i = lane; i < n; i += 32) z[i] = double(w[4 * kTriMax + i]);
-    *resid = fabs(bn) * double(tail);
     __syncwarp();
+    *resid = fabs(bn * z[n - 1]);  // (`tail` is off by up to a tenth, see above)
     return a[0] + double(th);
   }
   const double t = warp_lowest_eig_f32(a, b, n, z, work, false, false, 0.0, 0.0);
