@@ -266,6 +266,7 @@ __global__ void __launch_bounds__(kCta, 1) k_lanczos_cta(const SmallProblem* pro
   __shared__ double s_sum[3];  // unit_reduce results: sum, sqrt, 1 / sqrt
   __shared__ double s_nb;      // |w|^2 before the latest pass
   __shared__ double s_thr;     // the step's space is exhausted when beta is not above it
+  __shared__ double s_lim;     // a further pass is needed when |w|^2 is below it
   __shared__ int s_exh, s_more;  // ... and whether; a further pass is needed
   __shared__ __align__(16) double s_work[3 * kMaxM];
   __shared__ double s_theta, s_resid;
@@ -532,6 +533,7 @@ __global__ void __launch_bounds__(kCta, 1) k_lanczos_cta(const SmallProblem* pro
           double scl = fabs(s_alpha[j]);
           if (j > 0) scl = fmax(scl, s_beta[j - 1]);
           s_thr = tiny_rel * fmax(scl, 1.0);
+          s_lim = 1e-4 * s_nb;
         }
         // w -= sum_b h_b V_b.  Mixed: the leading parts by TwoSum, the
         // trailing parts apart, renormalised at the end (Dot2 form)
@@ -580,8 +582,7 @@ __global__ void __launch_bounds__(kCta, 1) k_lanczos_cta(const SmallProblem* pro
             s_rb[1] = narrow(rs - widen(rh));
           }
           s_exh = (b > s_thr) ? 0 : 1;
-          // high words as logarithms: 1e-4 is 13.3 binades
-          s_more = __double2hiint(sv) < __double2hiint(s_nb) - 13933000 ? 1 : 0;
+          s_more = sv < s_lim ? 1 : 0;
           s_nb = sv;
         });
         if (!s_more || pass + 1 >= prm.reorth) break;
