@@ -1046,18 +1046,35 @@ std::string small_ground_states(const std::vector<SmallJob>& jobs, const SmallPa
   int rows = prm.rows_per_thread;
   int cl = cl_env ? cl_env : 1;
   static std::mutex mu;
-  static std::map<std::tuple<int, int, int, int>, std::pair<int, int>> cache;
-  const auto key = std::make_tuple(maxN, int(nunits), mixed ? 1 : 0, cl_env);
+  // by what a shape's time depends on: the batch, the models' moves and the
+  // Krylov dimension (whether lists and basis fit the shared memory), the device
+  int dev = 0;
+  SCK(cudaGetDevice(&dev));
+  uint32_t models = 0;
+  for (const SmallJob& jb : jobs) models |= 1u << (jb.pattern->model & 31u);
+  using Key = std::tuple<int, int, int, int, int, uint32_t, int, int>;
+  static std::map<Key, std::pair<int, int>> cache;
+  const Key key(maxN, int(nunits), mixed ? 1 : 0, cl_env, dev, models, prm.max_moves, prm.m);
   if (rows == 0) {
     // Autotuner over the launch shape: CTAs per unit (1, or a cluster of 2
     // holding half the rows each) and rows per thread R0 (the fewest that
     // fit 512 threads), R0 + 1 or 2 R0 (fewer warps: fewer instructions per
-    // basis vector, less latency hiding); timed on this batch once per
-    // (largest sector, units, precision), the solve then runs with the
-    // fastest.  A solve from a given start vector takes the tuned shape when
-    // there is one, else the smallest.
+    // basis vector, less latency hiding); timed on this batch once per key,
+    // the solve then runs with the fastest.  A solve from a given start vector
+    // takes the tuned shape when there is one (else that of another Krylov
+    // dimension), else the smallest.
     std::unique_lock<std::mutex> lk(mu);
     auto it = cache.find(key);
+    if (it == cache.end() && prm.start_given) {
+      Key first = key;
+      std::get<7>(first) = 0;
+      const auto at = cache.lower_bound(first);
+      if (at != cache.end()) {
+        Key k = at->first;
+        std::get<7>(k) = prm.m;
+        if (k == key) it = at;
+      }
+    }
     if (it != cache.end()) {
       rows = it->second.first;
       cl = it->second.second;
