@@ -1003,7 +1003,7 @@ __global__ void k_check_lowest(const double* alpha, const double* beta, int ldT,
   double th, r;
   bool conv;
   if (fp32) {
-    th = warp_lowest_eig_f32(s_a, s_b, n, s_z, s_work, warm, false, tp, rp);
+    th = warp_lowest_eig_f32(s_a, s_b, n, s_z, s_work, warm, tp, rp);
     r = fabs(bn * s_z[n - 1]);
     conv = r <= tol;
   } else {

@@ -557,7 +557,7 @@ __global__ void __launch_bounds__(Threads<S>::n, 1) k_lanczos_grid(GridArgs<S> a
             double th, r;
             bool conv, vec = true;  // vec: s_tz holds the vector
             if constexpr (kDF) {
-              th = warp_lowest_eig_f32(s_ta, s_tb, n, s_tz, s_work, warm, false, tp, rp);
+              th = warp_lowest_eig_f32(s_ta, s_tb, n, s_tz, s_work, warm, tp, rp);
               r = fabs(bn * s_tz[n - 1]);
               conv = r <= a.tol;
             } else {

@@ -56,18 +56,13 @@ __device__ inline int sturm_below(const double* a, const double* bb, int n, doub
 }
 
 // Lowest eigenpair of the n x n symmetric tridiagonal (a, b) by warp-parallel
-// multisection of the Sturm count (32 probes per round), then inverse
-// iteration on the positive-definite T - (theta - delta) I by lane 0,
-// starting from z when warm (z holds the previous eigenvector, padded with
-// zeros, warm_z) or from ones.  When warm, the previous lowest Ritz value th_prev
-// (an upper bound: the lowest Ritz value only decreases as the Krylov space
-// grows) and its residual r_prev bracket the search, [th_prev - 2 r_prev,
-// th_prev], if the Sturm count confirms the lower end; otherwise the
-// Gershgorin interval is used.  Called by one full warp; bb (n entries of
-// work space after the first kTriMax) and z are written by lane 0 / the warp.
+// multisection of the Sturm count (32 probes per round) over the Gershgorin
+// interval, then two inverse iterations on the positive-definite T - (theta -
+// delta) I by lane 0, starting from ones.  Called by one full warp; bb (n
+// entries of work space after the first kTriMax) and z are written by lane 0 /
+// the warp.
 __device__ inline double warp_lowest_eig(const double* a, const double* b, int n, double* z,
-                                         double* work, bool warm, bool warm_z, double th_prev,
-                                         double r_prev) {
+                                         double* work) {
   const int lane = threadIdx.x & 31;
   double* bb = work + 2 * kTriMax;
   for (int i = lane; i < n - 1; i += 32) bb[i] = b[i] * b[i];
@@ -79,18 +74,6 @@ __device__ inline double warp_lowest_eig(const double* a, const double* b, int n
     hi = fmax(hi, a[i] + r);
   }
   const double scale = fmax(fmax(fabs(lo), fabs(hi)), 1e-300);
-  if (warm) {
-    const double whi = fmin(hi, th_prev + 8.0 * 2.2e-16 * scale);
-    const double wlo = fmax(lo, th_prev - fmax(2.0 * r_prev, 1e-9 * scale));
-    // lane 0 probes the lower end, lane 1 the upper end
-    const double xp = (lane == 0) ? wlo : whi;
-    const int c = sturm_below(a, bb, n, xp);
-    const int c_lo = __shfl_sync(0xffffffffu, c, 0), c_hi = __shfl_sync(0xffffffffu, c, 1);
-    if (c_lo == 0 && c_hi >= 1) {
-      lo = wlo;
-      hi = whi;
-    }
-  }
   for (int it = 0; it < 40; ++it) {
     if (hi - lo <= 2.2e-16 * scale) break;
     const double step = (hi - lo) / 33.0;
@@ -117,11 +100,9 @@ __device__ inline double warp_lowest_eig(const double* a, const double* b, int n
   const double shift = theta - 4.0 * 2.2e-16 * scale;
   double* d = work;  // reciprocal pivots
   double* l = work + kTriMax;
-  if (!warm_z)
-    for (int i = lane; i < n; i += 32) z[i] = 1.0;
+  for (int i = lane; i < n; i += 32) z[i] = 1.0;
   __syncwarp();
-  const int reps = warm_z ? 1 : 2;
-  for (int rep = 0; rep < reps; ++rep) {
+  for (int rep = 0; rep < 2; ++rep) {
     if (lane == 0) {
       double dprev = 0.0, bprev = 0.0, zprev = 0.0;
       for (int i0 = 0; i0 < n; i0 += 8) {
@@ -236,10 +217,14 @@ __device__ inline int sturm_below_f(const float* a, const float* bb, int n, floa
 // (GB300's FP64 pipe makes a one-warp FP64 recurrence a long latency
 // chain).  theta is good to ~1e-6 |T| and z to FP32 accuracy: the FP32
 // Krylov basis resolves no more, and the energy returned by the solver is
-// the FP64 Rayleigh quotient of the final vector.
+// the FP64 Rayleigh quotient of the final vector.  When warm, the previous
+// lowest Ritz value th_prev (an upper bound: the lowest Ritz value only
+// decreases as the Krylov space grows) and its residual r_prev bracket the
+// search, [th_prev - 2 r_prev, th_prev], if Sturm counts confirm its ends;
+// otherwise the Gershgorin interval is used.
 __device__ inline double warp_lowest_eig_f32(const double* a64, const double* b64, int n,
-                                             double* z, double* work, bool warm, bool warm_z,
-                                             double th_prev, double r_prev) {
+                                             double* z, double* work, bool warm, double th_prev,
+                                             double r_prev) {
   const int lane = threadIdx.x & 31;
   float* a = reinterpret_cast<float*>(work);
   float* b = a + kTriMax;
@@ -304,10 +289,9 @@ __device__ inline double warp_lowest_eig_f32(const double* a64, const double* b6
   // operands eight entries ahead so that the sweep waits on its arithmetic
   // rather than on shared-memory loads; the scaling by the whole warp
   const float shift = theta - 4e-7f * scale;
-  for (int i = lane; i < n; i += 32) zf[i] = warm_z ? float(z[i]) : 1.0f;
+  for (int i = lane; i < n; i += 32) zf[i] = 1.0f;
   __syncwarp();
-  const int reps = warm_z ? 1 : 2;
-  for (int rep = 0; rep < reps; ++rep) {
+  for (int rep = 0; rep < 2; ++rep) {
     if (lane == 0) {
       float dprev = 0.0f, bprev = 0.0f, zprev = 0.0f;
       for (int i0 = 0; i0 < n; i0 += 8) {
@@ -701,7 +685,7 @@ __device__ inline double warp_check_lowest_f32(const double* a, const double* b,
     *resid = fabs(bn * z[n - 1]);  // (`tail` is off by up to a tenth, see above)
     return a[0] + double(th);
   }
-  const double t = warp_lowest_eig_f32(a, b, n, z, work, false, false, 0.0, 0.0);
+  const double t = warp_lowest_eig_f32(a, b, n, z, work, false, 0.0, 0.0);
   *resid = fabs(bn * z[n - 1]);
   return t;
 }
@@ -796,7 +780,7 @@ __device__ inline bool warp_check_lowest(const double* a, const double* b, int n
       return *resid <= tol;
     }
   }
-  *theta = warp_lowest_eig(a, b, n, z, work, false, false, 0.0, 0.0);
+  *theta = warp_lowest_eig(a, b, n, z, work);
   *resid = fabs(bn * z[n - 1]);
   return *resid <= tol;
 }
