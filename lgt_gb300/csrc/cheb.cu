@@ -11,8 +11,8 @@
 // T_n (gathered) and T_{n-1} once and writes T_{n+1}, and one pass at the end
 // sums the stored panels.  Measured against the Krylov step, observables
 // included: 4x4 K = 8 mixed, two steps of dt = 0.05, 114.6 -> 36.4 ms; 4x4
-// K = 3 FP64 with plaquettes, one step, 85.1 -> 36.5 ms (bound by the FP64
-// pipe of the products); 3x4 K = 1 FP64, ten steps, 13.5 -> 2.3 ms.
+// K = 3 FP64 with plaquettes, one step, 85.1 -> 36.5 ms (issue of the products'
+// integer sums); 3x4 K = 1 FP64, ten steps, 13.5 -> 2.3 ms.
 //
 // Errors.  FP64: that of the Krylov steps (3e-15 to 9e-15).  Mixed: every T_n is
 // rounded to FP32 once, when it is stored.  The couplings of the products are

@@ -38,8 +38,9 @@ constexpr int kTabThreads = kTabWarps * 32;
 // 4x4 lattice, K = 8 complex FP32: 5 blocks with 8 rows in flight beat 6
 // with 4 (0.714 vs 0.757 ms); 8 blocks (32 registers) spill.  With the tiles
 // in the order of the mask segments one vector a lane is the best load mode
-// (0.694 ms; two vectors 0.726, one 32-byte access 0.745): nothing but the
-// gathers' traffic from L2, 7.3 GB, is near a limit.
+// (0.694 ms; two vectors 0.726, one 32-byte access 0.745).  No unit is near a
+// limit then (L1 wavefronts 64 %, issue 66 %, DRAM 49 %, L2 reads 48 %): the
+// lanes wait for their gathers, 7.3 stalled warps an issue.
 #ifndef LGT_TABLE_MINB
 #define LGT_TABLE_MINB 5
 #endif

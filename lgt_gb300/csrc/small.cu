@@ -3,18 +3,21 @@
 //
 // For sectors up to kSmallMaxN states the step latency of the panel path
 // (about ten dependent kernels per Lanczos step) dominates, so here every
-// (problem, point) unit is one CTA of just enough warps for R rows per
-// thread (at most 512 threads) that keeps the current Lanczos residual in
-// registers (row r of thread t: r = t + i * blockDim) and the Krylov basis
-// in global memory (L2-resident), and runs matvec, classical Gram-Schmidt
-// against the whole basis (FP64 accumulation, warp reduce-scatter; a second
-// pass only on cancellation), the tridiagonal check (lgt_tridiag.cuh),
-// restarts and the FP64 finish without leaving the kernel.  Units of
-// different sectors and sizes share one launch (uneven batch); the largest
-// are scheduled first.  When the basis of the largest sector fits (the
-// FP32-mixed path up to about 1000 states at krylovdim 50), it sits in
-// shared memory instead: one CTA per SM either way, and the Gram-Schmidt
-// and matvec loads then wait on shared memory, not on L2.
+// (problem, point) unit is one CTA, or a cluster of two that split the rows,
+// of just enough warps for R rows per thread (at most 512 threads).  It keeps
+// the current Lanczos residual in registers (row r of thread t: r = t + i *
+// blockDim) and runs matvec, classical Gram-Schmidt against the whole basis
+// (eight vectors a round; sums in double-float on the mixed path, in FP64 with
+// the lanes added in integers on the other; a second pass only on
+// cancellation), the tridiagonal check (lgt_tridiag.cuh), restarts and the
+// FP64 finish without leaving the kernel.  Units of different sectors and
+// sizes share one launch (uneven batch); the largest are scheduled first.
+//
+// A CTA's own rows of the Krylov basis with the whole current vector, and for
+// R <= 4 its neighbour lists, sit in shared memory where the largest sector's
+// fit 200 KB (on two CTAs and krylovdim 50: up to about 1900 states mixed, 950
+// FP64); the basis is in global memory (L2) otherwise.  One CTA per SM either
+// way.
 //
 // The neighbour ranks of a lattice are computed once by a device "lookup
 // pass" (k_pattern_*: the move enumeration and rank of the H*psi kernel)

@@ -7,7 +7,7 @@ namespace lgt {
 // Slices of 16 bytes where they divide the panel row, else of 8.  (32-byte
 // ones take half the instructions, but the lanes wait on L2 and have more rows
 // in flight with the smaller ones: 4x4 K = 8 quench, FP32-mixed, 35.9 ms a run
-// with 32-byte slices, 35.1 with 16, 40.5 with 8.)
+// with 32-byte slices, 35.1 with 16, 40.5 with 8, all with one chain of sums.)
 cudaError_t launch_cheb_product(const NbrTable& T, uint32_t model, int64_t N, int K, const float* x,
                                 float* y, const float* prev, float* low, const float* coef,
                                 cudaStream_t s) {
