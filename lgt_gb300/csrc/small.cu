@@ -585,7 +585,8 @@ __global__ void __launch_bounds__(kCta, 1) k_lanczos_cta(const SmallProblem* pro
             s_rb[1] = narrow(rs - widen(rh));
           }
           s_exh = (b > s_thr) ? 0 : 1;
-          s_more = sv < s_lim ? 1 : 0;
+          // (as integers: neither is negative, and an FP64 comparison is 64 cycles)
+          s_more = __double_as_longlong(sv) < __double_as_longlong(s_lim) ? 1 : 0;
           s_nb = sv;
         });
         if (!s_more || pass + 1 >= prm.reorth) break;
