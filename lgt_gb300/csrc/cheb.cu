@@ -10,7 +10,7 @@
 // earlier vectors per product, 55 % of a 4x4 K = 8 step): a product reads
 // T_n (gathered) and T_{n-1} once and writes T_{n+1}, and one pass at the end
 // sums the stored panels.  Measured against the Krylov step, observables
-// included: 4x4 K = 8 mixed, two steps of dt = 0.05, 114.6 -> 36.4 ms; 4x4
+// included: 4x4 K = 8 mixed, two steps of dt = 0.05, 114.6 -> 35.0 ms; 4x4
 // K = 3 FP64 with plaquettes, one step, 85.1 -> 36.5 ms (issue of the products'
 // integer sums); 3x4 K = 1 FP64, ten steps, 13.5 -> 2.3 ms.
 //

@@ -15,10 +15,11 @@
 // FP32 panels: A x + B sum_hops + C sum_plaq - prev with the scale folded into
 // the couplings, these as pairs of FP32 numbers (PairCoef below), and the
 // neighbours added pairwise, so that a new entry sees about three roundings
-// of its own size (errors: cheb.cu).  The 4x4 K = 8 quench takes 36.4 ms a run
-// with them, 35.2 with FP32 couplings, one chain of sums and the scale apart;
-// with every error carried by TwoSum and TwoProduct 48.0 (and two thirds of
-// the state's error).  Where `low` is given, an entry's products and their sum
+// of its own size (errors: cheb.cu).  The 4x4 quench takes 35.0 ms a run with
+// them for K = 8, 27.2 for K = 5 and 54.3 for K = 8 with plaquettes (with FP32
+// couplings, one chain of sums and the scale apart 35.2, 26.6 and 51.8); with
+// every error carried by TwoSum and TwoProduct 48.0 for K = 8 (and two thirds
+// of the state's error).  Where `low` is given, an entry's products and their sum
 // carry their errors and what its rounding drops is stored.
 #pragma once
 
@@ -156,7 +157,7 @@ __device__ __forceinline__ float diag_lo(const float* c, int K, float e2, float 
 
 // U: entries in flight (FP64; FP32 has eight).
 template <typename T, int W, int U, bool PLAQ, bool JW>
-__global__ void __launch_bounds__(kThreads, PLAQ || JW || sizeof(T) == 8 ? 4 : 5)
+__global__ void __launch_bounds__(kThreads, PLAQ || JW || W * sizeof(T) != 8 ? 4 : 5)
     k_cheb_product(Args<T> a) {
   static_assert(W % 2 == 0, "a slice holds whole points");
   extern __shared__ __align__(16) unsigned char smem[];
@@ -221,12 +222,20 @@ __global__ void __launch_bounds__(kThreads, PLAQ || JW || sizeof(T) == 8 ? 4 : 5
 #pragma unroll
       for (int e = 0; e < W; ++e) out[e] = fma(cf[5 * K + (e >> 1)], out[e], -ah[e]);
     } else {
+      // T_{n-1} is loaded ahead of the gathers where the 64 registers of four
+      // blocks have room (the same quench, K = 8: 35.0 ms against 36.4; at five
+      // blocks 39.5; with plaquettes 56.2 against 53.1, so not there)
+      constexpr bool kAhead = W == 4 && !PLAQ && !JW;
       T ah[W], ap[W], pv[W];
+      auto load_prev = [&] {
+#pragma unroll
+        for (int e = 0; e < W; ++e) pv[e] = 0.f;
+        if (a.prev) ld_cols<T, W>(a.prev + at, pv);
+      };
+      if (kAhead) load_prev();
       sum_slices<W, JW>(x, C, col0, l, 0, nh, ah);
       if (PLAQ) sum_slices<W, false>(x, C, col0, l, nh, n1, ap);
-#pragma unroll
-      for (int e = 0; e < W; ++e) pv[e] = 0.f;
-      if (a.prev) ld_cols<T, W>(a.prev + at, pv);
+      if (!kAhead) load_prev();
       if (a.low) {
         T low[W];
 #pragma unroll
