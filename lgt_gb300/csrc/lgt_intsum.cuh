@@ -12,7 +12,9 @@
 // has them, but a sector of few states might) add the rest in FP64.
 // Infinities, NaNs,
 // magnitudes within 2^15 of overflow and subnormal ranges take plain FP64
-// additions instead (below 2^-1042 a value counts as zero).
+// additions instead; a row whose high words are all zero (values below
+// 2^-1042, or zeros) is summed exactly in units of 2^-1074.  (The solvers'
+// sums over a warp's lanes count such values as zeros.)
 #pragma once
 
 #include <cstdint>
@@ -47,6 +49,15 @@ __device__ __forceinline__ double fix_to(long long t, int eb) {
   if (t == 0) return 0.0;
   const double d = __ll2double_rn(t);
   return __hiloint2double(__double2hiint(d) + (eb - (1080 << 20)), __double2loint(d));
+}
+
+// The sum of terms whose high words are all zero, from the sum t of their
+// fix_of(v, 0): each is +-(2^57 + 32 m) for a value of +-m 2^-1074, so what
+// is left of t modulo 2^57 is 32 times the sum of the +-m.
+__device__ __forceinline__ double fix_tiny(long long t) {
+  const long long m = static_cast<long long>(static_cast<unsigned long long>(t) << 7) >> 12;
+  const double d = __longlong_as_double(m < 0 ? -m : m);
+  return m < 0 ? -d : d;
 }
 
 // s = sum of the W-column slices load(entry index) of lst[n0 .. n1), U of
@@ -93,7 +104,9 @@ __device__ __forceinline__ void int_sum_part(const uint32_t* lst, int n0, int n1
     s[e] = 0.0;
     if (fix_range(top[e])) {
       s[e] = fix_to(acc[e], top[e] & 0x7ff00000);
-    } else if (top[e] != 0) {
+    } else if (top[e] == 0) {
+      s[e] = fix_tiny(acc[e]);
+    } else {
       for (int n = n0; n < n1; ++n) {
         double v[W];
         load(lst[n] & 0x7fffffffu, v);
